@@ -230,7 +230,7 @@ int filter_impl(sep_ctx* c, const double* d_start, long ns, const double* an_re,
   if (K < 1) K = 1;
   const long long B = (ns + 1) / 2;
   const size_t per_pair = sizeof(cx<T>) * (size_t)n * (size_t)(K + 1) +
-                          sizeof(T) * 2 * (size_t)ms * (size_t)n;
+                          sizeof(T) * accumulator_values<T>(n, ms);
   const size_t have = c->w_hist.bytes + c->w_fft.bytes + c->w_acc.bytes;
   size_t budget = (size_t)(0.6 * (double)free_device_bytes()) + have;
   long long Bc = (long long)(budget / per_pair);
@@ -239,7 +239,7 @@ int filter_impl(sep_ctx* c, const double* d_start, long ns, const double* an_re,
   if (Bc > 65535) Bc = 65535;
   RET(grow(c, c->w_hist, sizeof(cx<T>) * (size_t)n * K * Bc));
   RET(grow(c, c->w_fft, sizeof(cx<T>) * (size_t)n * Bc));
-  RET(grow(c, c->w_acc, sizeof(T) * 2 * (size_t)ms * n * Bc));
+  RET(grow(c, c->w_acc, sizeof(T) * accumulator_values<T>(n, ms) * Bc));
   RET(grow(c, c->w_coef, sizeof(T) * (size_t)ms * nc));
   RET(grow(c, c->w_steps, sizeof(T) * 2 * (size_t)nc));
   // coefficients and per-step epilogue scalars (hnorm.c:17-23)
@@ -1010,7 +1010,7 @@ template <typename T> int time_passes_impl(sep_ctx* c, long npairs, int reps, do
   const int ms = 8;
   RET(grow(c, c->w_hist, sizeof(cx<T>) * (size_t)n * K * npairs));
   RET(grow(c, c->w_fft, sizeof(cx<T>) * (size_t)n * npairs));
-  RET(grow(c, c->w_acc, sizeof(T) * 2 * (size_t)ms * n * npairs));
+  RET(grow(c, c->w_acc, sizeof(T) * accumulator_values<T>(n, ms) * npairs));
   RET(grow(c, c->w_coef, sizeof(T) * (size_t)ms * K));
   CK(cudaMemsetAsync(c->w_hist.p, 0, c->w_hist.bytes, c->stream));
   CK(cudaMemsetAsync(c->w_fft.p, 0, c->w_fft.bytes, c->stream));
@@ -1137,7 +1137,7 @@ template <typename T> int batch_job_prepare(sep_ctx* c, long ns, long ms, long n
   const long long B = (ns + 1) / 2;
   RET(grow(c, c->w_hist, sizeof(cx<T>) * (size_t)n * K * B));
   RET(grow(c, c->w_fft, sizeof(cx<T>) * (size_t)n * B));
-  RET(grow(c, c->w_acc, sizeof(T) * 2 * (size_t)ms * n * B));
+  RET(grow(c, c->w_acc, sizeof(T) * accumulator_values<T>(n, ms) * B));
   RET(grow(c, c->w_coef, sizeof(T) * (size_t)ms * nc));
   RET(grow(c, c->w_steps, sizeof(T) * 2 * (size_t)nc));
   return kOk;

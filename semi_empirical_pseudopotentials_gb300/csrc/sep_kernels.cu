@@ -2,6 +2,7 @@
 // contractions (see sep_kernels.cuh).
 #include "sep_kernels.cuh"
 
+#include <algorithm>
 #include <type_traits>
 
 namespace sep {
@@ -47,7 +48,9 @@ __global__ void k_unpack(const cx<T>* __restrict__ in, long long nstates, long l
 // -------------------------------------------------------------------------
 constexpr int kMaxBlockSteps = 128;  // history grids per accumulation pass
 constexpr int kLoadBatch = 8;       // history loads in flight per thread (ms > 4)
+constexpr int kX2Threads = 128;     // k_accumulate_x2
 
+// FP64 and double-float histories (bound by their arithmetic pipes)
 template <typename T, typename TA, int MSMAX>
 __global__ void __launch_bounds__(kThreads)
 k_accumulate(const cx<T>* __restrict__ hist, int slots, int B, long long n, long long j0,
@@ -105,65 +108,36 @@ k_accumulate(const cx<T>* __restrict__ hist, int slots, int B, long long n, long
     // the 2 ms accumulators of (pair b, point g) are adjacent: targets of
     // state 2b, then of state 2b + 1
     TA* __restrict__ pa = acc + (b * n + g) * (2 * ms);
-    bool stored = false;
-    if constexpr (std::is_same<TA, float>::value) {
-    if (MSMAX <= 16 && ms == MSMAX) {
-      float4* p4 = reinterpret_cast<float4*>(pa);
 #pragma unroll
-      for (int q = 0; q < MSMAX / 2; ++q) {
-        TA v[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int k = 4 * q + u;
-          v[u] = k < MSMAX ? re[k] : im[k - MSMAX];
-        }
-        float4 o = make_float4((float)v[0], (float)v[1], (float)v[2], (float)v[3]);
-        if (!init) {
-          const float4 old = p4[q];
-          o = make_float4(old.x + o.x, old.y + o.y, old.z + o.z, old.w + o.w);
-        }
-        p4[q] = o;
-      }
-    } else if (ms % 2 == 0) {
-      float2* q0 = reinterpret_cast<float2*>(pa);
-      float2* q1 = reinterpret_cast<float2*>(pa + ms);
-#pragma unroll
-      for (int e = 0; e < MSMAX; e += 2) {
-        if (e < ms) {
-          float2 r = make_float2((float)re[e], (float)re[e + 1]);
-          float2 i = make_float2((float)im[e], (float)im[e + 1]);
-          if (!init) {
-            const float2 r0 = q0[e / 2], i0 = q1[e / 2];
-            r = make_float2(r0.x + r.x, r0.y + r.y);
-            i = make_float2(i0.x + i.x, i0.y + i.y);
-          }
-          q0[e / 2] = r;
-          q1[e / 2] = i;
-        }
-      }
-    }
-    stored = (MSMAX <= 16 && ms == MSMAX) || ms % 2 == 0;
-    }
-    if (!stored) {
-#pragma unroll
-      for (int e = 0; e < MSMAX; ++e) {
-        if (e < ms) {
-          pa[e] = init ? re[e] : pa[e] + re[e];
-          pa[ms + e] = init ? im[e] : pa[ms + e] + im[e];
-        }
+    for (int e = 0; e < MSMAX; ++e) {
+      if (e < ms) {
+        pa[e] = init ? re[e] : pa[e] + re[e];
+        pa[ms + e] = init ? im[e] : pa[ms + e] + im[e];
       }
     }
   }
 }
 
-// Complex64 history, FP32 accumulators and exactly MS targets (the common
-// case): as k_accumulate, with two adjacent grid points per thread (16-byte
-// history loads) and the coefficients of four steps per 16-byte shared load,
-// so that the shared-memory pipe issues a quarter of the loads per multiply-
-// add.  Each point's sums take the same products in the same order as in
-// k_accumulate, so the results are equal bit for bit.  n is even.
+// Complex64 history, FP32 accumulators and exactly MS targets: two adjacent
+// grid points per thread (16-byte history loads) and the coefficients of four
+// steps per 16-byte shared load, so that the shared-memory pipe issues one
+// load per 16 multiply-adds.  One kernel per target count: the accumulators
+// are indexed at compile time and no multiply-add is spent on targets that do
+// not exist.  The sums of 64 adjacent points are stored as [quad q][thread of
+// the warp]: every 16-byte access of a warp covers 512 adjacent bytes (with a
+// point's 2 MS sums adjacent, a warp's accesses are 16 MS bytes apart and the
+// load/store unit bounds the kernel).  Bound by HBM: a point reads its history
+// once, and its 2 MS sums are read and written once per block of steps.  32
+// steps of 24 pairs of 80 x 64 x 64: 10 targets 0.47 ms (7.0 TB/s), 16 0.64 ms
+// (6.3), 20 0.66 ms (6.8; 1.9 ms with one point per thread, scalar coefficient
+// loads and room for 32 targets); 8 pairs of 128^3, 8 targets: 0.91 ms (7.1;
+// 1.05 ms with a point's sums adjacent).  128 registers (four blocks of 128
+// threads per SM) hold up to 24 targets, three blocks 32.
+// Each point's sums take the products in step order, so a target's sums do
+// not depend on how many targets there are.  n is even (every supported axis
+// length is).
 template <int MS>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kX2Threads, MS <= 24 ? 4 : 3)
 k_accumulate_x2(const float4* __restrict__ hist, int slots, int B, long long n2, long long j0,
                 int count, const float* __restrict__ an, long long nc,
                 float* __restrict__ acc, int init) {
@@ -219,27 +193,65 @@ k_accumulate_x2(const float4* __restrict__ hist, int slots, int B, long long n2,
         im1[e] += c * h.w;
       }
     }
-    // the 2 MS accumulators of (pair b, point g): targets of state 2b, then
-    // of state 2b + 1; points 2 g2 and 2 g2 + 1 are adjacent
-    float4* p4 = reinterpret_cast<float4*>(acc + (b * 2 * n2 + 2 * g2) * (2 * MS));
+    // the thread's 4 MS sums, quad q at [chunk of 64 points][q][thread]: value
+    // k = 4 q + u is target e of state 2b + c at point 2 g2 + pt, with k =
+    // (2 pt + c) MS + e
+    float4* p4 = reinterpret_cast<float4*>(acc) +
+                 ((b * ((n2 + 31) / 32) + g2 / 32) * MS * 32 + (g2 & 31));
 #pragma unroll
-    for (int pt = 0; pt < 2; ++pt) {
+    for (int q = 0; q < MS; ++q) {
+      float v[4];
 #pragma unroll
-      for (int q = 0; q < MS / 2; ++q) {
-        float v[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int k = 4 * q + u;
-          v[u] = pt == 0 ? (k < MS ? re0[k] : im0[k - MS]) : (k < MS ? re1[k] : im1[k - MS]);
-        }
-        float4 o = make_float4(v[0], v[1], v[2], v[3]);
-        float4* dst = p4 + pt * (MS / 2) + q;
-        if (!init) {
-          const float4 old = *dst;
-          o = make_float4(old.x + o.x, old.y + o.y, old.z + o.z, old.w + o.w);
-        }
-        *dst = o;
+      for (int u = 0; u < 4; ++u) {
+        const int k = 4 * q + u, e = k % (2 * MS);
+        v[u] = k < 2 * MS ? (e < MS ? re0[e % MS] : im0[e % MS])
+                          : (e < MS ? re1[e % MS] : im1[e % MS]);
       }
+      float4 o = make_float4(v[0], v[1], v[2], v[3]);
+      if (!init) {
+        const float4 old = p4[q * 32];
+        o = make_float4(old.x + o.x, old.y + o.y, old.z + o.z, old.w + o.w);
+      }
+      p4[q * 32] = o;
+    }
+  }
+}
+
+template <int MS>
+cudaError_t launch_x2(dim3 g, const cx<float>* hist, int slots, int B, long long n, long long j0,
+                      int count, const float* an, long long nc, int ms, float* acc, bool init,
+                      cudaStream_t s) {
+  if constexpr (MS <= 32) {
+    if (ms != MS)
+      return launch_x2<MS + 1>(g, hist, slots, B, n, j0, count, an, nc, ms, acc, init, s);
+    k_accumulate_x2<MS><<<g, kX2Threads, 0, s>>>(reinterpret_cast<const float4*>(hist), slots, B,
+                                               n / 2, j0, count, an, nc, acc, init);
+    return cudaGetLastError();
+  } else {
+    return cudaErrorInvalidValue;
+  }
+}
+
+// k_accumulate_x2's sums -> out[(2b + c) ms + e][g] (state-major, double): a
+// thread takes the two points of one thread of that kernel, so both the
+// 16-byte loads and the 16-byte stores of a warp are adjacent.  Bound by HBM:
+// 48 states x 20 targets of 80 x 64 x 64 in 0.59 ms (6.4 TB/s), 0.73 ms with a
+// point's sums adjacent.
+__global__ void k_unpack_x2(const float4* __restrict__ acc, long long B, long long n2, int ms,
+                            long long nstates, double* __restrict__ out) {
+  const long long chunks = (n2 + 31) / 32;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < B * chunks * 32;
+       i += (long long)gridDim.x * blockDim.x) {
+    const long long b = i / (chunks * 32), g2 = i - b * (chunks * 32);
+    if (g2 >= n2) continue;
+    const float* p = reinterpret_cast<const float*>(
+        acc + ((b * chunks + g2 / 32) * ms * 32 + (g2 & 31)));
+    double2* o = reinterpret_cast<double2*>(out) + 2 * b * ms * n2 + g2;
+    const int count = 2 * b + 1 < nstates ? 2 * ms : ms;
+    for (int k = 0; k < count; ++k) {  // k = c ms + e; point 2 g2 + 1 is 2 ms values on
+      const int k1 = k + 2 * ms;
+      const float x = p[(k / 4) * 128 + k % 4], y = p[(k1 / 4) * 128 + k1 % 4];
+      o[(long long)k * n2] = make_double2((double)x, (double)y);
     }
   }
 }
@@ -580,32 +592,36 @@ cudaError_t newton_accumulate(const cx<T>* hist, int slots, int B, long long n, 
                               long long nstates, bool init, cudaStream_t s) {
   if (count < 1 || count > kMaxBlockSteps || ms < 1 || ms > 32 || B > 65535)
     return cudaErrorInvalidValue;
-  // each thread sees about 4 grid points of one pair (enough blocks to keep
-  // 64 warps per SM resident while the history loads are in flight)
-  long long per = (n + 4LL * kThreads - 1) / (4LL * kThreads);
-  if (per > 65535) per = 65535;
-  if (per < 1) per = 1;
-  const dim3 g((unsigned)per, (unsigned)B);
   if constexpr (std::is_same<T, float>::value && std::is_same<TA, float>::value) {
-    if (n % 2 == 0 && ms == 8) {  // two points per thread
-      k_accumulate_x2<8><<<g, kThreads, 0, s>>>(reinterpret_cast<const float4*>(hist), slots,
-                                                 B, n / 2, j0, count, an, nc, acc, init);
-      return cudaGetLastError();
-    }
+    if (n % 2 != 0) return cudaErrorInvalidValue;
+    // 8 points per thread where that still leaves four blocks per SM to run
+    // four times over (128^3: 1.00 against 1.03 ms with 4 points), else 2
+    const long long pts = (long long)B * n >= 8LL * kX2Threads * 16 * 152 ? 8 : 2;
+    const dim3 g((unsigned)std::min<long long>(65535, (n + pts * kX2Threads - 1) /
+                                                          (pts * kX2Threads)),
+                 (unsigned)B);
+    return launch_x2<1>(g, hist, slots, B, n, j0, count, an, nc, ms, acc, init, s);
+  } else {
+    // each thread sees about 4 grid points of one pair (enough blocks to keep
+    // 64 warps per SM resident while the history loads are in flight)
+    long long per = (n + 4LL * kThreads - 1) / (4LL * kThreads);
+    if (per > 65535) per = 65535;
+    if (per < 1) per = 1;
+    const dim3 g((unsigned)per, (unsigned)B);
+    if (ms <= 4)
+      k_accumulate<T, TA, 4><<<g, kThreads, 0, s>>>(hist, slots, B, n, j0, count, an, nc, ms,
+                                                    acc, nstates, init);
+    else if (ms <= 8)
+      k_accumulate<T, TA, 8><<<g, kThreads, 0, s>>>(hist, slots, B, n, j0, count, an, nc, ms,
+                                                    acc, nstates, init);
+    else if (ms <= 16)
+      k_accumulate<T, TA, 16><<<g, kThreads, 0, s>>>(hist, slots, B, n, j0, count, an, nc, ms,
+                                                     acc, nstates, init);
+    else
+      k_accumulate<T, TA, 32><<<g, kThreads, 0, s>>>(hist, slots, B, n, j0, count, an, nc, ms,
+                                                     acc, nstates, init);
+    return cudaGetLastError();
   }
-  if (ms <= 4)
-    k_accumulate<T, TA, 4><<<g, kThreads, 0, s>>>(hist, slots, B, n, j0, count, an, nc, ms, acc,
-                                                  nstates, init);
-  else if (ms <= 8)
-    k_accumulate<T, TA, 8><<<g, kThreads, 0, s>>>(hist, slots, B, n, j0, count, an, nc, ms, acc,
-                                                  nstates, init);
-  else if (ms <= 16)
-    k_accumulate<T, TA, 16><<<g, kThreads, 0, s>>>(hist, slots, B, n, j0, count, an, nc, ms,
-                                                   acc, nstates, init);
-  else
-    k_accumulate<T, TA, 32><<<g, kThreads, 0, s>>>(hist, slots, B, n, j0, count, an, nc, ms,
-                                                   acc, nstates, init);
-  return cudaGetLastError();
 }
 template cudaError_t newton_accumulate<double, double>(const cx<double>*, int, int, long long,
                                                        long long, int, const double*, long long,
@@ -622,8 +638,14 @@ template cudaError_t newton_accumulate<ddf, ddf>(const cx<ddf>*, int, int, long 
 template <typename TA>
 cudaError_t unpack_accumulators(const TA* acc, long long B, long long n, int ms,
                                 long long nstates, double* out, cudaStream_t s) {
-  k_unpack_acc<TA><<<blocks_for(B * n, kThreads, 152LL * 16), kThreads, 0, s>>>(acc, B, n, ms,
-                                                                                 nstates, out);
+  if constexpr (std::is_same<TA, float>::value) {
+    if (n % 2 != 0) return cudaErrorInvalidValue;
+    k_unpack_x2<<<blocks_for(B * n / 2, kThreads, 152LL * 16), kThreads, 0, s>>>(
+        reinterpret_cast<const float4*>(acc), B, n / 2, ms, nstates, out);
+  } else {
+    k_unpack_acc<TA><<<blocks_for(B * n, kThreads, 152LL * 16), kThreads, 0, s>>>(
+        acc, B, n, ms, nstates, out);
+  }
   return cudaGetLastError();
 }
 template cudaError_t unpack_accumulators<float>(const float*, long long, long long, int,

@@ -20,8 +20,15 @@ cudaError_t unpack_pairs(const cx<T>* in, long long nstates, long long n, TR* re
 // ---- Newton accumulation (filter/filter.c:60-78), blocked over K steps:
 //   acc[b][g][c ms + e] (+)= sum_{s<count} an[e nc + j0 + s] * comp_c(hist[slot(j0+s)][b][g])
 // hist is a ring of `slots` grids [slots][B][n]; slot(j) = j % slots.  The 2 ms
-// accumulators of a point are adjacent; unpack_accumulators writes them out
-// state-major, out[(2b + c) ms + e][g] as double (the reference's psitot).
+// accumulators of a point are adjacent in FP64 and double-float; in FP32 those
+// of 64 adjacent points are interleaved in 16-byte quads (k_accumulate_x2), a
+// whole number of such chunks per pair.  accumulator_values: values per pair.
+// unpack_accumulators writes them out state-major, out[(2b + c) ms + e][g] as
+// double (the reference's psitot).
+template <typename TA> inline size_t accumulator_values(long long n, long ms) {
+  const size_t points = sizeof(TA) == sizeof(float) ? ((size_t)n + 63) / 64 * 64 : (size_t)n;
+  return 2 * (size_t)ms * points;
+}
 template <typename T, typename TA>
 cudaError_t newton_accumulate(const cx<T>* hist, int slots, int B, long long n, long long j0,
                               int count, const TA* an, long long nc, int ms, TA* acc,

@@ -127,3 +127,28 @@ def test_two_point_accumulation_equals_the_generic_kernel(dims, K):
     out8 = ctx.filter(start, np.ascontiguousarray(ar[:8]), zn, 4.0 / dE, vmin)
     ctx.close()
     assert np.array_equal(out8, out9[:, :8])
+
+
+@pytest.mark.parametrize("ms", [1, 2, 3, 4, 7, 12, 13, 16, 20, 21, 31])
+def test_accumulation_of_any_target_count(ms):
+    """Each target count has its own complex64 accumulation kernel; a target's
+    sums take the same products in the same order whatever the count, so a
+    filter of ms targets equals the first ms targets of a 32-target one bit for
+    bit (blocks of 32 steps and a last one of 6), which is the FP64 filter
+    within single precision (bound 1e-4 over 70 steps, as the 36^3 test's).
+    14 x 18 x 20 points are not a whole number of the kernel's 64-point chunks."""
+    dims = (14, 18, 20)
+    ctx, pot, dv, npts = _job(dims, 6, "mixed")
+    vmin = float(pot.min())
+    nc, dE = 70, 40.0
+    ar, ai, zn = sep.coefficients(np.linspace(-1.2, -0.2, 32), nc, dE, vmin,
+                                  (nc / (2.5 * dE)) ** 2)
+    start = sep.start_states(-15, 3, npts, dv)
+    full = ctx.filter(start, ar, zn, 4.0 / dE, vmin)
+    part = ctx.filter(start, np.ascontiguousarray(ar[:ms]), zn, 4.0 / dE, vmin)
+    ctx.close()
+    assert np.array_equal(part, full[:, :ms])
+    ref_ctx = _job(dims, 6, "f64")[0]
+    ref = ref_ctx.filter(start, ar, zn, 4.0 / dE, vmin)
+    ref_ctx.close()
+    assert np.abs(full - ref).max() <= 1e-4 * np.abs(ref).max()
