@@ -80,8 +80,9 @@ int sep_ctx_set_block_steps(sep_ctx *ctx, int k);
  * y transform's R-point stage (R = 4 or 8), and a fused pass per sub-plane of
  * L / R rows for the rest of the y transform, the x transforms and the
  * epilogue (same transforms with y and z split differently: equal to the line
- * passes within FP32 rounding).  On other grids with nx = ny in {40, 48, 56,
- * 64, 72, 80, 96, 112, 128}: the z line pass and one fused pass per z-plane
+ * passes within FP32 rounding).  On other grids with nx and ny in {32, 40,
+ * 48, 56, 64, 72, 80, 96, 112, 128} at most a factor of two apart, or nx = ny
+ * in {14, 16, 18, 20, 24, 36}: the z line pass and one fused pass per z-plane
  * for the x and y transforms and the epilogue (same arithmetic per line as
  * the line passes).  enable = 0 selects the four line passes.  Default 1. */
 int sep_ctx_set_fusion(sep_ctx *ctx, int enable);

@@ -446,8 +446,9 @@ class Context:
     def set_fusion(self, enable):
         """Fused two-pass complex64 Newton steps: the sub-plane and zy passes for
         cubic grids with nx in {96, 112, 128, 160, 192, 256}, else the xy plane
-        pass for nx = ny in {40, 48, ..., 128}.  On by default; off: the four
-        line passes."""
+        pass for nx and ny in {32, 40, 48, ..., 128} at most a factor of two
+        apart and for nx = ny in {14, 16, 18, 20, 24, 36}.  On by default; off:
+        the four line passes."""
         _check(lib().sep_ctx_set_fusion(self.h, 1 if enable else 0))
 
     def set_arith(self, mode):

@@ -26,7 +26,8 @@ NVCC_FLAGS = ["-std=c++17", "-O3", "-lineinfo", "--expt-relaxed-constexpr",
 CUDA_UNITS = ["sep_pass_f64.cu", "sep_pass_f32.cu", "sep_pass_f64_v1.cu", "sep_pass_f32_v1.cu",
               "sep_pass_dd.cu", "sep_pass_dd_g0.cu", "sep_pass_dd_g1.cu", "sep_pass_dd_g2.cu",
               "sep_pass_dd_g3.cu",
-              "sep_xy_f32.cu", "sep_sp_f32.cu",
+              "sep_xy_f32.cu", "sep_xy_f32_g0.cu", "sep_xy_f32_g1.cu", "sep_xy_f32_g2.cu",
+              "sep_xy_f32_g3.cu", "sep_sp_f32.cu",
               "sep_kernels.cu", "sep_ctx.cu",
               "sep_api.cu", "sep_vbuild.cu", "sep_noalloc.cu",
               "sep_ozaki.cu", "sep_bulk.cu", "sep_spinor.cu", "sep_spinor_path.cu",

@@ -152,3 +152,27 @@ def test_accumulation_of_any_target_count(ms):
     ref = ref_ctx.filter(start, ar, zn, 4.0 / dE, vmin)
     ref_ctx.close()
     assert np.abs(full - ref).max() <= 1e-4 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("dims", [(80, 64, 64), (64, 80, 24), (48, 96, 16), (96, 48, 40),
+                                  (32, 40, 36), (64, 32, 14), (56, 112, 20), (72, 40, 72),
+                                  (112, 128, 16), (128, 112, 48), (128, 64, 128), (32, 32, 32),
+                                  (36, 36, 36), (24, 24, 24), (20, 20, 16), (18, 18, 20),
+                                  (16, 16, 14), (14, 14, 14)])
+def test_plane_pass_of_rectangles_and_short_lengths(dims):
+    """Planes of two lengths (their own splits and twiddle tables, rows of one
+    length and columns of the other) and the short squares run the plane form:
+    the filters equal the line passes' bit for bit, with more planes than the
+    blocks that walk them in the larger cases and an odd number of states."""
+    ctx, pot, dv, npts = _job(dims, 8, "mixed")
+    assert ctx.time_fused_step(1, reps=1).min() > 0.0
+    vmin = float(pot.min())
+    nc, dE = 40, 40.0
+    ar, ai, zn = sep.coefficients([-1.0, -0.6], nc, dE, vmin, (nc / (2.5 * dE)) ** 2)
+    start = sep.start_states(-21, 7, npts, dv)
+    fused = ctx.filter(start, ar, zn, 4.0 / dE, vmin)
+    ctx.set_fusion(False)
+    lines = ctx.filter(start, ar, zn, 4.0 / dE, vmin)
+    ctx.close()
+    assert np.abs(lines).max() > 0.0
+    assert np.array_equal(fused, lines)
