@@ -531,7 +531,9 @@ int sep_spinor_neighbour_lists(long nx, long ny, long nz, const double *vx, cons
  * sep_spinor_set_operator: the neighbour lists (natom x nnlc sep_nlc, nl[a]
  *   used per atom, every jxyz on the grid), sigma (Gaussian form) or
  *   flagkb = 1 with elkb (2 natom energies); copied to the device, kept by
- *   the context until set again.
+ *   the context until set again.  The Gaussian form also keeps its kernel
+ *   K(j1, j2) of every atom (8 nl^2 bytes each) when that is at most an
+ *   eighth of the free device memory, and forms it on each apply otherwise.
  * sep_spinor_hamiltonian: hpsi = H psi for nspinors spinors
  *   (filterSpinors/hamiltonian.c:8-46).
  * sep_spinor_energy_range: filterSpinors/energy.c:49-109 from four

@@ -12,7 +12,10 @@
 //   K = (Vr1 + Vr2)/2 exp(-((r1 - r2) sigma_1)^2) / ((r2_1 + r2_2)/2),
 // combined with tmp Y_m(j1), tmp = 0.5 dv / sqrt(2 pi sigma^2).  One CTA per
 // atom; the j2 points are staged through shared memory in tiles of 256 with
-// conj(Y) psi already formed, so each pair costs one exp and 12 FMAs.
+// conj(Y) psi already formed, so each pair costs one exp and 12 FMAs.  K
+// depends on the operator alone: a context that applies it many times keeps
+// K(j1, j2) of every atom (k_vso_kernel, k_vso_stored), and each pair costs
+// the 12 FMAs.
 // Kleinman-Bylander form (filterSpinors/hamiltonian.c:193-401): twelve
 // projections per atom (block reduction), scaled by Elkb dv, then spread back
 // over the atom's points with the reference's coefficients, term by term.
@@ -53,7 +56,7 @@ int fail(int status, const std::string& msg) {
 struct C2 {
   double re, im;
 };
-__device__ __forceinline__ C2 ld(const double* p) { return {p[0], p[1]}; }
+__device__ __forceinline__ C2 ld2(const double* p) { return {p[0], p[1]}; }
 // conj(y) psi, as the reference forms it (hamiltonian.c:139-140)
 __device__ __forceinline__ C2 conj_mul(C2 y, C2 p) {
   return {y.re * p.re + y.im * p.im, y.re * p.im - y.im * p.re};
@@ -67,6 +70,20 @@ __device__ __forceinline__ C2 sub(C2 a, C2 b) { return {a.re - b.re, a.im - b.im
 __device__ __forceinline__ void atomic_add(double* p, C2 v) {
   atomicAdd(p, v.re);
   atomicAdd(p + 1, v.im);
+}
+
+// Vso psi at one point from its six sums (hamiltonian.c:167-186), added to out
+__device__ __forceinline__ void vso_gauss_out(const sep_nlc& e, long ngrid, double tmp,
+                                              const C2 (&acc)[6], double* __restrict__ out) {
+  const double sqrttwo = sqrt(2.0);
+  const C2 t11 = scale(tmp, ld2(e.y11)), t10 = scale(tmp, ld2(e.y10)),
+           t1_1 = scale(tmp, ld2(e.y1_1));
+  const C2 up = add(sub(mul(t11, acc[0]), mul(t1_1, acc[2])),
+                    scale(sqrttwo, add(mul(t10, acc[3]), mul(t1_1, acc[4]))));
+  const C2 dn = add(sub(scale(-1.0, mul(t11, acc[3])), mul(t1_1, acc[5])),
+                    scale(sqrttwo, add(mul(t10, acc[2]), mul(t11, acc[1]))));
+  atomic_add(out + 2 * e.jxyz, up);
+  atomic_add(out + 2 * (ngrid + e.jxyz), dn);
 }
 
 // sums index: 0 y11 up, 1 y10 up, 2 y1_1 up, 3 y11 dn, 4 y10 dn, 5 y1_1 dn
@@ -83,7 +100,6 @@ __global__ void __launch_bounds__(kT) k_vso_gauss(const double* __restrict__ psi
   const long n = nl[a];
   const sep_nlc* base = nlc + a * nnlc;
   const int tid = threadIdx.x;
-  const double sqrttwo = sqrt(2.0);
   for (long j1b = 0; j1b < n; j1b += kT) {
     const long j1 = j1b + tid;
     const bool act = j1 < n;
@@ -101,8 +117,8 @@ __global__ void __launch_bounds__(kT) k_vso_gauss(const double* __restrict__ psi
       const long j2 = t0 + tid;
       if (j2 < n) {
         const sep_nlc& e = base[j2];
-        const C2 up = ld(psi + 2 * e.jxyz), dn = ld(psi + 2 * (ngrid + e.jxyz));
-        const C2 y11 = ld(e.y11), y10 = ld(e.y10), y1_1 = ld(e.y1_1);
+        const C2 up = ld2(psi + 2 * e.jxyz), dn = ld2(psi + 2 * (ngrid + e.jxyz));
+        const C2 y11 = ld2(e.y11), y10 = ld2(e.y10), y1_1 = ld2(e.y1_1);
         sr[tid] = e.r;
         sr2[tid] = e.r2;
         svr[tid] = e.Vr;
@@ -128,18 +144,84 @@ __global__ void __launch_bounds__(kT) k_vso_gauss(const double* __restrict__ psi
       }
     }
     if (act) {
-      const sep_nlc& e = base[j1];
-      const C2 t11 = scale(tmp, ld(e.y11)), t10 = scale(tmp, ld(e.y10)),
-               t1_1 = scale(tmp, ld(e.y1_1));
-      // hamiltonian.c:167-186
-      const C2 up = add(sub(mul(t11, acc[0]), mul(t1_1, acc[2])),
-                        scale(sqrttwo, add(mul(t10, acc[3]), mul(t1_1, acc[4]))));
-      const C2 dn = add(sub(scale(-1.0, mul(t11, acc[3])), mul(t1_1, acc[5])),
-                        scale(sqrttwo, add(mul(t10, acc[2]), mul(t11, acc[1]))));
-      atomic_add(out + 2 * e.jxyz, up);
-      atomic_add(out + 2 * (ngrid + e.jxyz), dn);
+      vso_gauss_out(base[j1], ngrid, tmp, acc, out);
     }
   }
+}
+
+// K(j1, j2) of every atom, km[(a nmax + j2) ld + j1], by the expression of
+// k_vso_gauss: once per operator
+__global__ void __launch_bounds__(kT) k_vso_kernel(long nnlc, const sep_nlc* __restrict__ nlc,
+                                                   const long* __restrict__ nl, double sigma_1,
+                                                   long nmax, long ld, double* __restrict__ km) {
+  const long a = blockIdx.x, n = nl[a];
+  const sep_nlc* base = nlc + a * nnlc;
+  const long j1 = (long)blockIdx.y * kT + threadIdx.x;
+  if (j1 >= n) return;
+  const double r1 = base[j1].r, r21 = base[j1].r2, vr1 = base[j1].Vr;
+  double* col = km + (size_t)a * nmax * ld + j1;
+  for (long j2 = 0; j2 < n; ++j2) {
+    const double d = (r1 - base[j2].r) * sigma_1;
+    col[(size_t)j2 * ld] =
+        0.5 * (vr1 + base[j2].Vr) * exp(-(d * d)) / (0.5 * (r21 + base[j2].r2));
+  }
+}
+
+// The Gaussian form with K read back: block (atom, 64 points j1, spinor).
+// Bound by the FP64 pipe: 12 FMAs per pair and spinor, where forming K costs
+// about 45 more FP64 operations.  Two warps a block, so that the points of an
+// atom spread over several SMs (one block per atom and spinor left most of
+// them with one or two blocks).  64 atoms x 340 points,
+// 4 spinors: 0.73 ms (12 FMAs per pair at the pipe's rate: 0.57 ms), 2.83 ms
+// forming K in place; K itself 0.79 ms once.
+constexpr int kTS = 64;
+__global__ void __launch_bounds__(kTS)
+    k_vso_stored(const double* __restrict__ psi, long ngrid, long nnlc,
+                 const sep_nlc* __restrict__ nlc, const long* __restrict__ nl,
+                 const double* __restrict__ km, long nmax, long ld, double tmp,
+                 double* __restrict__ out) {
+  __shared__ C2 sx[kTS][6];
+  const long a = blockIdx.x, n = nl[a];
+  if ((long)blockIdx.y * kTS >= n) return;
+  psi += (size_t)blockIdx.z * 4 * (size_t)ngrid;
+  out += (size_t)blockIdx.z * 4 * (size_t)ngrid;
+  const sep_nlc* base = nlc + a * nnlc;
+  const int tid = threadIdx.x;
+  const long j1 = (long)blockIdx.y * kTS + tid;
+  const bool act = j1 < n;
+  const double* kc = km + (size_t)a * nmax * ld + j1;
+  C2 acc[6];
+#pragma unroll
+  for (int m = 0; m < 6; ++m) acc[m] = {0.0, 0.0};
+  for (long t0 = 0; t0 < n; t0 += kTS) {
+    __syncthreads();
+    const long j2 = t0 + tid;
+    if (j2 < n) {
+      const sep_nlc& e = base[j2];
+      const C2 up = ld2(psi + 2 * e.jxyz), dn = ld2(psi + 2 * (ngrid + e.jxyz));
+      const C2 y11 = ld2(e.y11), y10 = ld2(e.y10), y1_1 = ld2(e.y1_1);
+      sx[tid][0] = conj_mul(y11, up);
+      sx[tid][1] = conj_mul(y10, up);
+      sx[tid][2] = conj_mul(y1_1, up);
+      sx[tid][3] = conj_mul(y11, dn);
+      sx[tid][4] = conj_mul(y10, dn);
+      sx[tid][5] = conj_mul(y1_1, dn);
+    }
+    __syncthreads();
+    if (act) {
+      const int cnt = (int)((n - t0) < kTS ? (n - t0) : kTS);
+#pragma unroll 4
+      for (int jj = 0; jj < cnt; ++jj) {
+        const double k = kc[(size_t)(t0 + jj) * ld];
+#pragma unroll
+        for (int m = 0; m < 6; ++m) {
+          acc[m].re += k * sx[jj][m].re;
+          acc[m].im += k * sx[jj][m].im;
+        }
+      }
+    }
+  }
+  if (act) vso_gauss_out(base[j1], ngrid, tmp, acc, out);
 }
 
 // projections p[g][m][s] (g: 0 G1, 1 G_2; m: 0 y10, 1 y11, 2 y1_1; s: 0 up, 1 dn)
@@ -161,8 +243,8 @@ __global__ void __launch_bounds__(kT) k_vso_kb(const double* __restrict__ psi, l
   for (int i = 0; i < 24; ++i) p[i] = 0.0;
   for (long j = tid; j < n; j += kT) {
     const sep_nlc& e = base[j];
-    const C2 s[2] = {ld(psi + 2 * e.jxyz), ld(psi + 2 * (ngrid + e.jxyz))};
-    const C2 y[3] = {ld(e.y10), ld(e.y11), ld(e.y1_1)};
+    const C2 s[2] = {ld2(psi + 2 * e.jxyz), ld2(psi + 2 * (ngrid + e.jxyz))};
+    const C2 y[3] = {ld2(e.y10), ld2(e.y11), ld2(e.y1_1)};
     const double g[2] = {e.Vs0G1, e.Vs0G_2};
 #pragma unroll
     for (int gi = 0; gi < 2; ++gi)
@@ -198,7 +280,7 @@ __global__ void __launch_bounds__(kT) k_vso_kb(const double* __restrict__ psi, l
   const double o6 = 1.0 / 6.0, o3 = 1.0 / 3.0, t3 = 2.0 / 3.0;
   for (long j = tid; j < n; j += kT) {
     const sep_nlc& e = base[j];
-    const C2 y10 = ld(e.y10), y11 = ld(e.y11), y1_1 = ld(e.y1_1);
+    const C2 y10 = ld2(e.y10), y11 = ld2(e.y11), y1_1 = ld2(e.y1_1);
     const double g1 = e.Vs0G1, g2 = e.Vs0G_2;
     // hamiltonian.c:318-353, in its order: G_2 terms, then G1 terms
     C2 up = scale(o6 * g2, mul(P(1, 2, 0), y1_1));
@@ -228,11 +310,24 @@ __global__ void __launch_bounds__(kT) k_vso_kb(const double* __restrict__ psi, l
 }  // namespace
 
 namespace sep {
+// K of every atom for spinor_vso_launch: natom x nmax x ld doubles, nmax the
+// largest list, ld >= nmax
+cudaError_t spinor_vso_kernel(long natom, long nnlc, const sep_nlc* nlc, const long* nl,
+                              double sigma, long nmax, long ld, double* km, cudaStream_t st) {
+  const long tiles = (nmax + kT - 1) / kT;
+  if (natom == 0 || nmax == 0) return cudaSuccess;
+  if (tiles > 65535) return cudaErrorInvalidValue;
+  k_vso_kernel<<<dim3((unsigned)natom, (unsigned)tiles), kT, 0, st>>>(
+      nnlc, nlc, nl, sqrt(0.5) / sigma, nmax, ld, km);  // init.c:97
+  return cudaGetLastError();
+}
 // Vso on nsp spinors (4 ngrid doubles apart) into psinl (zeroed first), on st;
-// the arguments are already checked.  nsp <= 65535.
+// the arguments are already checked.  nsp <= 65535.  km: the operator's K
+// (spinor_vso_kernel), or null: formed on the fly.
 cudaError_t spinor_vso_launch(const double* psi, long ngrid, long nsp, long natom, long nnlc,
                               const sep_nlc* nlc, const long* nl, double sigma, double dv,
-                              int flagkb, const double* elkb, double* psinl, cudaStream_t st) {
+                              int flagkb, const double* elkb, const double* km, long nmax,
+                              long ld, double* psinl, cudaStream_t st) {
   cudaError_t e = cudaMemsetAsync(psinl, 0, sizeof(double) * 4 * (size_t)ngrid * nsp, st);
   if (e != cudaSuccess || natom == 0) return e;
   const dim3 grid((unsigned)natom, (unsigned)nsp);
@@ -240,8 +335,13 @@ cudaError_t spinor_vso_launch(const double* psi, long ngrid, long nsp, long nato
     k_vso_kb<<<grid, kT, 0, st>>>(psi, ngrid, nnlc, nlc, nl, elkb, natom, dv, psinl);
   } else {
     const double tmp = 0.5 / sqrt(kTwoPi * (sigma * sigma)) * dv;  // hamiltonian.c:89
-    const double sigma_1 = sqrt(0.5) / sigma;                       // init.c:97
-    k_vso_gauss<<<grid, kT, 0, st>>>(psi, ngrid, nnlc, nlc, nl, tmp, sigma_1, psinl);
+    if (km) {
+      const dim3 g((unsigned)natom, (unsigned)((nmax + kTS - 1) / kTS), (unsigned)nsp);
+      k_vso_stored<<<g, kTS, 0, st>>>(psi, ngrid, nnlc, nlc, nl, km, nmax, ld, tmp, psinl);
+    } else {
+      const double sigma_1 = sqrt(0.5) / sigma;  // init.c:97
+      k_vso_gauss<<<grid, kT, 0, st>>>(psi, ngrid, nnlc, nlc, nl, tmp, sigma_1, psinl);
+    }
   }
   return cudaGetLastError();
 }
@@ -256,8 +356,8 @@ int sep_spinor_vso_dev(const double* psi, long ngrid, long natom, long nnlc, con
       (flagkb && !elkb) || (!flagkb && !(sigma > 0.0)))
     return fail(SEP_ERR_ARG, "sep_spinor_vso: bad arguments");
   cudaStream_t st = (cudaStream_t)cuda_stream;
-  SK(sep::spinor_vso_launch(psi, ngrid, 1, natom, nnlc, nlc, nl, sigma, dv, flagkb, elkb, psinl,
-                            st));
+  SK(sep::spinor_vso_launch(psi, ngrid, 1, natom, nnlc, nlc, nl, sigma, dv, flagkb, elkb,
+                            nullptr, 0, 0, psinl, st));
   return SEP_OK;
 }
 

@@ -146,3 +146,45 @@ def test_spinor_pipeline_library_eigensolver_matches_cusolver():
     assert out[0]["mkept"] == out[1]["mkept"]
     assert np.abs(out[0]["eval"] - out[1]["eval"]).max() <= 1e-10
     assert np.abs(out[0]["sigma"] - out[1]["sigma"]).max() <= 1e-8
+
+
+def _list_entries(rng, n, ngrid):
+    """n neighbour-list entries at random grid points, radii spread over (0.1, 2.6)."""
+    e = np.zeros(n, dtype=spinor.NLC_DTYPE)
+    e["jxyz"] = rng.choice(ngrid, n, replace=False)
+    for f in ("y10", "y11", "y1_1"):
+        e[f] = rng.normal(size=n) + 1j * rng.normal(size=n)
+    e["r"] = rng.uniform(0.1, 2.6, n)
+    e["r2"] = e["r"] ** 2
+    e["Vr"] = 0.1 * np.exp(-e["r2"] / 0.49)
+    return e
+
+
+@pytest.mark.parametrize("counts", [(1, 31, 32, 33, 0), (63, 64, 65, 128), (200, 3, 129),
+                                    (4096,) + (1,) * 299])
+def test_kept_kernel_equals_the_operator_applied_alone(counts):
+    """A context keeps the Gaussian form's K(j1, j2); sep_spinor_vso forms it in
+    place.  H with the operator less H without it is Vso psi: both take the same
+    products in the same order per atom, atoms add in any order, and H rounds
+    the sum once more (tolerance 1e-13 of the largest value of H psi).  Lists
+    around the 32- and 64-point tiles, an empty one, and one so long that the
+    atoms' K (40 GB) would take more than an eighth of the device's memory and
+    is not kept."""
+    rng = np.random.default_rng(sum(counts))
+    dims, h = (32, 32, 40), 0.5
+    ngrid = int(np.prod(dims))
+    nlc = np.zeros((len(counts), max(counts)), dtype=spinor.NLC_DTYPE)
+    for a, n in enumerate(counts):
+        nlc[a, :n] = _list_entries(rng, n, ngrid)
+    nl = np.array(counts, dtype=np.int64)
+    psi = rng.normal(size=(3, 2 * ngrid)) + 1j * rng.normal(size=(3, 2 * ngrid))
+    ctx = binding.Context(dims, (h, h, h), potl=np.zeros(ngrid), precision="f64", ekinmax=20.0)
+    full = spinor.SpinorPath(ctx, nlc, nl, sigma=h).hamiltonian(psi)
+    bare = spinor.SpinorPath(ctx, nlc, np.zeros_like(nl), sigma=h).hamiltonian(psi)
+    again = spinor.SpinorPath(ctx, nlc, nl, sigma=h).hamiltonian(psi)
+    ctx.close()
+    for s in range(3):
+        ref = spinor.nonlocal_potential(psi[s], nlc, nl, h, h ** 3)
+        assert np.abs(ref).max() > 0.0
+        for got in (full, again):
+            assert np.abs(got[s] - bare[s] - ref).max() <= 1e-13 * np.abs(full[s]).max()
