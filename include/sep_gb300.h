@@ -452,8 +452,8 @@ int sep_read_grid_source(const char *path, long *ngrid);
  * sep_bulk_solver_path: 2 when the library's batched solver ran, 1 when
  *   cuSOLVER's batched eigensolver ran, 0 when the matrices went to cuSOLVER
  *   one per call, -1 before the first solve.
- * sep_bulk_set_eigensolver: 1 (default) = the library's batched solver (one
- *   CTA per k-point, up to 512 plane waves; larger bases use cuSOLVER);
+ * sep_bulk_set_eigensolver: 1 (default) = the library's batched solver (a
+ *   cluster per k-point, up to 512 plane waves; larger bases use cuSOLVER);
  *   0 = cuSOLVER.
  * sep_bulk_set_solver: for cuSOLVER, 1 (default) = its batched eigensolver,
  *   one matrix per call where it declines the size; 0 = one matrix per call. */

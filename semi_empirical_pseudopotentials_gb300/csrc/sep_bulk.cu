@@ -12,7 +12,7 @@
 //      (hamiltonian.c:11-52), column-major nbv x nbv complex;
 //   3. finds the lowest nev (+ 16, for degenerate clusters that reach past
 //      band nev) eigenpairs of all nk matrices at once with the library's
-//      batched Hermitian solver (sep_heevb.cu: one CTA per matrix), in place
+//      batched Hermitian solver (sep_heevb.cu: a cluster per matrix), in place
 //      of one zheev per k-point (diag.c:12-48); cuSOLVER's batched routine
 //      (cusolverDnXsyevBatched, or Zheevd per matrix where it declines the
 //      size) stays selectable;

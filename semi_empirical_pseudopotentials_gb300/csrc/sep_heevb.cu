@@ -3,17 +3,17 @@
 // where the reference calls zheev for every k-point and keeps the lowest
 // bands, fit.c:86-88).
 //
-// One CTA per matrix (n <= 512, column-major, both triangles stored):
-//  1. k_hetrd: Householder reduction to real symmetric tridiagonal form with
-//     LAPACK zhetd2's conventions (lower triangle; H_j = I - tau_j v_j v_j^H
-//     with v_j(j+1) = 1 and a real beta_j, so T = Q^H A Q has a real
-//     diagonal d and off-diagonal e).  Per step: the reflector of the next
+// Per matrix (n <= 512, column-major, both triangles stored):
+//  1. k_hetrd (a cluster of blocks per matrix): Householder reduction to real
+//     symmetric tridiagonal form with LAPACK zhetd2's conventions (lower
+//     triangle; H_j = I - tau_j v_j v_j^H with v_j(j+1) = 1 and a real beta_j,
+//     so T = Q^H A Q has a real diagonal d and off-diagonal e).  Per step: the reflector of the next
 //     column, p = tau A22 v, w = p - (tau/2)(p^H v) v and the rank-2 update
 //     A22 -= v w^H + w v^H of the lower triangle.  Warps take columns (lanes
 //     on consecutive rows: coalesced); for p each column adds A_ik v_k to
 //     its rows' per-lane sums (scatter) and sum_{i>k} conj(A_ik) v_i to p_k
-//     (gather), and the warps' scatter sums are added in a fixed order, so
-//     the result does not depend on timing.  The reflectors stay below the
+//     (gather), and the sums of warps and blocks are added in a fixed order,
+//     so the result does not depend on timing.  The reflectors stay below the
 //     subdiagonal for the back-transformation.
 //  2. k_stebz: the lowest nw eigenvalues of T by bisection on Sturm counts
 //     (one thread per eigenvalue; the counts by the division-free continuant
@@ -26,7 +26,9 @@
 //  4. k_unmtr: x = H_0 H_1 ... H_{n-2} z for each vector (a warp per vector,
 //     the vector in registers).
 // On GB300 every FP64 operation goes through the FP64 pipe (about 2 FMAs per
-// clock per SM); the reduction costs 8 n^3 / 3 FMAs per matrix.
+// clock per SM); the reduction costs 8 n^3 / 3 FMAs per matrix, 35 ms on one
+// SM at n = 377.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -41,6 +43,7 @@ namespace sep {
 namespace hb {
 namespace {
 
+namespace cg = cooperative_groups;
 using Z = double2;
 constexpr int kWarps = 16;
 constexpr int kThreads = 32 * kWarps;
@@ -76,103 +79,162 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
+// sums over the warp of 8 values per lane, with 9 additions a lane instead of
+// 40 (on this part an FP64 warp instruction holds its sub-partition for 64
+// clocks): value q's total ends in the lanes with lane / 4 == q
+__device__ __forceinline__ double warp_sum8(const double (&x)[8], int lane) {
+  double a[4], b[2];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const bool up = lane & 16;
+    a[q] = (up ? x[4 + q] : x[q]) + __shfl_xor_sync(0xffffffffu, up ? x[q] : x[4 + q], 16);
+  }
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const bool up = lane & 8;
+    b[q] = (up ? a[2 + q] : a[q]) + __shfl_xor_sync(0xffffffffu, up ? a[q] : a[2 + q], 8);
+  }
+  const bool up = lane & 4;
+  double c = (up ? b[1] : b[0]) + __shfl_xor_sync(0xffffffffu, up ? b[0] : b[1], 4);
+  c += __shfl_xor_sync(0xffffffffu, c, 2);
+  return c + __shfl_xor_sync(0xffffffffu, c, 1);
+}
+
 // ---------------------------------------------------------------------------
-// 1. tridiagonal reduction; shared memory: v, w, p, gather sums (4 n complex)
-//    and the warps' scatter sums (kWarps x n complex)
-template <int MAXR>
+// 1. tridiagonal reduction: a cluster of G blocks per matrix.  Column k always
+//    belongs to warp k % (G kWarps) of the cluster, so a block reads and
+//    writes its own columns only, and the column that becomes the next
+//    reflector is the one thing every block reads (from L2).  Each block holds
+//    v, w and its part of A22 v in shared memory; the parts are added over
+//    distributed shared memory in block order, so every block has the same p.
+//    Two cluster barriers per step.  A warp takes kCols columns at a time:
+//    their products go into the rows' sums with one shared read and write, and
+//    their gather sums are reduced together (warp_sum8).  Bound by the FP64
+//    pipe (16 FMAs per element of the trailing triangle and step) and, for
+//    large G or small n, by the chain of each step (about 16 us).  42 matrices of
+//    377: 20.8 ms with clusters of 3, 55 ms with one block per matrix.
+//    shared memory: v, w, gather sums, this block's part (4 n complex) and the
+//    warps' scatter sums (kWarps x n complex)
+constexpr int kCols = 4;
+
 __global__ void __launch_bounds__(kThreads, 1)
-    k_hetrd(Z* __restrict__ Aall, int n, double* __restrict__ dall, double* __restrict__ eall,
-            Z* __restrict__ tauall) {
+    k_hetrd(Z* Aall, int n, int G, double* __restrict__ dall,
+            double* __restrict__ eall, Z* __restrict__ tauall) {
   extern __shared__ __align__(16) unsigned char hb_smem[];
+  const cg::cluster_group cluster = cg::this_cluster();
   Z* v = reinterpret_cast<Z*>(hb_smem);
   Z* w = v + n;
-  Z* gs = w + n;                 // gather part of p per column
-  Z* pw = gs + n;                // scatter parts: kWarps x n
+  Z* gs = w + n;                 // gather part of p per own column
+  Z* part = gs + n;              // this block's part of A22 v
+  Z* pw = part + n;              // scatter parts: kWarps x n
   __shared__ double red[2 * kWarps];
   __shared__ Z sh_tau, sh_scale;
   __shared__ int sh_skip;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  Z* A = Aall + (size_t)blockIdx.x * n * n;
-  double* d = dall + (size_t)blockIdx.x * n;
-  double* e = eall + (size_t)blockIdx.x * n;
-  Z* tau = tauall + (size_t)blockIdx.x * n;
+  const int rank = blockIdx.x % G, m = blockIdx.x / G;
+  const int stride = G * kWarps, own = rank * kWarps + warp;
+  Z* A = Aall + (size_t)m * n * n;
+  double* d = dall + (size_t)m * n;
+  double* e = eall + (size_t)m * n;
+  Z* tau = tauall + (size_t)m * n;
 
   for (int j = 0; j < n - 1; ++j) {
     const int r0 = j + 1;
-    // ---- reflector of column j (rows r0 .. n-1), warp 0
+    // ---- reflector of column j (rows r0 .. n-1), warp 0 of every block
     if (warp == 0) {
-      double part = 0.0;
+      double part2 = 0.0;
       for (int i = r0 + 1 + lane; i < n; i += 32) {
-        const Z x = A[(size_t)j * n + i];
-        part = fma(x.x, x.x, fma(x.y, x.y, part));
+        const Z x = __ldcg(&A[(size_t)j * n + i]);
+        part2 = fma(x.x, x.x, fma(x.y, x.y, part2));
       }
-      const double xn2 = warp_sum(part);
+      const double xn2 = warp_sum(part2);
       if (lane == 0) {
-        d[j] = A[(size_t)j * n + j].x;
-        const Z al = A[(size_t)j * n + r0];
+        const Z al = __ldcg(&A[(size_t)j * n + r0]);
+        double ej = al.x;
+        Z tj = zmk(0.0, 0.0);
         if (xn2 == 0.0 && al.y == 0.0) {  // already reduced: H_j = I
           sh_skip = 1;
-          e[j] = al.x;
-          tau[j] = zmk(0.0, 0.0);
         } else {
           const double beta = -copysign(sqrt(al.x * al.x + al.y * al.y + xn2), al.x);
-          const Z t = zmk((beta - al.x) / beta, -al.y / beta);
+          tj = zmk((beta - al.x) / beta, -al.y / beta);
           const double dx = al.x - beta, dy = al.y, dd = dx * dx + dy * dy;
           sh_scale = zmk(dx / dd, -dy / dd);  // 1 / (alpha - beta)
-          sh_tau = t;
+          sh_tau = tj;
           sh_skip = 0;
-          e[j] = beta;
-          tau[j] = t;
+          ej = beta;
+        }
+        if (rank == 0) {
+          d[j] = __ldcg(&A[(size_t)j * n + j]).x;
+          e[j] = ej;
+          tau[j] = tj;
         }
       }
     }
     __syncthreads();
-    if (sh_skip) {  // uniform; the barrier keeps sh_skip until every thread has read it
+    if (sh_skip) {  // the same in every block; the barrier keeps sh_skip until every thread has read it
       __syncthreads();
       continue;
     }
     const Z sc = sh_scale, tj = sh_tau;
-    for (int i = r0 + tid; i < n; i += kThreads) {
-      Z vi = zmk(1.0, 0.0);
-      if (i > r0) {
-        vi = zmul(A[(size_t)j * n + i], sc);
-        A[(size_t)j * n + i] = vi;  // kept for the back-transformation
-      }
-      v[i] = vi;
-    }
-    __syncthreads();
-    // ---- p = tau A22 v: warps on columns k, lanes on rows i >= k (each FP64
-    // instruction of the loop has every lane working: on this part an FP64
-    // warp instruction costs the same however many lanes are active); the
-    // scatter sums of each warp in shared memory
+    for (int i = r0 + tid; i < n; i += kThreads)
+      v[i] = i > r0 ? zmul(__ldcg(&A[(size_t)j * n + i]), sc) : zmk(1.0, 0.0);
     Z* mine = pw + (size_t)warp * n;
     for (int i = r0 + lane; i < n; i += 32) mine[i] = zmk(0.0, 0.0);
-    __syncwarp();
-    for (int k = r0 + warp; k < n; k += kWarps) {
-      const Z vk = v[k];
-      const Z* col = A + (size_t)k * n;
-      Z g = zmk(0.0, 0.0);
-      for (int i = k + lane; i < n; i += 32) {
-        const Z a = col[i];
-        mine[i] = zfma(a, vk, mine[i]);
-        if (i > k) g = zfmac(a, v[i], g);
+    __syncthreads();
+    const int kfirst = r0 + ((own - r0) % stride + stride) % stride;
+    // ---- this block's part of A22 v: warps on columns k, lanes on rows i >= k
+    // in groups of 32 that end at the last row
+    for (int k = kfirst; k < n; k += kCols * stride) {
+      Z vk[kCols];
+      double g[2 * kCols];
+#pragma unroll
+      for (int c = 0; c < kCols; ++c) {
+        vk[c] = k + c * stride < n ? v[k + c * stride] : zmk(0.0, 0.0);
+        g[2 * c] = g[2 * c + 1] = 0.0;
       }
-      g.x = warp_sum(g.x);
-      g.y = warp_sum(g.y);
-      if (lane == 0) gs[k] = g;
+      for (int i0 = n - (n - k + 31) / 32 * 32; i0 < n; i0 += 32) {
+        const int i = i0 + lane;
+        const bool in = i >= k;
+        const Z vi = in ? v[i] : zmk(0.0, 0.0);
+        Z s = in ? mine[i] : zmk(0.0, 0.0);
+#pragma unroll
+        for (int c = 0; c < kCols; ++c) {
+          const int kc = k + c * stride;
+          if (kc < n && i0 + 31 >= kc) {  // uniform: some row of the group lies in column kc
+            const Z a = i >= kc ? A[(size_t)kc * n + i] : zmk(0.0, 0.0);
+            s = zfma(a, vk[c], s);
+            const Z b = i > kc ? a : zmk(0.0, 0.0);
+            const Z q = zfmac(b, vi, zmk(g[2 * c], g[2 * c + 1]));
+            g[2 * c] = q.x;
+            g[2 * c + 1] = q.y;
+          }
+        }
+        if (in) mine[i] = s;
+      }
+      const double t = warp_sum8(g, lane);
+      const int kc = k + (lane >> 3) * stride;
+      if ((lane & 3) == 0 && kc < n) reinterpret_cast<double*>(gs)[2 * kc + ((lane >> 2) & 1)] = t;
     }
     __syncthreads();
-    // p_i = tau (gather_i + sum_w scatter_w,i), then p^H v
-    double px = 0.0, py = 0.0;
     for (int i = r0 + tid; i < n; i += kThreads) {
-      Z s = gs[i];
+      Z s = i % stride / kWarps == rank ? gs[i] : zmk(0.0, 0.0);
 #pragma unroll
       for (int q = 0; q < kWarps; ++q) s = zadd(s, pw[(size_t)q * n + i]);
+      part[i] = s;
+    }
+    cluster.sync();  // every part is written, every block has read column j
+    // ---- p = tau A22 v, p^H v, w = p - (tau / 2) (p^H v) v, in every block
+    double px = 0.0, py = 0.0;
+    for (int i = r0 + tid; i < n; i += kThreads) {
+      Z s = *cluster.map_shared_rank(&part[i], 0);
+      for (int q = 1; q < G; ++q) s = zadd(s, *cluster.map_shared_rank(&part[i], q));
       const Z pi = zmul(tj, s);
       w[i] = pi;
       const Z c = zfmac(pi, v[i], zmk(0.0, 0.0));  // conj(p_i) v_i
       px += c.x;
       py += c.y;
+      if (j % stride / kWarps == rank && i > r0)
+        A[(size_t)j * n + i] = v[i];  // kept for the back-transformation
     }
     px = warp_sum(px);
     py = warp_sum(py);
@@ -191,21 +253,37 @@ __global__ void __launch_bounds__(kThreads, 1)
     const Z alpha = zmul(zmk(-0.5 * tj.x, -0.5 * tj.y), zmk(dx, dy));
     for (int i = r0 + tid; i < n; i += kThreads) w[i] = zfma(alpha, v[i], w[i]);
     __syncthreads();
-    // ---- A22 -= v w^H + w v^H, lower triangle (v_i, w_i from shared memory)
-    for (int k = r0 + warp; k < n; k += kWarps) {
-      const Z vk = v[k], wk = w[k];
-      Z* col = A + (size_t)k * n;
-      for (int i = k + lane; i < n; i += 32) {
-        Z a = zfnmsc(v[i], wk, col[i]);
-        a = zfnmsc(w[i], vk, a);
-        if (i == k) a.y = 0.0;  // the diagonal stays real
-        col[i] = a;
+    // ---- A22 -= v w^H + w v^H, lower triangle of the own columns
+    for (int k = kfirst; k < n; k += kCols * stride) {
+      Z vk[kCols], wk[kCols];
+#pragma unroll
+      for (int c = 0; c < kCols; ++c) {
+        const int kc = min(k + c * stride, n - 1);
+        vk[c] = v[kc];
+        wk[c] = w[kc];
+      }
+      for (int i0 = n - (n - k + 31) / 32 * 32; i0 < n; i0 += 32) {
+        const int i = i0 + lane;
+        const bool in = i >= k;
+        const Z vi = in ? v[i] : zmk(0.0, 0.0), wi = in ? w[i] : zmk(0.0, 0.0);
+#pragma unroll
+        for (int c = 0; c < kCols; ++c) {
+          const int kc = k + c * stride;
+          if (kc < n && i0 + 31 >= kc) {
+            Z* p = &A[(size_t)kc * n + i];
+            Z a = i >= kc ? *p : zmk(0.0, 0.0);
+            a = zfnmsc(vi, wk[c], a);
+            a = zfnmsc(wi, vk[c], a);
+            if (i == kc) a.y = 0.0;  // the diagonal stays real
+            if (i >= kc) *p = a;
+          }
+        }
       }
     }
-    __syncthreads();
+    cluster.sync();  // column j + 1 is final, the parts have been read
   }
-  if (tid == 0) {
-    d[n - 1] = A[(size_t)(n - 1) * n + n - 1].x;
+  if (tid == 0 && rank == 0) {
+    d[n - 1] = __ldcg(&A[(size_t)(n - 1) * n + n - 1]).x;
     e[n - 1] = 0.0;
   }
 }
@@ -494,20 +572,61 @@ __global__ void k_put_vectors(const Z* __restrict__ xall, int n, int nw, long nm
   }
 }
 
-template <int MAXR> size_t hetrd_smem(int n) { return (size_t)(3 + kWarps) * n * sizeof(Z); }
+size_t hetrd_smem(int n) { return (size_t)(4 + kWarps) * n * sizeof(Z); }
+
+// Blocks per matrix: the cluster size G of the least estimated time, the
+// number of rounds that nmat clusters need (the clusters of G that the device
+// holds at once, one block per SM) times the time of one, which falls as
+// 1 / G + 64 / n (measured, 42 or 20 matrices, whole band solve without
+// vectors: n = 377 G = 1 52.4 ms, 2 32.3, 3 25.8, 6 19.3, and 42 clusters of 4
+// need a second round: 40.2; n = 219 14.6, 10.3, 8.9, 7.8; n = 73 2.33, 2.13,
+// 2.08, 1.97).
+cudaError_t cluster_size(cudaLaunchConfig_t cfg, int n, int nmat, int* size) {
+  double best = 0.0;
+  *size = 1;
+  for (int g = 1; g <= 8; ++g) {
+    int active = 0;
+    cfg.gridDim = dim3((unsigned)g);
+    cfg.attrs[0].val.clusterDim.x = (unsigned)g;
+    const cudaError_t e = cudaOccupancyMaxActiveClusters(&active, k_hetrd, &cfg);
+    if (e != cudaSuccess) return e;
+    if (active < 1) continue;
+    const double t = (double)((nmat + active - 1) / active) * (1.0 / g + 64.0 / n);
+    if (g == 1 || t < best) {
+      best = t;
+      *size = g;
+    }
+  }
+  return cudaSuccess;
+}
+
+cudaError_t launch_hetrd(Z* A, int n, int nmat, const Work& wk, cudaStream_t s) {
+  // the limit is set to what the largest n needs, the same value from every
+  // thread: calls for different n may run at once from several host threads
+  cudaError_t e = cudaFuncSetAttribute(k_hetrd, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)hetrd_smem(512));
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = hetrd_smem(n);
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  int g = 1;
+  if ((e = cluster_size(cfg, n, nmat, &g)) != cudaSuccess) return e;
+  at[0].val.clusterDim.x = (unsigned)g;
+  cfg.gridDim = dim3((unsigned)(nmat * g));
+  return cudaLaunchKernelEx(&cfg, k_hetrd, A, n, g, wk.d, wk.e, wk.tau);
+}
 
 template <int MAXR>
 cudaError_t run_all(Z* A, int n, int nmat, int nw, bool vectors, double* w, const Work& wk,
                     cudaStream_t s) {
-  // the shared-memory limits are set to what the largest n of this
-  // instantiation needs, the same value from every thread: calls for
-  // different n may run at once from several host threads
-  const size_t smem = hetrd_smem<MAXR>(n);
-  cudaError_t e = cudaFuncSetAttribute(k_hetrd<MAXR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)hetrd_smem<MAXR>(32 * MAXR));
+  cudaError_t e = launch_hetrd(A, n, nmat, wk, s);
   if (e != cudaSuccess) return e;
-  k_hetrd<MAXR><<<nmat, kThreads, smem, s>>>(A, n, wk.d, wk.e, wk.tau);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
   k_stebz<<<nmat, 128, 2 * n * sizeof(double), s>>>(wk.d, wk.e, n, nw, w, wk.tnorm);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   if (!vectors) return cudaSuccess;

@@ -93,3 +93,29 @@ def test_bad_arguments():
         sep.hermitian_lowest(np.eye(600, dtype=complex), 4)
     with pytest.raises(sep.SepError):
         sep.hermitian_lowest(np.eye(10, dtype=complex), 11)
+
+
+@pytest.mark.parametrize("n,nmat", [(2, 1), (5, 3), (33, 1), (64, 2), (129, 1), (129, 40),
+                                    (200, 80), (257, 5), (512, 1)])
+def test_cluster_sizes(n, nmat):
+    """The reduction takes 1 to 8 blocks per matrix by n and nmat: eigenvalues
+    within 1e-12 of the largest and residuals within 1e-11, the bounds of the
+    tests above, where most warps of a cluster have no column, at a single
+    large matrix and with more matrices than clusters of two fit.  A third of
+    each matrix's rows is diagonal, so steps without a reflector occur."""
+    rng = np.random.default_rng(n + nmat)
+    a = rng.normal(size=(nmat, n, n)) + 1j * rng.normal(size=(nmat, n, n))
+    a = a + np.conj(np.transpose(a, (0, 2, 1)))
+    k = n // 3
+    diag = np.diagonal(a, axis1=1, axis2=2).copy()
+    a[:, :k, :] = 0.0
+    a[:, :, :k] = 0.0
+    a[:, np.arange(n), np.arange(n)] = diag
+    nw = min(n, 8)
+    w, v = sep.hermitian_lowest(a, nw)
+    for m in range(nmat):
+        ref = np.linalg.eigvalsh(a[m])
+        scale = np.abs(ref).max()
+        assert np.abs(w[m] - ref[:nw]).max() <= 1e-12 * scale
+        r = a[m] @ v[m] - v[m] * w[m]
+        assert np.abs(r).max() <= 1e-11 * scale
