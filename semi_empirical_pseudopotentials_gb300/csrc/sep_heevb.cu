@@ -15,8 +15,8 @@
 //     (gather), and the sums of warps and blocks are added in a fixed order,
 //     so the result does not depend on timing.  The reflectors stay below the
 //     subdiagonal for the back-transformation.
-//  2. k_stebz: the lowest nw eigenvalues of T by bisection on Sturm counts
-//     (one thread per eigenvalue; the counts by the division-free continuant
+//  2. k_stebz: the lowest nw eigenvalues of T by multisection on Sturm counts
+//     (four threads per eigenvalue; the counts by the division-free continuant
 //     recursion with exact power-of-two rescaling).
 //  3. k_stein: their eigenvectors by inverse iteration (LAPACK dstein's
 //     scheme): Gaussian elimination with partial pivoting of T - lambda I,
@@ -24,7 +24,7 @@
 //     orthogonalised against each other (modified Gram-Schmidt), eigenvalues
 //     inside a group closer than 10 eps |lambda| are moved apart by that much.
 //  4. k_unmtr: x = H_0 H_1 ... H_{n-2} z for each vector (a warp per vector,
-//     the vector in registers).
+//     the vector in shared memory).
 // On GB300 every FP64 operation goes through the FP64 pipe (about 2 FMAs per
 // clock per SM); the reduction costs 8 n^3 / 3 FMAs per matrix, 35 ms on one
 // SM at n = 377.
@@ -330,9 +330,17 @@ __device__ int sturm_count(const double* d, const double* e2, int n, double x) {
   return c;
 }
 
-// 2. lowest nw eigenvalues, one thread each; w[nw .. n-1] = NaN
-__global__ void k_stebz(const double* __restrict__ dall, const double* __restrict__ eall, int n,
-                        int nw, double* __restrict__ wall, double* __restrict__ tnorm) {
+// 2. lowest nw eigenvalues, kSect threads each; w[nw .. n-1] = NaN.  Every
+//    round the kSect threads count at the points that cut the interval into
+//    kSect + 1 parts, so an eigenvalue takes log2(kSect + 1) times fewer
+//    rounds of n dependent steps than bisection.  Bound by that chain: four
+//    points per round give a 377-row matrix's 32 eigenvalues one warp per
+//    sub-partition.  42 matrices of 377: 2.1 ms, 4.9 ms by bisection.
+constexpr int kSect = 4;
+
+__global__ void __launch_bounds__(kSect * kMaxWanted)
+    k_stebz(const double* __restrict__ dall, const double* __restrict__ eall, int n, int nw,
+            double* __restrict__ wall, double* __restrict__ tnorm) {
   extern __shared__ double sb[];
   double* d = sb;
   double* e2 = sb + n;
@@ -345,40 +353,56 @@ __global__ void k_stebz(const double* __restrict__ dall, const double* __restric
     e2[i] = (i < n - 1) ? eg[i] * eg[i] : 0.0;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (threadIdx.x < 32) {  // Gershgorin interval, |T|_1 and the largest e^2
     double lo = d[0], hi = d[0], emax = 0.0, onenrm = 0.0;
-    for (int i = 0; i < n; ++i) {
+    for (int i = threadIdx.x; i < n; i += 32) {
       const double r = (i > 0 ? fabs(eg[i - 1]) : 0.0) + (i < n - 1 ? fabs(eg[i]) : 0.0);
       lo = fmin(lo, d[i] - r);
       hi = fmax(hi, d[i] + r);
       onenrm = fmax(onenrm, fabs(d[i]) + r);
       emax = fmax(emax, e2[i]);
     }
-    const double span = fmax(hi - lo, DBL_MIN);
-    sh_lo = lo - 2.1 * DBL_EPSILON * span - 1e-300;
-    sh_hi = hi + 2.1 * DBL_EPSILON * span + 1e-300;
-    sh_piv = DBL_MIN * fmax(1.0, emax);
-    tnorm[blockIdx.x] = onenrm;
+    for (int o = 16; o > 0; o >>= 1) {
+      lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+      hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+      onenrm = fmax(onenrm, __shfl_xor_sync(0xffffffffu, onenrm, o));
+      emax = fmax(emax, __shfl_xor_sync(0xffffffffu, emax, o));
+    }
+    if (threadIdx.x == 0) {
+      const double span = fmax(hi - lo, DBL_MIN);
+      sh_lo = lo - 2.1 * DBL_EPSILON * span - 1e-300;
+      sh_hi = hi + 2.1 * DBL_EPSILON * span + 1e-300;
+      sh_piv = DBL_MIN * fmax(1.0, emax);
+      tnorm[blockIdx.x] = onenrm;
+    }
   }
   __syncthreads();
-  for (int t = threadIdx.x; t < n; t += blockDim.x) {
-    if (t >= nw) {
-      w[t] = __longlong_as_double(0x7ff8000000000000LL);  // NaN: not computed
-      continue;
+  for (int t = nw + threadIdx.x; t < n; t += blockDim.x)
+    w[t] = __longlong_as_double(0x7ff8000000000000LL);  // NaN: not computed
+  const int t = threadIdx.x / kSect, q = threadIdx.x % kSect;
+  double lo = sh_lo, hi = sh_hi;
+  bool done = t >= nw;
+  for (int it = 0; it < 200; ++it) {
+    // this thread's point; the interval is done when it is as short as the
+    // eigenvalue's precision or a point no longer lies inside it
+    const double x = lo + (hi - lo) * ((q + 1) * (1.0 / (kSect + 1)));
+    const bool last = hi - lo <= 2.0 * DBL_EPSILON * fmax(fabs(lo), fabs(hi)) + sh_piv ||
+                      x <= lo || x >= hi;
+    const unsigned over = __ballot_sync(0xffffffffu, last);
+    const int base = threadIdx.x & 31 & ~(kSect - 1);
+    done = done || ((over >> base) & ((1u << kSect) - 1u)) != 0;
+    if (__all_sync(0xffffffffu, done)) break;
+    const bool above = !done && sturm_count(d, e2, n, x) > t;  // eigenvalue t lies below x
+    const unsigned ab = (__ballot_sync(0xffffffffu, above) >> base) & ((1u << kSect) - 1u);
+    const int first = ab ? __ffs(ab) - 1 : kSect;  // the lowest point above eigenvalue t
+    const double xl = __shfl_sync(0xffffffffu, x, base + max(first - 1, 0));
+    const double xh = __shfl_sync(0xffffffffu, x, base + min(first, kSect - 1));
+    if (!done) {
+      if (first > 0) lo = xl;
+      if (first < kSect) hi = xh;
     }
-    double lo = sh_lo, hi = sh_hi;
-    for (int it = 0; it < 200; ++it) {
-      const double mid = 0.5 * (lo + hi);
-      if (hi - lo <= 2.0 * DBL_EPSILON * fmax(fabs(lo), fabs(hi)) + sh_piv || mid <= lo ||
-          mid >= hi)
-        break;
-      if (sturm_count(d, e2, n, mid) > t)
-        hi = mid;
-      else
-        lo = mid;
-    }
-    w[t] = 0.5 * (lo + hi);
   }
+  if (t < nw && q == 0) w[t] = 0.5 * (lo + hi);
 }
 
 // ---------------------------------------------------------------------------
@@ -523,42 +547,44 @@ __global__ void __launch_bounds__(kSteinThreads)
 }
 
 // ---------------------------------------------------------------------------
-// 4. X = Q Z: warps on vectors, the vector in shared memory, lanes on the
-//    rows of each reflector
-template <int MAXR>
-__global__ void __launch_bounds__(kThreads)
+// 4. X = Q Z: warps on vectors, the vector in shared memory, lanes on the rows
+//    of each reflector.  Blocks of 4 vectors: bound by the FP64 pipe (8 FMAs
+//    per row and reflector) once a crystal's vectors cover every SM, which one
+//    block per matrix did not (42 matrices of 377, 32 vectors each: 2.7 ms, 7.3 ms
+//    with one block of 16 warps per matrix)
+constexpr int kUnWarps = 4;
+
+__global__ void __launch_bounds__(32 * kUnWarps)
     k_unmtr(const Z* __restrict__ Aall, const Z* __restrict__ tauall,
             const double* __restrict__ zall, int n, int nw, Z* __restrict__ xall) {
   extern __shared__ __align__(16) unsigned char hb_smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int m = blockIdx.x;
+  const int m = blockIdx.x, c = blockIdx.y * kUnWarps + warp;
+  if (c >= nw) return;
   const Z* A = Aall + (size_t)m * n * n;
   const Z* tau = tauall + (size_t)m * n;
   Z* x = reinterpret_cast<Z*>(hb_smem) + (size_t)warp * n;
-  for (int c = warp; c < nw; c += kWarps) {
-    const double* z = zall + ((size_t)m * nw + c) * n;
-    for (int i = lane; i < n; i += 32) x[i] = zmk(z[i], 0.0);
-    __syncwarp();
-    for (int j = n - 2; j >= 0; --j) {
-      const Z tj = tau[j];
-      if (tj.x == 0.0 && tj.y == 0.0) continue;
-      const Z* col = A + (size_t)j * n;
-      Z s = zmk(0.0, 0.0);  // v^H x
-      for (int i = j + 1 + lane; i < n; i += 32)
-        s = zfmac(i == j + 1 ? zmk(1.0, 0.0) : col[i], x[i], s);
-      s.x = warp_sum(s.x);
-      s.y = warp_sum(s.y);
-      const Z f = zmul(tj, s);
-      for (int i = j + 1 + lane; i < n; i += 32) {
-        const Z vi = (i == j + 1) ? zmk(1.0, 0.0) : col[i];
-        x[i] = zfnms(f, vi, x[i]);
-      }
-      __syncwarp();
+  const double* z = zall + ((size_t)m * nw + c) * n;
+  for (int i = lane; i < n; i += 32) x[i] = zmk(z[i], 0.0);
+  __syncwarp();
+  for (int j = n - 2; j >= 0; --j) {
+    const Z tj = tau[j];
+    if (tj.x == 0.0 && tj.y == 0.0) continue;
+    const Z* col = A + (size_t)j * n;
+    Z s = zmk(0.0, 0.0);  // v^H x
+    for (int i = j + 1 + lane; i < n; i += 32)
+      s = zfmac(i == j + 1 ? zmk(1.0, 0.0) : col[i], x[i], s);
+    s.x = warp_sum(s.x);
+    s.y = warp_sum(s.y);
+    const Z f = zmul(tj, s);
+    for (int i = j + 1 + lane; i < n; i += 32) {
+      const Z vi = (i == j + 1) ? zmk(1.0, 0.0) : col[i];
+      x[i] = zfnms(f, vi, x[i]);
     }
-    Z* xo = xall + ((size_t)m * nw + c) * n;
-    for (int i = lane; i < n; i += 32) xo[i] = x[i];
     __syncwarp();
   }
+  Z* xo = xall + ((size_t)m * nw + c) * n;
+  for (int i = lane; i < n; i += 32) xo[i] = x[i];
 }
 
 // the vectors into the first nw columns of each matrix
@@ -622,24 +648,19 @@ cudaError_t launch_hetrd(Z* A, int n, int nmat, const Work& wk, cudaStream_t s) 
   return cudaLaunchKernelEx(&cfg, k_hetrd, A, n, g, wk.d, wk.e, wk.tau);
 }
 
-template <int MAXR>
 cudaError_t run_all(Z* A, int n, int nmat, int nw, bool vectors, double* w, const Work& wk,
                     cudaStream_t s) {
   cudaError_t e = launch_hetrd(A, n, nmat, wk, s);
   if (e != cudaSuccess) return e;
-  k_stebz<<<nmat, 128, 2 * n * sizeof(double), s>>>(wk.d, wk.e, n, nw, w, wk.tnorm);
+  k_stebz<<<nmat, (kSect * nw + 31) / 32 * 32, 2 * n * sizeof(double), s>>>(wk.d, wk.e, n, nw, w, wk.tnorm);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   if (!vectors) return cudaSuccess;
   if ((e = cudaMemsetAsync(wk.info, 0, sizeof(int) * nmat, s)) != cudaSuccess) return e;
   k_stein<<<nmat, kSteinThreads, 0, s>>>(wk.d, wk.e, w, wk.tnorm, n, nw, wk.z, wk.scratch,
                                          wk.info);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  const size_t usmem = (size_t)kWarps * n * sizeof(Z);
-  if ((e = cudaFuncSetAttribute(k_unmtr<MAXR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)((size_t)kWarps * 32 * MAXR * sizeof(Z)))) != cudaSuccess)
-    return e;
-  k_unmtr<MAXR><<<nmat, kThreads, usmem, s>>>(A, wk.tau, wk.z, n, nw, wk.x);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  k_unmtr<<<dim3((unsigned)nmat, (unsigned)((nw + kUnWarps - 1) / kUnWarps)), 32 * kUnWarps,
+            (size_t)kUnWarps * n * sizeof(Z), s>>>(A, wk.tau, wk.z, n, nw, wk.x);
   const long tot = (long)nmat * n * nw;
   k_put_vectors<<<(unsigned)std::min<long>((tot + 255) / 256, 152L * 16), 256, 0, s>>>(
       wk.x, n, nw, nmat, A);
@@ -685,9 +706,7 @@ cudaError_t lowest(Z* A, int n, int nmat, int nw, bool vectors, double* w, void*
                    cudaStream_t s) {
   if (!supported(n, nw) || nmat < 1) return cudaErrorInvalidValue;
   const Work wk = carve(work, n, nmat, nw);
-  if (n <= 128) return run_all<4>(A, n, nmat, nw, vectors, w, wk, s);
-  if (n <= 256) return run_all<8>(A, n, nmat, nw, vectors, w, wk, s);
-  return run_all<16>(A, n, nmat, nw, vectors, w, wk, s);
+  return run_all(A, n, nmat, nw, vectors, w, wk, s);
 }
 
 cudaError_t failed_vectors(const void* work, int n, int nmat, int nw, int* host_count,
