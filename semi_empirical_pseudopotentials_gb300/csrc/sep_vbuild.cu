@@ -7,7 +7,9 @@
 // The reference loops over every atom for every point.  Here each block owns
 // a brick of grid points, keeps (in atom order) only the atoms whose table
 // range reaches the brick, and sums those; the dropped atoms contribute
-// exactly zero, so the per-point sum is the reference's, term for term.
+// exactly zero, so the per-point sum is the reference's, term for term.  What
+// the pairs of a segment, or of a brick and an atom, have in common is formed
+// once, by the same operations.
 // Products and sums are issued with explicit round-to-nearest intrinsics so
 // the compiler cannot contract them into FMAs: the result is bit-identical to
 // the reference's C loop.
@@ -39,8 +41,11 @@ using namespace sep;
 
 namespace {
 
-constexpr int BX = 8, BY = 8, BZ = 4;  // 256 points per block
-constexpr int kListCap = 2048;         // atoms kept per round
+constexpr int BX = 8, BY = 8, BZ = 8;  // points per brick
+constexpr int kNT = 128;               // threads per block, four z points each
+constexpr int kPZ = 4;
+constexpr int kListCap = 512;          // atoms kept per round
+constexpr int kTile = 64;              // atoms whose squares are in shared memory at once
 
 struct VArgs {
   const double* xyz;     // natom x 3
@@ -50,29 +55,42 @@ struct VArgs {
   const double* tab_v;
   const long* tab_n;
   const double* rcut;    // ntype: (n - 1) * dr, beyond which the table gives 0
+  double2* seg;          // ntype x stride, made by k_segments
   long long natom;
   long long stride;
   const double* vx;      // axis coordinates (running sums, filter/init.c:157-159)
   const double* vy;
   const double* vz;
   int nx, ny, nz;
-  double rcut_max;
 };
 
-__device__ __forceinline__ double seg_value(double r, const double* tr, const double* tv,
-                                            long n, double s, bool scaled) {
-  const double dr = __dadd_rn(tr[1], -tr[0]);
-  const long i = (long)(r / dr);
-  if (i > n - 2) return 0.0;
-  double a, b;
-  if (scaled) {
-    a = __dmul_rn(s, __dadd_rn(tv[i + 1], -tv[i])) / __dadd_rn(tr[i + 1], -tr[i]);
-    b = __dadd_rn(__dmul_rn(s, tv[i]), -__dmul_rn(tr[i], a));
-  } else {
-    a = __dadd_rn(tv[i + 1], -tv[i]) / __dadd_rn(tr[i + 1], -tr[i]);
-    b = __dadd_rn(tv[i], -__dmul_rn(tr[i], a));
+// What a pair needs of table segment i, once per call: the line (a, b) of the
+// forward (filter/interpolate.c:11-23), or (r_i, 1 / (r_{i+1} - r_i)) of the
+// backward
+__global__ void k_segments(VArgs v, long ntype, int backward) {
+  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < ntype * v.stride;
+       q += (long long)gridDim.x * blockDim.x) {
+    const long t = (long)(q / v.stride), i = (long)(q - t * v.stride);
+    if (i > v.tab_n[t] - 2) continue;
+    const double* tr = v.tab_r + t * v.stride;
+    const double* tv = v.tab_v + t * v.stride;
+    if (backward) {
+      v.seg[q] = make_double2(tr[i], 1.0 / (tr[i + 1] - tr[i]));
+    } else {
+      const double a = __dadd_rn(tv[i + 1], -tv[i]) / __dadd_rn(tr[i + 1], -tr[i]);
+      v.seg[q] = make_double2(a, __dadd_rn(tv[i], -__dmul_rn(tr[i], a)));
+    }
   }
-  return __dadd_rn(__dmul_rn(a, r), b);
+}
+
+// (long)(r / dr) of the reference, -1 beyond segment n - 2, from q = r / dr in
+// FP32 (sqrtf of r^2: within 3e-7 relative) unless that leaves the integer
+// open: then the division itself.
+__device__ __forceinline__ long segment(float q, double r, double dr, long n) {
+  const float i = truncf(q), f = q - i, e = 4e-7f * q + 1e-30f;
+  if (f > e && f < 1.0f - e) return (long)i > n - 2 ? -1 : (long)i;
+  const long k = (long)(r / dr);
+  return k > n - 2 ? -1 : k;
 }
 
 // distance from point p to the interval [lo, hi] along one axis
@@ -80,10 +98,10 @@ __device__ __forceinline__ double gap(double p, double lo, double hi) {
   return p < lo ? lo - p : (p > hi ? p - hi : 0.0);
 }
 
-// in-order compaction of the atoms of one 256-atom chunk that can reach the brick
+// in-order compaction of the atoms of one kNT-atom chunk that can reach the brick
 __device__ int collect(const VArgs& a, long long a0, double bx0, double bx1, double by0,
                        double by1, double bz0, double bz1, int* list, int base) {
-  __shared__ int warp_tot[8];
+  __shared__ int warp_tot[kNT / 32];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const long long ai = a0 + tid;
   bool keep = false;
@@ -98,7 +116,7 @@ __device__ int collect(const VArgs& a, long long a0, double bx0, double bx1, dou
   if (lane == 0) warp_tot[w] = __popc(m);
   __syncthreads();
   int off = 0, tot = 0;
-  for (int k = 0; k < 8; ++k) {
+  for (int k = 0; k < kNT / 32; ++k) {
     if (k < w) off += warp_tot[k];
     tot += warp_tot[k];
   }
@@ -107,103 +125,145 @@ __device__ int collect(const VArgs& a, long long a0, double bx0, double bx1, dou
   return tot;
 }
 
-__global__ void __launch_bounds__(256) k_vbuild(VArgs a, double* __restrict__ potl) {
-  __shared__ int list[kListCap + 256];
-  const int tx = threadIdx.x % BX, ty = (threadIdx.x / BX) % BY, tz = threadIdx.x / (BX * BY);
+// Calls body(u, d, atom, type, segment) in atom order for the four points u of
+// this thread (x, y, z0 + u of the brick) and every atom whose table reaches
+// them; d = |r_g - R_a| with the reference's roundings.  (x - X)^2, (y - Y)^2
+// and (z - Z)^2 take 24 values per atom and brick, which the block forms once,
+// so a pair costs one addition and the square root; a third of the pairs of a
+// brick lie beyond the table, which FP32 decides where all of a warp do.
+template <typename F> __device__ __forceinline__ void each_pair(const VArgs& a, F body) {
+  __shared__ int list[kListCap];
+  __shared__ double sq[kTile][BX + BY + BZ];
+  __shared__ int atom_type[kTile];
+  __shared__ double tab_dr[kTile];
+  __shared__ float tab_inv[kTile], tab_end[kTile];
+  const int tid = threadIdx.x;
+  const int x = tid % BX, y = tid / BX % BY, z0 = tid / (BX * BY) * kPZ;
   const int jx0 = blockIdx.x * BX, jy0 = blockIdx.y * BY, jz0 = blockIdx.z * BZ;
-  const int jx = jx0 + tx, jy = jy0 + ty, jz = jz0 + tz;
-  const bool inside = jx < a.nx && jy < a.ny && jz < a.nz;
   const int ex = min(jx0 + BX, a.nx) - 1, ey = min(jy0 + BY, a.ny) - 1,
             ez = min(jz0 + BZ, a.nz) - 1;
   const double bx0 = a.vx[jx0], bx1 = a.vx[ex], by0 = a.vy[jy0], by1 = a.vy[ey],
                bz0 = a.vz[jz0], bz1 = a.vz[ez];
-  const double px = inside ? a.vx[jx] : 0.0, py = inside ? a.vy[jy] : 0.0,
-               pz = inside ? a.vz[jz] : 0.0;
-  double sum = 0.0;
   long long a0 = 0;
   while (a0 < a.natom) {
     int cnt = 0;
     // fill the list with up to kListCap kept atoms, in atom order
-    while (a0 < a.natom && cnt <= kListCap - 256) {
+    while (a0 < a.natom && cnt <= kListCap - kNT) {
       cnt += collect(a, a0, bx0, bx1, by0, by1, bz0, bz1, list, cnt);
-      a0 += 256;
+      a0 += kNT;
     }
-    if (inside) {
-      for (int k = 0; k < cnt; ++k) {
-        const int ia = list[k];
-        const double dx = __dadd_rn(px, -a.xyz[3 * ia]);
-        const double dy = __dadd_rn(py, -a.xyz[3 * ia + 1]);
-        const double dz = __dadd_rn(pz, -a.xyz[3 * ia + 2]);
-        const double d = sqrt(__dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)),
-                                        __dmul_rn(dz, dz)));
-        const int t = a.types[ia];
-        sum = __dadd_rn(sum, seg_value(d, a.tab_r + t * a.stride, a.tab_v + t * a.stride,
-                                       a.tab_n[t], a.scale ? a.scale[ia] : 1.0,
-                                       a.scale != nullptr));
+    for (int c0 = 0; c0 < cnt; c0 += kTile) {
+      const int m = min(kTile, cnt - c0);
+      for (int q = tid; q < m * (BX + BY + BZ); q += kNT) {
+        const int k = q / (BX + BY + BZ), p = q - k * (BX + BY + BZ);
+        const long long ia = list[c0 + k];
+        const double at = p < BX        ? a.vx[min(jx0 + p, ex)]
+                          : p < BX + BY ? a.vy[min(jy0 + p - BX, ey)]
+                                        : a.vz[min(jz0 + p - BX - BY, ez)];
+        const double df = __dadd_rn(at, -a.xyz[3 * ia + (p < BX ? 0 : (p < BX + BY ? 1 : 2))]);
+        sq[k][p] = __dmul_rn(df, df);
+        if (p == 0) {
+          const int t = a.types[ia];
+          const double* tr = a.tab_r + t * a.stride;
+          const double dr = __dadd_rn(tr[1], -tr[0]);
+          atom_type[k] = t;
+          tab_dr[k] = dr;
+          tab_inv[k] = 1.0f / (float)dr;
+          tab_end[k] = (float)a.tab_n[t] * 1.00001f + 1.0f;
+        }
       }
+      __syncthreads();
+      for (int k = 0; k < m; ++k) {
+        const int t = atom_type[k];
+        const double dr = tab_dr[k];
+        const float inv = tab_inv[k], fn = tab_end[k];
+        const long n = a.tab_n[t];
+        const double xy = __dadd_rn(sq[k][x], sq[k][BX + y]);
+#pragma unroll
+        for (int u = 0; u < kPZ; ++u) {
+          const double d2 = __dadd_rn(xy, sq[k][BX + BY + z0 + u]);
+          const float q = sqrtf((float)d2) * inv;
+          if (q > fn && q < 1e30f) continue;  // past n - 1 by more than the rounding
+          const double d = sqrt(d2);
+          const long i = segment(q, d, dr, n);
+          if (i >= 0) body(u, d, list[c0 + k], t, i);
+        }
+      }
+      __syncthreads();
     }
-    __syncthreads();
   }
-  if (inside) potl[(long long)a.nx * ((long long)a.ny * jz + jy) + jx] = sum;
 }
 
-constexpr int kMaxTypesSmem = 4;
+// this thread's points inside the grid: offset of point u, or -1
+__device__ __forceinline__ long long point_of(const VArgs& a, int u) {
+  const int tid = threadIdx.x;
+  const int jx = blockIdx.x * BX + tid % BX, jy = blockIdx.y * BY + tid / BX % BY,
+            jz = blockIdx.z * BZ + tid / (BX * BY) * kPZ + u;
+  return jx < a.nx && jy < a.ny && jz < a.nz
+             ? (long long)a.nx * ((long long)a.ny * jz + jy) + jx
+             : -1;
+}
 
-__global__ void __launch_bounds__(256)
-k_vbuild_bwd(VArgs a, const double* __restrict__ dpotl, int ntype, int nbins_smem,
+// Bound by the FP64 pipe: a pair's sum, square root and line (about 16
+// operations; with the two divisions of the segment's line and of r / dr in
+// each pair, and a thread per point, about 45).  2260 atoms on 128^3, 310 M
+// pairs within the tables: 11.9 ms, 30.1 ms before.
+__global__ void __launch_bounds__(kNT) k_vbuild(VArgs a, double* __restrict__ potl) {
+  double sum[kPZ] = {};
+  each_pair(a, [&](int u, double d, int ia, int t, long i) {
+    double2 l;
+    if (a.scale) {  // filterStrainCube/interpolate.c:11-25
+      const double* tr = a.tab_r + t * a.stride;
+      const double* tv = a.tab_v + t * a.stride;
+      const double s = a.scale[ia];
+      l.x = __dmul_rn(s, __dadd_rn(tv[i + 1], -tv[i])) / __dadd_rn(tr[i + 1], -tr[i]);
+      l.y = __dadd_rn(__dmul_rn(s, tv[i]), -__dmul_rn(tr[i], l.x));
+    } else {
+      l = a.seg[t * a.stride + i];
+    }
+    sum[u] = __dadd_rn(sum[u], __dadd_rn(__dmul_rn(l.x, d), l.y));
+  });
+#pragma unroll
+  for (int u = 0; u < kPZ; ++u) {
+    const long long g = point_of(a, u);
+    if (g >= 0) potl[g] = sum[u];
+  }
+}
+
+// Bound by the FP64 pipe and by the two shared-memory additions of a pair.
+// The same case: 15.7 ms, 30.3 ms before.
+__global__ void __launch_bounds__(kNT)
+k_vbuild_bwd(VArgs a, const double* __restrict__ dpotl, int nbins_smem,
              double* __restrict__ dtab, double* __restrict__ dscale) {
   extern __shared__ double hist[];  // ntype * stride when it fits
-  __shared__ int list[kListCap + 256];
   const bool use_smem = nbins_smem > 0;
   for (int i = threadIdx.x; i < nbins_smem; i += blockDim.x) hist[i] = 0.0;
   __syncthreads();
-  const int tx = threadIdx.x % BX, ty = (threadIdx.x / BX) % BY, tz = threadIdx.x / (BX * BY);
-  const int jx0 = blockIdx.x * BX, jy0 = blockIdx.y * BY, jz0 = blockIdx.z * BZ;
-  const int jx = jx0 + tx, jy = jy0 + ty, jz = jz0 + tz;
-  const bool inside = jx < a.nx && jy < a.ny && jz < a.nz;
-  const int ex = min(jx0 + BX, a.nx) - 1, ey = min(jy0 + BY, a.ny) - 1,
-            ez = min(jz0 + BZ, a.nz) - 1;
-  const double bx0 = a.vx[jx0], bx1 = a.vx[ex], by0 = a.vy[jy0], by1 = a.vy[ey],
-               bz0 = a.vz[jz0], bz1 = a.vz[ez];
-  const double px = inside ? a.vx[jx] : 0.0, py = inside ? a.vy[jy] : 0.0,
-               pz = inside ? a.vz[jz] : 0.0;
-  const double gval =
-      inside ? dpotl[(long long)a.nx * ((long long)a.ny * jz + jy) + jx] : 0.0;
-  long long a0 = 0;
-  while (a0 < a.natom) {
-    int cnt = 0;
-    while (a0 < a.natom && cnt <= kListCap - 256) {
-      cnt += collect(a, a0, bx0, bx1, by0, by1, bz0, bz1, list, cnt);
-      a0 += 256;
-    }
-    if (inside && gval != 0.0) {
-      for (int k = 0; k < cnt; ++k) {
-        const int ia = list[k];
-        const double dx = px - a.xyz[3 * ia], dy = py - a.xyz[3 * ia + 1],
-                     dz = pz - a.xyz[3 * ia + 2];
-        const double d = sqrt(dx * dx + dy * dy + dz * dz);
-        const int t = a.types[ia];
-        const double* tr = a.tab_r + t * a.stride;
-        const double* tv = a.tab_v + t * a.stride;
-        const long n = a.tab_n[t];
-        const long i = (long)(d / (tr[1] - tr[0]));
-        if (i > n - 2) continue;
-        const double w = (d - tr[i]) / (tr[i + 1] - tr[i]);
-        const double s = a.scale ? a.scale[ia] : 1.0;
-        const double g0 = gval * s * (1.0 - w), g1 = gval * s * w;
-        const long long b = (long long)t * a.stride + i;
-        if (use_smem) {
-          atomicAdd(&hist[b], g0);
-          atomicAdd(&hist[b + 1], g1);
-        } else {
-          atomicAdd(&dtab[b], g0);
-          atomicAdd(&dtab[b + 1], g1);
-        }
-        if (dscale) atomicAdd(&dscale[ia], gval * ((1.0 - w) * tv[i] + w * tv[i + 1]));
-      }
-    }
-    __syncthreads();
+  double gval[kPZ];
+#pragma unroll
+  for (int u = 0; u < kPZ; ++u) {
+    const long long g = point_of(a, u);
+    gval[u] = g >= 0 ? dpotl[g] : 0.0;
   }
+  each_pair(a, [&](int u, double d, int ia, int t, long i) {
+    if (gval[u] == 0.0) return;
+    const long long b = (long long)t * a.stride + i;
+    const double2 l = a.seg[b];
+    const double w = (d - l.x) * l.y;
+    const double g = a.scale ? gval[u] * a.scale[ia] : gval[u];
+    const double g1 = g * w, g0 = g - g1;
+    if (use_smem) {
+      atomicAdd(&hist[b], g0);
+      atomicAdd(&hist[b + 1], g1);
+    } else {
+      atomicAdd(&dtab[b], g0);
+      atomicAdd(&dtab[b + 1], g1);
+    }
+    if (dscale) {
+      const double* tv = a.tab_v + t * a.stride;
+      atomicAdd(&dscale[ia], gval[u] * ((1.0 - w) * tv[i] + w * tv[i + 1]));
+    }
+  });
   __syncthreads();
   for (int i = threadIdx.x; i < nbins_smem; i += blockDim.x)
     if (hist[i] != 0.0) atomicAdd(&dtab[i], hist[i]);
@@ -211,12 +271,11 @@ k_vbuild_bwd(VArgs a, const double* __restrict__ dpotl, int ntype, int nbins_sme
 
 struct VHost {
   std::vector<double> vx, vy, vz, rcut;
-  double rmax = 0.0;
 };
 
 int prepare(sep_ctx* c, long natom, const double* xyz, const int* types, const double* scale,
             long ntype, const double* tab_r, const double* tab_v, const long* tab_n,
-            long stride, const double mins[3], VHost& h, VArgs& a, DevBuf& buf) {
+            long stride, const double mins[3], bool backward, VHost& h, VArgs& a, DevBuf& buf) {
   if (natom < 1 || ntype < 1 || stride < 2 || !xyz || !types || !tab_r || !tab_v || !tab_n ||
       !mins)
     return arg_fail("sep_vbuild: bad argument");
@@ -234,11 +293,10 @@ int prepare(sep_ctx* c, long natom, const double* xyz, const int* types, const d
       // i = (long)(r/dr) <= n - 2 needs r < (n - 1) dr
       const double dr = tab_r[t * stride + 1] - tab_r[t * stride];
       h.rcut[t] = (double)(n - 1) * dr;
-      h.rmax = std::max(h.rmax, h.rcut[t]);
     }
   }
   const size_t sz_xyz = 3 * (size_t)natom, sz_tab = (size_t)ntype * stride;
-  const size_t doubles = sz_xyz + (scale ? natom : 0) + 2 * sz_tab + ntype + c->nx + c->ny +
+  const size_t doubles = sz_xyz + (scale ? natom : 0) + 4 * sz_tab + ntype + c->nx + c->ny +
                          c->nz + 16;
   const size_t bytes = doubles * sizeof(double) + (size_t)natom * sizeof(int) +
                        (size_t)ntype * sizeof(long) + 256;
@@ -260,12 +318,15 @@ int prepare(sep_ctx* c, long natom, const double* xyz, const int* types, const d
   a.vz = (const double*)put(h.vz.data(), sizeof(double) * c->nz);
   a.types = (const int*)put(types, sizeof(int) * natom);
   a.tab_n = (const long*)put(tab_n, sizeof(long) * ntype);
+  a.seg = reinterpret_cast<double2*>(p);
   a.natom = natom;
   a.stride = stride;
   a.nx = (int)c->nx;
   a.ny = (int)c->ny;
   a.nz = (int)c->nz;
-  a.rcut_max = h.rmax;
+  CK(cudaGetLastError());
+  k_segments<<<(unsigned)std::min<size_t>((sz_tab + 255) / 256, 1024), 256, 0, c->stream>>>(
+      a, ntype, backward ? 1 : 0);
   CK(cudaGetLastError());
   return kOk;
 }
@@ -282,8 +343,8 @@ int sep_vbuild(sep_ctx* c, long natom, const double* xyz, const int* types, cons
   DevBuf in;
   VHost h;
   VArgs a;
-  int r = prepare(c, natom, xyz, types, scale, ntype, tab_r, tab_v, tab_n, tab_stride, mins, h,
-                  a, in);
+  int r = prepare(c, natom, xyz, types, scale, ntype, tab_r, tab_v, tab_n, tab_stride, mins,
+                  false, h, a, in);
   if (r != kOk) {
     in.release();
     return r;
@@ -296,7 +357,7 @@ int sep_vbuild(sep_ctx* c, long natom, const double* xyz, const int* types, cons
   }
   dim3 g((unsigned)((c->nx + BX - 1) / BX), (unsigned)((c->ny + BY - 1) / BY),
          (unsigned)((c->nz + BZ - 1) / BZ));
-  k_vbuild<<<g, 256, 0, c->stream>>>(a, d_pot);
+  k_vbuild<<<g, kNT, 0, c->stream>>>(a, d_pot);
   e = cudaGetLastError();
   if (e == cudaSuccess && potl)
     e = cudaMemcpyAsync(potl, d_pot, sizeof(double) * c->n, cudaMemcpyDeviceToHost, c->stream);
@@ -319,8 +380,8 @@ int sep_vbuild_backward(sep_ctx* c, long natom, const double* xyz, const int* ty
   DevBuf in;
   VHost h;
   VArgs a;
-  int r = prepare(c, natom, xyz, types, scale, ntype, tab_r, tab_v, tab_n, tab_stride, mins, h,
-                  a, in);
+  int r = prepare(c, natom, xyz, types, scale, ntype, tab_r, tab_v, tab_n, tab_stride, mins,
+                  true, h, a, in);
   if (r != kOk) {
     in.release();
     return r;
@@ -335,11 +396,11 @@ int sep_vbuild_backward(sep_ctx* c, long natom, const double* xyz, const int* ty
   if (e == cudaSuccess) e = cudaMemsetAsync(d_tab, 0, sizeof(double) * nb, c->stream);
   if (e == cudaSuccess && d_sc) e = cudaMemsetAsync(d_sc, 0, sizeof(double) * natom, c->stream);
   if (e == cudaSuccess) {
-    const int smem_bins = (nb * sizeof(double) <= 36 * 1024) ? (int)nb : 0;
+    const int smem_bins = (nb * sizeof(double) <= 32 * 1024) ? (int)nb : 0;  // beside 15 KB
     dim3 g((unsigned)((c->nx + BX - 1) / BX), (unsigned)((c->ny + BY - 1) / BY),
            (unsigned)((c->nz + BZ - 1) / BZ));
-    k_vbuild_bwd<<<g, 256, smem_bins * sizeof(double), c->stream>>>(a, d_g, (int)ntype,
-                                                                    smem_bins, d_tab, d_sc);
+    k_vbuild_bwd<<<g, kNT, smem_bins * sizeof(double), c->stream>>>(a, d_g, smem_bins, d_tab,
+                                                                    d_sc);
     e = cudaGetLastError();
   }
   if (e == cudaSuccess)

@@ -295,3 +295,52 @@ def test_fp64_refinement_reduces_residuals():
         ctx.close()
     assert np.abs(out[1][0] - ref_ev[win]).max() < 1e-8
     assert np.median(out[1][1]) < 0.1 * np.median(out[0][1]), (np.median(out[0][1]), np.median(out[1][1]))
+
+
+@pytest.mark.parametrize("dims", [(16, 16, 16), (14, 18, 20), (36, 24, 16)])
+@pytest.mark.parametrize("scaled", [False, True])
+def test_vbuild_at_segment_edges(dims, scaled):
+    """V(r) bit for bit where r / dr is at or one rounding from an integer
+    (atoms on grid points, the step a multiple of the table's), beyond the last
+    segment, and with bricks that the grid cuts; three types with tables of
+    1024, 300 and 2 entries.  With a scale, the oracle's per-atom factor."""
+    rng = np.random.default_rng(int(np.prod(dims)))
+    dr = 0.0251327412287
+    h = 16 * dr
+    ctx = sep.Context(dims, (h, h, h))
+    mins = [-0.5 * n * h for n in dims]
+    axes = []
+    for n, m in zip(dims, mins):
+        axes.append(np.cumsum(np.concatenate([[m], np.full(n - 1, h)])))
+    xyz = np.stack([rng.choice(axes[d], 40) for d in range(3)], axis=1)
+    xyz[30:] += rng.uniform(-1, 1, (10, 3))
+    types = rng.integers(0, 3, 40).astype(np.int32)
+    tab_r = np.cumsum(np.concatenate([[[0.0]] * 3, np.full((3, 1023), dr)], axis=1), axis=1)
+    tab_v = np.exp(-tab_r) * np.array([[-1.0], [2.0], [0.5]])
+    tab_n = [1024, 300, 2]
+    scale = rng.uniform(0.9, 1.1, 40) if scaled else None
+    got = ctx.vbuild(xyz, types, tab_r, tab_v, tab_n, mins, scale=scale)
+    ref = np.zeros(int(np.prod(dims)))
+    for g in range(len(ref)):
+        p = (axes[0][g % dims[0]], axes[1][g // dims[0] % dims[1]],
+             axes[2][g // (dims[0] * dims[1])])
+        for a in range(40):
+            d = [p[k] - xyz[a][k] for k in range(3)]
+            r = np.sqrt(d[0] * d[0] + d[1] * d[1] + d[2] * d[2])
+            t = types[a]
+            i = int(r / (tab_r[t][1] - tab_r[t][0]))
+            if i > tab_n[t] - 2:
+                continue
+            dv, dx = tab_v[t][i + 1] - tab_v[t][i], tab_r[t][i + 1] - tab_r[t][i]
+            s = scale[a] if scaled else 1.0
+            slope = s * dv / dx if scaled else dv / dx
+            ref[g] += slope * r + ((s * tab_v[t][i] if scaled else tab_v[t][i])
+                                   - tab_r[t][i] * slope)
+        if g > 1500:
+            break
+    assert np.array_equal(got[:1500], ref[:1500])
+    dtab, dsc = ctx.vbuild_backward(xyz, types, tab_r, tab_v, tab_n, mins,
+                                    rng.normal(size=len(got)), scale=scale)
+    assert np.all(np.isfinite(dtab)) and np.all(dtab[1, 300:] == 0.0)
+    assert np.all(dtab[2, 2:] == 0.0)
+    ctx.close()
