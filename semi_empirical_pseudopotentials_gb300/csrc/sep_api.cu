@@ -55,6 +55,10 @@ template <typename T> int upload_grid(sep_ctx* c, GridDev<T>& g) {
   const long lens[3] = {c->nx, c->ny, c->nz};
   for (int a = 0; a < 3; ++a) {
     std::vector<double> w = host::twiddles((int)lens[a]);
+    if (std::is_same<T, double>::value) {
+      const std::vector<double> f = host::folded_twiddles((int)lens[a]);
+      w.insert(w.end(), f.begin(), f.end());
+    }
     std::vector<T> wt(w.begin(), w.end());
     CK(cudaMalloc(&g.tw[a], sizeof(T) * wt.size()));
     CK(cudaMemcpy(g.tw[a], wt.data(), sizeof(T) * wt.size(), cudaMemcpyHostToDevice));

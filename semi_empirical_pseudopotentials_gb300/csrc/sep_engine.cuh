@@ -21,7 +21,7 @@ namespace sep {
 template <typename T> struct GridDev {
   int nx = 0, ny = 0, nz = 0;
   long long n = 0;
-  cx<T>* tw[3] = {nullptr, nullptr, nullptr};  // x, y, z twiddles
+  cx<T>* tw[3] = {nullptr, nullptr, nullptr};  // x, y, z twiddles (FP64: plain, then factored)
   T* kx = nullptr;
   T* ky = nullptr;
   T* kz = nullptr;

@@ -289,6 +289,19 @@ std::vector<double> twiddles(int L) {
   return w;
 }
 
+std::vector<double> folded_twiddles(int L) {
+  std::vector<double> w(2 * (size_t)L, 0.0);
+  if (L % 4 != 0) return w;
+  const long double half_pi = 1.5707963267948966192313216916397514421L;
+  for (int m = 0; m < L; ++m) {
+    const int q = (8 * m + L) / (2 * L);
+    const long double a = half_pi * (long double)(4 * m - q * L) / (long double)L;
+    w[2 * m] = (double)cosl(a);
+    w[2 * m + 1] = (double)tanl(a);
+  }
+  return w;
+}
+
 void form_factor_table(const double a[4], double vol_per_atom, double* r, double* v) {
   constexpr int n = 1024;
   const double dq = (5.0 - 0.0) / (double)n;

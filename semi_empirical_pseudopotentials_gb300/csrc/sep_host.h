@@ -41,6 +41,10 @@ void ksqr_grid(const KTables& t, long nx, long ny, long nz, double* ksqr);
 
 // exp(-2 pi i m / L) for m < L, as interleaved doubles (2L values)
 std::vector<double> twiddles(int L);
+// (cos, tan) of the angle of exp(-2 pi i m / L), m < L, less its nearest
+// multiple q = (8 m + L) / (2 L) of a quarter turn (all 0 when 4 does not
+// divide L), interleaved
+std::vector<double> folded_twiddles(int L);
 
 // pseudopotFitting/pot.c:35-63 + pseudopotFitting/hamiltonian.c:91-94
 void form_factor_table(const double a[4], double vol_per_atom, double* r, double* v);

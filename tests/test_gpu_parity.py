@@ -344,3 +344,27 @@ def test_vbuild_at_segment_edges(dims, scaled):
     assert np.all(np.isfinite(dtab)) and np.all(dtab[1, 300:] == 0.0)
     assert np.all(dtab[2, 2:] == 0.0)
     ctx.close()
+
+
+@pytest.mark.parametrize("dims", [(14, 16, 18), (20, 24, 32), (36, 40, 48), (56, 64, 72),
+                                  (80, 96, 14), (16, 112, 24), (18, 14, 128), (160, 20, 16),
+                                  (14, 192, 18), (16, 14, 256), (256, 16, 14), (32, 160, 192)])
+def test_fp64_transforms_of_every_length(dims):
+    """H psi in FP64 on grids that put every length on some axis, the ones whose
+    twiddles are folded into the second stage (splits with a factor 4, 8 or 16
+    on either side) and the others, against numpy's FFT.  Normwise bound of a
+    transform pair: about 5 u log2(N) = 1e-14 at 10^6 points, twice that here."""
+    rng = np.random.default_rng(int(sum(dims)))
+    nx, ny, nz = dims
+    n, h = nx * ny * nz, 0.7
+    pot = rng.normal(size=n)
+    psi = rng.normal(size=(3, n)) + 1j * rng.normal(size=(3, n))
+    ctx = sep.Context(dims, (h, h, h), potl=pot)
+    got = ctx.hamiltonian(psi)
+    ctx.close()
+    k = [0.5 * (2.0 * np.pi * np.fft.fftfreq(m, h)) ** 2 for m in dims]
+    t = np.minimum(k[2][:, None, None] + k[1][None, :, None] + k[0][None, None, :], 10.0)
+    for s in range(3):
+        g = psi[s].reshape(nz, ny, nx)
+        ref = np.fft.ifftn(np.fft.fftn(g) * t) + pot.reshape(nz, ny, nx) * g
+        assert np.linalg.norm(got[s] - ref.ravel()) <= 2e-14 * np.linalg.norm(ref)
