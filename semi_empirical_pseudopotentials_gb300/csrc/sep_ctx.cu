@@ -231,12 +231,16 @@ int filter_impl(sep_ctx* c, const double* d_start, long ns, const double* an_re,
   const long long B = (ns + 1) / 2;
   const size_t per_pair = sizeof(cx<T>) * (size_t)n * (size_t)(K + 1) +
                           sizeof(T) * accumulator_values<T>(n, ms);
-  const size_t have = c->w_hist.bytes + c->w_fft.bytes + c->w_acc.bytes;
-  size_t budget = (size_t)(0.6 * (double)free_device_bytes()) + have;
-  long long Bc = (long long)(budget / per_pair);
-  if (Bc < 1) return arg_fail("filter: not enough device memory for one pair of states");
-  if (Bc > B) Bc = B;
-  if (Bc > 65535) Bc = 65535;
+  long long Bc = std::min<long long>(B, 65535);
+  if (sizeof(cx<T>) * (size_t)n * K * Bc > c->w_hist.bytes ||
+      sizeof(cx<T>) * (size_t)n * Bc > c->w_fft.bytes ||
+      sizeof(T) * accumulator_values<T>(n, ms) * Bc > c->w_acc.bytes) {
+    // the workspace has to grow: as many pairs as the free memory holds
+    const size_t have = c->w_hist.bytes + c->w_fft.bytes + c->w_acc.bytes;
+    const size_t budget = (size_t)(0.6 * (double)free_device_bytes()) + have;
+    Bc = std::min(Bc, (long long)(budget / per_pair));
+    if (Bc < 1) return arg_fail("filter: not enough device memory for one pair of states");
+  }
   RET(grow(c, c->w_hist, sizeof(cx<T>) * (size_t)n * K * Bc));
   RET(grow(c, c->w_fft, sizeof(cx<T>) * (size_t)n * Bc));
   RET(grow(c, c->w_acc, sizeof(T) * accumulator_values<T>(n, ms) * Bc));
@@ -379,10 +383,15 @@ int filter_impl(sep_ctx* c, const double* d_start, long ns, const double* an_re,
 template <typename T>
 int apply_h_chunked_t(sep_ctx* c, const cx<T>* in, cx<T>* out, long long nst) {
   const long long n = c->n;
-  long long chunk = (long long)((0.25 * (double)free_device_bytes() + c->w_fft.bytes) /
-                                (sizeof(cx<T>) * (double)n));
-  if (chunk < 1) return arg_fail("hamiltonian: not enough device memory");
-  chunk = std::min<long long>(chunk, std::min<long long>(nst, 4096));
+  long long chunk = std::min<long long>(nst, 4096);
+  // the free memory is asked for only where the scratch has to grow: the query
+  // costs more than a small grid's passes
+  if (sizeof(cx<T>) * (size_t)n * chunk > c->w_fft.bytes) {
+    const long long fit = (long long)((0.25 * (double)free_device_bytes() + c->w_fft.bytes) /
+                                      (sizeof(cx<T>) * (double)n));
+    if (fit < 1) return arg_fail("hamiltonian: not enough device memory");
+    chunk = std::min(chunk, fit);
+  }
   RET(grow(c, c->w_fft, sizeof(cx<T>) * (size_t)n * chunk));
   for (long long b0 = 0; b0 < nst; b0 += chunk) {
     const int bc = (int)std::min<long long>(chunk, nst - b0);
