@@ -12,9 +12,9 @@ cudaError_t launch_sp(const PassArgs<float>& a, int B, cudaStream_t s) {
   using T = SpTune<L>;
   using S = SpShape<L, T::nt>;
   if (B < 1) return cudaErrorInvalidValue;
-  // min_blocks blocks per SM walk the units (grid, z, residue)
-  const long long units = (long long)B * S::n1y * a.nz;
-  const long long walkers = (long long)sm_count() * T::min_blocks;
+  // min_blocks (or few_blocks) blocks per SM walk the units (grid, z, residue)
+  const long long units = (long long)B * S::n1y * a.nz, sms = sm_count();
+  const long long walkers = sms * (units < 2 * sms * T::min_blocks ? T::few_blocks : T::min_blocks);
   const long long grid = units < walkers ? units : walkers;
   if (grid > 0x7fffffffLL) return cudaErrorInvalidValue;
   subplane_pass<L, MODE><<<(int)grid, T::nt, S::smem_bytes, s>>>(a, B);

@@ -36,33 +36,37 @@ namespace sep {
 // sub-plane pass launch shape per length: threads per block, blocks per SM,
 // whether the last stage of a unit runs with the first of the next (fastest
 // measured, step pass on 0.5 GB of grids, fraction of the copy bandwidth:
-// 96^2 0.83, 112^2 0.74, 128^2 0.84, 160^2 0.75, 192^2 0.84, 256^2 0.75)
+// 96^2 0.83, 112^2 0.78 (0.74 with 6 blocks per SM), 128^2 0.86, 160^2 0.76,
+// 192^2 0.86, 256^2 0.84 with two blocks and 248 registers (0.78 with three,
+// which spill))
+// few_blocks: blocks per SM that walk the units when they are less than two
+// rounds of min_blocks per SM (112^2 with 2 pairs: 23 us with 6, 25 with 8)
 template <int L> struct SpTune {
-  static constexpr int nt = 128, min_blocks = 4;
+  static constexpr int nt = 128, min_blocks = 4, few_blocks = 4;
   static constexpr bool fuse_next = true;
 };
 template <> struct SpTune<96> {
-  static constexpr int nt = 96, min_blocks = 5;
+  static constexpr int nt = 96, min_blocks = 5, few_blocks = 5;
   static constexpr bool fuse_next = true;
 };
 template <> struct SpTune<112> {
-  static constexpr int nt = 64, min_blocks = 6;
+  static constexpr int nt = 64, min_blocks = 8, few_blocks = 6;
   static constexpr bool fuse_next = true;
 };
 template <> struct SpTune<128> {  // 32-row sub-planes: the fused column stage spills
-  static constexpr int nt = 128, min_blocks = 4;
+  static constexpr int nt = 128, min_blocks = 4, few_blocks = 4;
   static constexpr bool fuse_next = false;
 };
 template <> struct SpTune<160> {
-  static constexpr int nt = 64, min_blocks = 6;
+  static constexpr int nt = 64, min_blocks = 6, few_blocks = 6;
   static constexpr bool fuse_next = true;
 };
 template <> struct SpTune<192> {
-  static constexpr int nt = 96, min_blocks = 4;
+  static constexpr int nt = 96, min_blocks = 4, few_blocks = 4;
   static constexpr bool fuse_next = true;
 };
 template <> struct SpTune<256> {
-  static constexpr int nt = 128, min_blocks = 3;
+  static constexpr int nt = 128, min_blocks = 2, few_blocks = 2;
   static constexpr bool fuse_next = true;
 };
 
@@ -90,17 +94,22 @@ template <int L, int NT> struct SpShape {
 // zy pass shape per length: TX adjacent columns per brick, threads per block,
 // blocks per SM.  A thread holds an R x 8 block (about 90 registers for
 // R = 4, 160 for R = 8); the brick is LZ x R TX elements (33 to 131 KB).
-// Fastest measured (zy pass on 0.5 GB of grids, fraction of the copy
-// bandwidth): 96^3 (R = 4) TX 8 0.75, 112^3 TX 8 0.64, 128^3 (R = 4) TX 8
-// 0.74, 160^3 TX 4 0.48, 192^3 TX 4 0.51, 256^3 TX 8 0.40.  With R = 8 the
-// pass is issue-bound (about 60 FP32 instructions per element for the two
-// 8-point y stages and the z transform pair) with 12 warps per SM; R = 4
-// needs no multiplies in its y stages and fits 20 warps per SM.
+// Fastest measured where the threads match the TX LZ / 8 items of the first
+// and last phase, so that no warp idles in them (zy pass on 0.5 GB of grids,
+// fraction of the copy bandwidth): 96^3 (R = 4) 0.77 (96 threads 0.81, but 2
+// to 4% slower with up to 4 pairs: 128 kept), 112^3 0.63, 128^3 (R = 4) 0.75, 160^3 TX 8 with 192 threads 0.55 (TX 4 with
+// 128: 0.48), 192^3 TX 4 0.51 (TX 8 0.46), 256^3 256 threads 0.49 (128: 0.40).
+// With R = 8 the pass is issue-bound (about 60 FP32 instructions per element
+// for the two 8-point y stages and the z transform pair) with 12 warps per SM;
+// R = 4 needs no multiplies in its y stages and fits 20 warps per SM.
 template <int L> struct ZyTune {
   static constexpr int tx = 8, nt = 128, min_blocks = 1;
 };
 template <> struct ZyTune<160> {
-  static constexpr int tx = 4, nt = 128, min_blocks = 1;
+  static constexpr int tx = 8, nt = 192, min_blocks = 1;
+};
+template <> struct ZyTune<256> {
+  static constexpr int tx = 8, nt = 256, min_blocks = 1;
 };
 template <> struct ZyTune<192> {
   static constexpr int tx = 4, nt = 128, min_blocks = 3;

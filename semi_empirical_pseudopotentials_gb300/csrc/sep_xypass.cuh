@@ -54,9 +54,11 @@ constexpr bool plane_pair(int lx, int ly) {
 // KB at 128^2).  Several blocks per SM let one block's transforms run while
 // another waits for memory; the shapes are the fastest measured per square
 // (step pass on 0.5 GB of grids, fraction of the copy bandwidth: 40^2 0.79,
-// 48^2 0.79, 56^2 0.75, 64^2 0.84, 72^2 0.79, 80^2 0.74, 96^2 0.76 against
+// 48^2 0.83, 56^2 0.75, 64^2 0.84, 72^2 0.79, 80^2 0.74, 96^2 0.76 against
 // 0.57 with one block of 512, 112^2 0.64, 128^2 0.73), and rectangles take
-// the shape of the squares of about their area.  Step (xy pass and z pass)
+// the shape of the squares of about their area; above 80^2 the best of 128 to
+// 512 threads (112 x 96 0.70 with two blocks of 192, 0.67 with 128; 128 x 112
+// 0.66 with one block of 384, 0.59 with 512, which spills).  Step (xy pass and z pass)
 // against the four line passes, measured over every pair: on 0.3 GB of grids
 // 80 x 64 0.329 against 0.527 ms, 64 x 48 0.334 against 0.504, 128 x 112 0.421
 // against 0.522, 32^2 0.310 against 0.497, 36^2 0.392 against 0.558, 14^2
@@ -64,19 +66,23 @@ constexpr bool plane_pair(int lx, int ly) {
 // against 18.5 us, 80 x 64 15.9 against 20.6, 128 x 96 27.2 against 30.9.
 template <int LX, int LY> struct XyTune {
   static constexpr int area = LX * LY;
-  static constexpr int nt = area <= 400    ? 32
-                            : area <= 2048 ? 64
-                            : (LX == 64 && LY == 64) ? 256
-                            : area <= 6400  ? 128
-                            : area <= 9216  ? 192
-                            : area <= 14000 ? 128
-                                            : 512;
-  static constexpr int min_blocks = area <= 400    ? 16
-                                    : area <= 2048 ? 8
-                                    : (LX == 64 && LY == 64) ? 3
-                                    : area <= 6400  ? 4
-                                    : area <= 14000 ? 2
-                                                    : 1;
+  static constexpr bool square = LX == LY;
+  static constexpr int nt = area <= 400            ? 32
+                            : area <= 2048         ? 64
+                            : square && LX == 48   ? 96
+                            : square && LX == 64   ? 256
+                            : area <= 6400         ? 128
+                            : square && LX == 112  ? 128
+                            : area <= 14000        ? 192
+                            : square               ? 512
+                                                   : 384;
+  static constexpr int min_blocks = area <= 400          ? 16
+                                    : area <= 2048       ? 8
+                                    : square && LX == 48 ? 6
+                                    : square && LX == 64 ? 3
+                                    : area <= 6400       ? 4
+                                    : area <= 14000      ? 2
+                                                         : 1;
 };
 
 template <int LX, int LY, int NT> struct XyShape {
