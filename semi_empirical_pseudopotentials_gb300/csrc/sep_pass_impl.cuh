@@ -18,9 +18,9 @@ cudaError_t launch_one(const PassArgs<T>& a, int B, cudaStream_t s) {
     if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
     grid = dim3((unsigned)blocks, 1, 1);
   } else {
-    const int other = (AXIS == 1) ? a.nz : a.ny;
+    const int lines = (AXIS == 1) ? a.nx : a.nx * a.ny, other = (AXIS == 1) ? a.nz : 1;
     if (other > 65535 || B > 65535) return cudaErrorInvalidValue;
-    grid = dim3((unsigned)((a.nx + TL - 1) / TL), (unsigned)other, (unsigned)B);
+    grid = dim3((unsigned)((lines + TL - 1) / TL), (unsigned)other, (unsigned)B);
   }
   line_pass<T, L, AXIS, MODE, V><<<grid, NT, 0, s>>>(a);
   return cudaGetLastError();
