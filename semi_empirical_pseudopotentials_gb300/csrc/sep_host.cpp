@@ -293,11 +293,20 @@ std::vector<double> folded_twiddles(int L) {
   std::vector<double> w(2 * (size_t)L, 0.0);
   if (L % 4 != 0) return w;
   const long double half_pi = 1.5707963267948966192313216916397514421L;
+  // the reduced angles are multiples of 2 pi / L in the half-quadrant: each is
+  // evaluated once (long double is software on some hosts)
+  const int half = L / 8;
+  std::vector<double> c((size_t)half + 1), t((size_t)half + 1);
+  for (int k = 0; k <= half; ++k) {
+    const long double a = half_pi * (long double)(4 * k) / (long double)L;
+    c[k] = (double)cosl(a);
+    t[k] = (double)tanl(a);
+  }
   for (int m = 0; m < L; ++m) {
     const int q = (8 * m + L) / (2 * L);
-    const long double a = half_pi * (long double)(4 * m - q * L) / (long double)L;
-    w[2 * m] = (double)cosl(a);
-    w[2 * m + 1] = (double)tanl(a);
+    const int k = m - q * (L / 4);  // |k| <= L / 8
+    w[2 * m] = c[k < 0 ? -k : k];
+    w[2 * m + 1] = k < 0 ? -t[-k] : t[k];
   }
   return w;
 }
