@@ -20,6 +20,8 @@
 // exchanges and no redistribution.
 #pragma once
 
+#include <type_traits>
+
 #include "sep_dft.cuh"
 
 namespace sep {
@@ -99,7 +101,18 @@ template <typename T, int L, int AXIS, int V = 0> struct Tile {
   static constexpr int tl_cap = (40 * 1024) / bytes_per_line;
   static constexpr int pow2_floor(int v) { return v >= 2 ? 2 * pow2_floor(v / 2) : 1; }
   static constexpr int tl = pow2_floor(tl_raw < tl_cap ? tl_raw : (tl_cap > 0 ? tl_cap : 1));
-  static constexpr int nt = tl * nmin;
+  // one item per thread in the stage with fewer of them, unless that leaves a
+  // part-filled warp (40, 56 and 160 lines of x, 18: the other stage's second
+  // round then runs mostly empty warps, which cost as much as full ones) or
+  // the two items of a 160-line's 16-point stage cost registers (FP64): one
+  // item per thread in the stage with more.  Sum of a Newton step's passes on
+  // 0.1 GB of grids, FP64: 56^3 3.52 -> 3.20 ms, 40^3 3.24 -> 3.04, 160^3 16.9
+  // -> 15.2; elsewhere fewer threads are as fast or faster (32^3 1.89 against
+  // 2.06, 48^3 2.53 against 2.63, 128^3 5.42 against 5.56).
+  static constexpr int nmax = n1 < n2 ? n2 : n1;
+  static constexpr bool wide =
+      (tl * nmin) % 32 != 0 || (std::is_same<T, double>::value && n1 == 10);
+  static constexpr int nt = tl * (wide ? nmax : nmin);
 };
 
 template <typename T, int L, int AXIS, int MODE, int V = 0>
