@@ -105,6 +105,8 @@ struct sep_ctx {
   bool so_ready = false;
   long so_kmax = 0, so_kld = 0;  // w_sok: natom x so_kmax x so_kld (0: K not kept)
   sep::DevBuf w_sok;  // the Gaussian form's kernel K(j1, j2) of every atom
+  sep::DevBuf w_sog;  // with it: off[n + 1], idx: the list points of each grid point
+  sep::DevBuf w_soc;  // the list points' contributions, 4 natom so_kmax doubles per spinor
   sep::DevBuf w_nlc, w_nl, w_elkb, w_so, w_so2, w_so3;
   sep::DevBuf w_eigh;  // workspace of the symmetric eigensolver
   sep::DevBuf w_hist, w_fft, w_acc, w_coef, w_steps, w_start, w_out, w_red, w_small,

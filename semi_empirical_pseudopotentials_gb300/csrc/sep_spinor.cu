@@ -15,11 +15,13 @@
 // conj(Y) psi already formed, so each pair costs one exp and 12 FMAs.  K
 // depends on the operator alone: a context that applies it many times keeps
 // K(j1, j2) of every atom (k_vso_kernel, k_vso_stored), and each pair costs
-// the 12 FMAs.
+// the 12 FMAs; there each list point's contribution is stored and a grid
+// point sums its own in list order (k_vso_gather).
 // Kleinman-Bylander form (filterSpinors/hamiltonian.c:193-401): twelve
 // projections per atom (block reduction), scaled by Elkb dv, then spread back
 // over the atom's points with the reference's coefficients, term by term.
-// Contributions of overlapping atoms are added with atomicAdd.
+// Contributions of overlapping atoms are added with atomicAdd in the
+// Kleinman-Bylander form and where K is formed in place.
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -72,18 +74,16 @@ __device__ __forceinline__ void atomic_add(double* p, C2 v) {
   atomicAdd(p + 1, v.im);
 }
 
-// Vso psi at one point from its six sums (hamiltonian.c:167-186), added to out
-__device__ __forceinline__ void vso_gauss_out(const sep_nlc& e, long ngrid, double tmp,
-                                              const C2 (&acc)[6], double* __restrict__ out) {
+// Vso psi at one point from its six sums (hamiltonian.c:167-186)
+__device__ __forceinline__ void vso_gauss_point(const sep_nlc& e, double tmp, const C2 (&acc)[6],
+                                                C2& up, C2& dn) {
   const double sqrttwo = sqrt(2.0);
   const C2 t11 = scale(tmp, ld2(e.y11)), t10 = scale(tmp, ld2(e.y10)),
            t1_1 = scale(tmp, ld2(e.y1_1));
-  const C2 up = add(sub(mul(t11, acc[0]), mul(t1_1, acc[2])),
-                    scale(sqrttwo, add(mul(t10, acc[3]), mul(t1_1, acc[4]))));
-  const C2 dn = add(sub(scale(-1.0, mul(t11, acc[3])), mul(t1_1, acc[5])),
-                    scale(sqrttwo, add(mul(t10, acc[2]), mul(t11, acc[1]))));
-  atomic_add(out + 2 * e.jxyz, up);
-  atomic_add(out + 2 * (ngrid + e.jxyz), dn);
+  up = add(sub(mul(t11, acc[0]), mul(t1_1, acc[2])),
+           scale(sqrttwo, add(mul(t10, acc[3]), mul(t1_1, acc[4]))));
+  dn = add(sub(scale(-1.0, mul(t11, acc[3])), mul(t1_1, acc[5])),
+           scale(sqrttwo, add(mul(t10, acc[2]), mul(t11, acc[1]))));
 }
 
 // sums index: 0 y11 up, 1 y10 up, 2 y1_1 up, 3 y11 dn, 4 y10 dn, 5 y1_1 dn
@@ -144,7 +144,10 @@ __global__ void __launch_bounds__(kT) k_vso_gauss(const double* __restrict__ psi
       }
     }
     if (act) {
-      vso_gauss_out(base[j1], ngrid, tmp, acc, out);
+      C2 up, dn;
+      vso_gauss_point(base[j1], tmp, acc, up, dn);
+      atomic_add(out + 2 * base[j1].jxyz, up);
+      atomic_add(out + 2 * (ngrid + base[j1].jxyz), dn);
     }
   }
 }
@@ -179,12 +182,12 @@ __global__ void __launch_bounds__(kTS)
     k_vso_stored(const double* __restrict__ psi, long ngrid, long nnlc,
                  const sep_nlc* __restrict__ nlc, const long* __restrict__ nl,
                  const double* __restrict__ km, long nmax, long ld, double tmp,
-                 double* __restrict__ out) {
+                 double2* __restrict__ contrib) {
   __shared__ C2 sx[kTS][6];
   const long a = blockIdx.x, n = nl[a];
   if ((long)blockIdx.y * kTS >= n) return;
   psi += (size_t)blockIdx.z * 4 * (size_t)ngrid;
-  out += (size_t)blockIdx.z * 4 * (size_t)ngrid;
+  contrib += (size_t)blockIdx.z * 2 * (size_t)gridDim.x * (size_t)nmax;
   const sep_nlc* base = nlc + a * nnlc;
   const int tid = threadIdx.x;
   const long j1 = (long)blockIdx.y * kTS + tid;
@@ -221,7 +224,42 @@ __global__ void __launch_bounds__(kTS)
       }
     }
   }
-  if (act) vso_gauss_out(base[j1], ngrid, tmp, acc, out);
+  if (act) {
+    C2 up, dn;
+    vso_gauss_point(base[j1], tmp, acc, up, dn);
+    double2* o = contrib + 2 * ((size_t)a * nmax + j1);
+    o[0] = make_double2(up.re, up.im);
+    o[1] = make_double2(dn.re, dn.im);
+  }
+}
+
+// Vso psi of every grid point from the list points' contributions: point g
+// sums the entries idx[off[g]] .. idx[off[g + 1] - 1] (a nmax + j, ascending),
+// so the result does not depend on the order in which blocks finish.  Added
+// atomically it did: three overlapping atoms change the last bit, and the
+// subspace steps keep directions down to 1e-10 of the largest, which turned
+// it into 1e-6 of the Ritz values of the states that are not converged.  It
+// writes every point (zero where no list reaches), so no memset goes before;
+// bound by that store.
+__global__ void __launch_bounds__(kT)
+    k_vso_gather(const double2* __restrict__ contrib, const int* __restrict__ off,
+                 const int* __restrict__ idx, long ngrid, long entries,
+                 double2* __restrict__ out) {
+  const long g = (long)blockIdx.x * kT + threadIdx.x;
+  if (g >= ngrid) return;
+  contrib += (size_t)blockIdx.y * 2 * (size_t)entries;
+  out += (size_t)blockIdx.y * 2 * (size_t)ngrid;
+  double2 up = make_double2(0.0, 0.0), dn = up;
+  const int end = off[g + 1];
+  for (int t = off[g]; t < end; ++t) {
+    const double2 u = contrib[2 * (size_t)idx[t]], d = contrib[2 * (size_t)idx[t] + 1];
+    up.x += u.x;
+    up.y += u.y;
+    dn.x += d.x;
+    dn.y += d.y;
+  }
+  out[g] = up;
+  out[ngrid + g] = dn;
 }
 
 // projections p[g][m][s] (g: 0 G1, 1 G_2; m: 0 y10, 1 y11, 2 y1_1; s: 0 up, 1 dn)
@@ -310,7 +348,7 @@ __global__ void __launch_bounds__(kT) k_vso_kb(const double* __restrict__ psi, l
 }  // namespace
 
 namespace sep {
-// K of every atom for spinor_vso_launch: natom x nmax x ld doubles, nmax the
+// K of every atom for spinor_vso_kept: natom x nmax x ld doubles, nmax the
 // largest list, ld >= nmax
 cudaError_t spinor_vso_kernel(long natom, long nnlc, const sep_nlc* nlc, const long* nl,
                               double sigma, long nmax, long ld, double* km, cudaStream_t st) {
@@ -321,13 +359,28 @@ cudaError_t spinor_vso_kernel(long natom, long nnlc, const sep_nlc* nlc, const l
       nnlc, nlc, nl, sqrt(0.5) / sigma, nmax, ld, km);  // init.c:97
   return cudaGetLastError();
 }
-// Vso on nsp spinors (4 ngrid doubles apart) into psinl (zeroed first), on st;
-// the arguments are already checked.  nsp <= 65535.  km: the operator's K
-// (spinor_vso_kernel), or null: formed on the fly.
+// The Gaussian form on nsp spinors (4 ngrid doubles apart) into psinl with the
+// operator's K (spinor_vso_kernel), on st.  off, idx: the list points of each
+// grid point (k_vso_gather); contrib: 4 natom nmax doubles per spinor.
+// 1 <= nsp <= 65535, natom, nmax >= 1.
+cudaError_t spinor_vso_kept(const double* psi, long ngrid, long nsp, long natom, long nnlc,
+                            const sep_nlc* nlc, const long* nl, double sigma, double dv,
+                            const double* km, long nmax, long ld, const int* off, const int* idx,
+                            double* contrib, double* psinl, cudaStream_t st) {
+  const double tmp = 0.5 / sqrt(kTwoPi * (sigma * sigma)) * dv;  // hamiltonian.c:89
+  const dim3 g((unsigned)natom, (unsigned)((nmax + kTS - 1) / kTS), (unsigned)nsp);
+  double2* cb = reinterpret_cast<double2*>(contrib);
+  k_vso_stored<<<g, kTS, 0, st>>>(psi, ngrid, nnlc, nlc, nl, km, nmax, ld, tmp, cb);
+  const dim3 gg((unsigned)((ngrid + kT - 1) / kT), (unsigned)nsp);
+  k_vso_gather<<<gg, kT, 0, st>>>(cb, off, idx, ngrid, natom * nmax,
+                                  reinterpret_cast<double2*>(psinl));
+  return cudaGetLastError();
+}
+// Vso on nsp spinors (4 ngrid doubles apart) into psinl (zeroed first), on st,
+// K formed in place; the arguments are already checked.  nsp <= 65535.
 cudaError_t spinor_vso_launch(const double* psi, long ngrid, long nsp, long natom, long nnlc,
                               const sep_nlc* nlc, const long* nl, double sigma, double dv,
-                              int flagkb, const double* elkb, const double* km, long nmax,
-                              long ld, double* psinl, cudaStream_t st) {
+                              int flagkb, const double* elkb, double* psinl, cudaStream_t st) {
   cudaError_t e = cudaMemsetAsync(psinl, 0, sizeof(double) * 4 * (size_t)ngrid * nsp, st);
   if (e != cudaSuccess || natom == 0) return e;
   const dim3 grid((unsigned)natom, (unsigned)nsp);
@@ -335,13 +388,8 @@ cudaError_t spinor_vso_launch(const double* psi, long ngrid, long nsp, long nato
     k_vso_kb<<<grid, kT, 0, st>>>(psi, ngrid, nnlc, nlc, nl, elkb, natom, dv, psinl);
   } else {
     const double tmp = 0.5 / sqrt(kTwoPi * (sigma * sigma)) * dv;  // hamiltonian.c:89
-    if (km) {
-      const dim3 g((unsigned)natom, (unsigned)((nmax + kTS - 1) / kTS), (unsigned)nsp);
-      k_vso_stored<<<g, kTS, 0, st>>>(psi, ngrid, nnlc, nlc, nl, km, nmax, ld, tmp, psinl);
-    } else {
-      const double sigma_1 = sqrt(0.5) / sigma;  // init.c:97
-      k_vso_gauss<<<grid, kT, 0, st>>>(psi, ngrid, nnlc, nlc, nl, tmp, sigma_1, psinl);
-    }
+    const double sigma_1 = sqrt(0.5) / sigma;  // init.c:97
+    k_vso_gauss<<<grid, kT, 0, st>>>(psi, ngrid, nnlc, nlc, nl, tmp, sigma_1, psinl);
   }
   return cudaGetLastError();
 }
@@ -357,7 +405,7 @@ int sep_spinor_vso_dev(const double* psi, long ngrid, long natom, long nnlc, con
     return fail(SEP_ERR_ARG, "sep_spinor_vso: bad arguments");
   cudaStream_t st = (cudaStream_t)cuda_stream;
   SK(sep::spinor_vso_launch(psi, ngrid, 1, natom, nnlc, nlc, nl, sigma, dv, flagkb, elkb,
-                            nullptr, 0, 0, psinl, st));
+                            psinl, st));
   return SEP_OK;
 }
 

@@ -44,8 +44,11 @@ namespace sep {
 
 cudaError_t spinor_vso_launch(const double* psi, long ngrid, long nsp, long natom, long nnlc,
                               const sep_nlc* nlc, const long* nl, double sigma, double dv,
-                              int flagkb, const double* elkb, const double* km, long nmax,
-                              long ld, double* psinl, cudaStream_t st);
+                              int flagkb, const double* elkb, double* psinl, cudaStream_t st);
+cudaError_t spinor_vso_kept(const double* psi, long ngrid, long nsp, long natom, long nnlc,
+                            const sep_nlc* nlc, const long* nl, double sigma, double dv,
+                            const double* km, long nmax, long ld, const int* off, const int* idx,
+                            double* contrib, double* psinl, cudaStream_t st);
 cudaError_t spinor_vso_kernel(long natom, long nnlc, const sep_nlc* nlc, const long* nl,
                               double sigma, long nmax, long ld, double* km, cudaStream_t st);
 
@@ -161,14 +164,26 @@ __global__ void k_unpack_spinor(const double* __restrict__ acc, long long slots,
   }
 }
 
+// bytes of w_soc per spinor of a Vso apply
+size_t vso_scratch(const sep_ctx* c) {
+  return sizeof(double) * 4 * (size_t)c->so_natom * (size_t)c->so_kmax;
+}
+
 // Vso applied to nsp spinors into out
 int vso(sep_ctx* c, const double* psi, long long nsp, double* out) {
   if (nsp > 65535) return arg_fail("spinor path: more than 65535 spinors in one call");
+  if (c->so_kmax > 0) {
+    RET(grow(c, c->w_soc, vso_scratch(c) * (size_t)nsp));
+    const int* off = c->w_sog.as<int>();
+    CK(spinor_vso_kept(psi, (long)c->n, (long)nsp, c->so_natom, c->so_nnlc,
+                       c->w_nlc.as<sep_nlc>(), c->w_nl.as<long>(), c->so_sigma, c->dv,
+                       c->w_sok.as<double>(), c->so_kmax, c->so_kld, off, off + c->n + 1,
+                       c->w_soc.as<double>(), out, c->stream));
+    return kOk;
+  }
   CK(spinor_vso_launch(psi, (long)c->n, (long)nsp, c->so_natom, c->so_nnlc,
                        c->w_nlc.as<sep_nlc>(), c->w_nl.as<long>(), c->so_sigma, c->dv,
-                       c->so_flagkb, c->w_elkb.as<double>(),
-                       c->so_kmax > 0 ? c->w_sok.as<double>() : nullptr, c->so_kmax, c->so_kld,
-                       out, c->stream));
+                       c->so_flagkb, c->w_elkb.as<double>(), out, c->stream));
   return kOk;
 }
 
@@ -177,8 +192,13 @@ int spinor_h(sep_ctx* c, const double* psi, double* out, long long nsp) {
   RET(apply_h_chunked(c, reinterpret_cast<const cx<double>*>(psi),
                       reinterpret_cast<cx<double>*>(out), 2 * nsp));
   const long long L = 4 * c->n;
-  for (long long s0 = 0; s0 < nsp; s0 += 4096) {
-    const long long k = std::min<long long>(4096, nsp - s0);
+  // spinors at a time: the contributions of the kept kernel take no more than w_so
+  long long most = 4096;
+  if (c->so_kmax > 0)
+    most = std::max<long long>(
+        1, std::min<long long>(most, (long long)(4096.0 * 8.0 * (double)L / (double)vso_scratch(c))));
+  for (long long s0 = 0; s0 < nsp; s0 += most) {
+    const long long k = std::min<long long>(most, nsp - s0);
     RET(grow(c, c->w_so, sizeof(double) * (size_t)(L * k)));
     RET(vso(c, psi + s0 * L, k, c->w_so.as<double>()));
     k_axpy<<<blocks(L * k), kT, 0, c->stream>>>(out + s0 * L, c->w_so.as<double>(), 1.0, L * k);
@@ -465,12 +485,15 @@ int spinor_set_operator(sep_ctx* c, long natom, long nnlc, const sep_nlc* nlc, c
   RET(grow(c, c->w_nl, sizeof(long) * (size_t)std::max<long>(1, natom)));
   RET(grow(c, c->w_elkb, sizeof(double) * (size_t)std::max<long>(2, 2 * natom)));
   if (natom > 0) {
-    CK(cudaMemcpy(c->w_nlc.p, nlc, sizeof(sep_nlc) * (size_t)natom * nnlc,
-                  cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(c->w_nl.p, nl, sizeof(long) * (size_t)natom, cudaMemcpyHostToDevice));
+    // on the context's stream, which the kernels below use
+    CK(cudaMemcpyAsync(c->w_nlc.p, nlc, sizeof(sep_nlc) * (size_t)natom * nnlc,
+                       cudaMemcpyHostToDevice, c->stream));
+    CK(cudaMemcpyAsync(c->w_nl.p, nl, sizeof(long) * (size_t)natom, cudaMemcpyHostToDevice,
+                       c->stream));
     if (flagkb)
-      CK(cudaMemcpy(c->w_elkb.p, elkb, sizeof(double) * 2 * (size_t)natom,
-                    cudaMemcpyHostToDevice));
+      CK(cudaMemcpyAsync(c->w_elkb.p, elkb, sizeof(double) * 2 * (size_t)natom,
+                         cudaMemcpyHostToDevice, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
   }
   // the Gaussian form's K(j1, j2) of every atom, kept while the operator is
   // set: an apply of 64 atoms x 340 points to 4 spinors takes 0.73 ms with it
@@ -479,13 +502,31 @@ int spinor_set_operator(sep_ctx* c, long natom, long nnlc, const sep_nlc* nlc, c
   // which the filter's history needs more.
   c->so_kmax = 0;
   if (!flagkb && natom > 0) {
-    long nmax = 0;
-    for (long a = 0; a < natom; ++a) nmax = std::max(nmax, nl[a]);
+    long nmax = 0, points = 0;
+    for (long a = 0; a < natom; ++a) {
+      nmax = std::max(nmax, nl[a]);
+      points += nl[a];
+    }
     const long ld = (nmax + 31) / 32 * 32;
     const double bytes = 8.0 * (double)natom * (double)nmax * (double)ld;
-    if (nmax > 0 && nmax <= 65535L * 64 &&
+    if (nmax > 0 && nmax <= 65535L * 64 && (double)natom * (double)nmax <= 2147483647.0 &&
         bytes <= 0.125 * (double)(free_device_bytes() + c->w_sok.bytes)) {
-      if (c->w_sok.ensure((size_t)bytes) == cudaSuccess) {
+      const size_t ints = (size_t)c->n + 1 + (size_t)points;
+      if (c->w_sok.ensure((size_t)bytes) == cudaSuccess &&
+          c->w_sog.ensure(sizeof(int) * ints) == cudaSuccess) {
+        // the list points of each grid point, in list order (counting sort)
+        std::vector<int> oi(ints, 0);
+        int* off = oi.data();
+        int* idx = off + c->n + 1;
+        for (long a = 0; a < natom; ++a)
+          for (long j = 0; j < nl[a]; ++j) ++off[nlc[(size_t)a * nnlc + j].jxyz];
+        for (long long g = 1; g <= c->n; ++g) off[g] += off[g - 1];
+        for (long a = natom - 1; a >= 0; --a)
+          for (long j = nl[a] - 1; j >= 0; --j)
+            idx[--off[nlc[(size_t)a * nnlc + j].jxyz]] = (int)(a * nmax + j);
+        CK(cudaMemcpyAsync(c->w_sog.p, oi.data(), sizeof(int) * ints, cudaMemcpyHostToDevice,
+                           c->stream));
+        CK(cudaStreamSynchronize(c->stream));
         CK(spinor_vso_kernel(natom, nnlc, c->w_nlc.as<sep_nlc>(), c->w_nl.as<long>(), sigma, nmax,
                              ld, c->w_sok.as<double>(), c->stream));
         c->so_kmax = nmax;
@@ -495,7 +536,11 @@ int spinor_set_operator(sep_ctx* c, long natom, long nnlc, const sep_nlc* nlc, c
       }
     }
   }
-  if (c->so_kmax == 0) c->w_sok.release();
+  if (c->so_kmax == 0) {
+    c->w_sok.release();
+    c->w_sog.release();
+    c->w_soc.release();
+  }
   c->so_natom = natom;
   c->so_nnlc = nnlc;
   c->so_sigma = sigma;
@@ -598,11 +643,12 @@ int spinor_filter_device(sep_ctx* c, const double* d_start, long ns, const doubl
   int K = std::max(1, std::min<int>(c->block_steps, (int)nc));
   const long ms2 = 2 * ms;
   // per spinor: 2 slots of (K history grids + 1 transform grid), 2 x 2 ms2
-  // accumulators per point, and Vso psi
+  // accumulators per point, Vso psi and the list points' contributions to it
   const size_t per_sp = 2 * (sizeof(cx<double>) * (size_t)n * (K + 1) +
                              sizeof(double) * 2 * (size_t)ms2 * n) +
-                        sizeof(double) * (size_t)L;
-  const size_t have = c->w_hist.bytes + c->w_fft.bytes + c->w_acc.bytes + c->w_so.bytes;
+                        sizeof(double) * (size_t)L + vso_scratch(c);
+  const size_t have = c->w_hist.bytes + c->w_fft.bytes + c->w_acc.bytes + c->w_so.bytes +
+                      c->w_soc.bytes;
   long long Bs = (long long)(((size_t)(0.6 * (double)free_device_bytes()) + have) / per_sp);
   if (Bs < 1) return arg_fail("spinor filter: not enough device memory for one spinor");
   Bs = std::min<long long>({Bs, (long long)ns, 32767LL});
