@@ -673,12 +673,10 @@ int energy_range_device(sep_ctx* c, double vmin, double* emax, double* dE, long*
   RET(apply_h_chunked(c, psi, hp, 1));  // H psi_0
   for (it = 0; std::fabs((ene - old) / ene) > 1.0e-4 && it < 500; ++it) {
     // psi <- H psi / |H psi| (normalize of norm.c:9-36 over re and im)
+    // (the norm stays on the device: the host waits once per iteration)
     CK(pair_dots<double>(hp, hp, 1, n, 1.0, d2, part, c->stream));
+    CK(normalize_copy<double>(hp, psi, n, d2, c->dv, c->stream));
     double2 nn;
-    CK(cudaMemcpyAsync(&nn, d2, sizeof nn, cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
-    const double nrm = std::sqrt((nn.x + nn.y) * c->dv);
-    CK(scale_copy<double>(hp, psi, n, 1.0 / nrm, c->stream));
     old = ene;
     RET(apply_h_chunked(c, psi, hp, 1));
     CK(pair_dots<double>(psi, hp, 1, n, c->dv, d2, part, c->stream));

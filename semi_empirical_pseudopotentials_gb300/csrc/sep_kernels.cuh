@@ -82,9 +82,10 @@ cudaError_t symmetrize_f64(double* A, long long m, cudaStream_t s);
 // S[l][i] = R[l][i] / sqrt(lam[l]), k x k
 cudaError_t scale_rows_isqrt(const double* R, const double* lam, long long k, double* S,
                              cudaStream_t s);
-// out = in * f (complex)
+// out = in / sqrt((norm2->x + norm2->y) dv) (complex; norm2 on the device)
 template <typename T>
-cudaError_t scale_copy(const cx<T>* in, cx<T>* out, long long count, double f, cudaStream_t s);
+cudaError_t normalize_copy(const cx<T>* in, cx<T>* out, long long count, const double2* norm2,
+                           double dv, cudaStream_t s);
 // out[j][i] = in[i][j]
 cudaError_t transpose_f64(const double* in, long long rows, long long cols, double* out,
                           cudaStream_t s);
