@@ -22,7 +22,8 @@
 //     scheme): Gaussian elimination with partial pivoting of T - lambda I,
 //     eigenvalues closer than 1e-3 ||T||_1 form a group whose vectors are
 //     orthogonalised against each other (modified Gram-Schmidt), eigenvalues
-//     inside a group closer than 10 eps |lambda| are moved apart by that much.
+//     inside a group closer than 10 eps |lambda| are moved apart by that much;
+//     a warp per group.
 //  4. k_unmtr: x = H_0 H_1 ... H_{n-2} z for each vector (a warp per vector,
 //     the vector in shared memory).
 // On GB300 every FP64 operation goes through the FP64 pipe (about 2 FMAs per
@@ -406,143 +407,193 @@ __global__ void __launch_bounds__(kSect * kMaxWanted)
 }
 
 // ---------------------------------------------------------------------------
-// 3. eigenvectors of T by inverse iteration.  Thread 0 splits the nw
-//    eigenvalues into groups; each group's vectors are made by one thread.
-//    Scratch per thread: the LU of T - lambda I (4 n) and two vectors.
-constexpr int kSteinThreads = 64;
-
-__device__ double lcg_uniform(unsigned long long& s) {  // (-1, 1)
-  s = s * 6364136223846793005ULL + 1442695040888963407ULL;
+// 3. eigenvectors of T by inverse iteration: block (matrix, i) is one warp
+//    that makes the vectors of the group whose first eigenvalue is i, if one
+//    begins there.  T - lambda I, its LU and the iterate are in shared memory
+//    (5 n doubles and n flags).  Lane 0 runs the three recurrences; sums,
+//    norms, scaling, reciprocal pivots and Gram-Schmidt take all lanes.  Bound
+//    by the recurrences' chains, about 24 dependent FP64 operations per row
+//    and vector (12 of them the elimination's division), which is why the groups
+//    spread over all SMs' sub-partitions, where an FP64 instruction of one lane
+//    holds its pipe as long as one of 32.  42 matrices of 377, 32 vectors each:
+//    1.95 ms; 5.6 ms with a thread per group in one block per matrix, every
+//    row through global scratch and a division per pivot and iteration.
+__device__ double lcg_uniform(unsigned long long s) {  // (-1, 1)
   return (double)(s >> 11) * (2.0 / 9007199254740992.0) - 1.0;
 }
 
-// The LU rows, the iterate and the vectors live in global scratch that this
-// thread both writes and reads back in the same loops (x[k + 1] after x[k]):
-// no __restrict__ on those pointers, and the recurrences are not unrolled, so
-// that no load is hoisted above the store it depends on.  (With restrict
-// qualifiers here the compiled forward elimination read every x[k] from before
-// the loop.)
-__global__ void __launch_bounds__(kSteinThreads)
-    k_stein(const double* dall, const double* eall, const double* wall, const double* tnorm,
-            int n, int nw, double* zall, double* scratch, int* info) {
-  __shared__ int gstart[kMaxWanted + 1];
-  __shared__ int ngroups;
-  const int m = blockIdx.x;
-  const double* d = dall + (size_t)m * n;
-  const double* e = eall + (size_t)m * n;
+// (value, index) of the largest value over the warp, the lowest index of equal ones
+__device__ __forceinline__ void warp_largest(unsigned long long& v, int& i) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const unsigned long long v2 = __shfl_xor_sync(0xffffffffu, v, o);
+    const int i2 = __shfl_xor_sync(0xffffffffu, i, o);
+    if (v2 > v || (v2 == v && i2 < i)) {
+      v = v2;
+      i = i2;
+    }
+  }
+}
+
+size_t stein_smem(int n) { return (size_t)n * (5 * sizeof(double) + 1); }
+
+__global__ void __launch_bounds__(32)
+    k_stein(const double* __restrict__ dall, const double* __restrict__ eall,
+            const double* __restrict__ wall, const double* __restrict__ tnorm, int n, int nw,
+            double* zall, int* __restrict__ info) {
+  extern __shared__ double st[];
+  double* u0 = st;          // T's diagonal, then U's reciprocal diagonal
+  double* lm = st + n;      // T's off-diagonal, then the multipliers
+  double* u1 = st + 2 * n;  // U's first superdiagonal
+  double* u2 = st + 3 * n;  // U's second superdiagonal
+  double* x = st + 4 * n;
+  char* piv = reinterpret_cast<char*>(st + 5 * n);
+  const int m = blockIdx.x, first = blockIdx.y, lane = threadIdx.x;
   const double* w = wall + (size_t)m * n;
-  double* Zm = zall + (size_t)m * n * nw;
   const double onenrm = tnorm[m];
   const double ortol = 1e-3 * onenrm;
-  if (threadIdx.x == 0) {
-    int g = 0;
-    gstart[g++] = 0;
-    for (int i = 1; i < nw; ++i)
-      if (w[i] - w[i - 1] > ortol) gstart[g++] = i;
-    gstart[g] = nw;
-    ngroups = g;
-  }
-  __syncthreads();
+  if (first > 0 && !(w[first] - w[first - 1] > ortol)) return;
+  const double* d = dall + (size_t)m * n;
+  const double* e = eall + (size_t)m * n;
+  double* Zm = zall + (size_t)m * n * nw;
   const double eps = DBL_EPSILON;
   const double dtpcrt = sqrt(0.1 / n);
-  for (int grp = threadIdx.x; grp < ngroups; grp += blockDim.x) {
-    double* sc = scratch + ((size_t)m * kSteinThreads + threadIdx.x) * 6 * n;
-    double* u0 = sc;          // U diagonal
-    double* u1 = sc + n;      // first superdiagonal
-    double* u2 = sc + 2 * n;  // second superdiagonal
-    double* lm = sc + 3 * n;  // multipliers
-    double* x = sc + 4 * n;
-    char* piv = reinterpret_cast<char*>(sc + 5 * n);
-    double xjm = 0.0;
-    for (int jj = gstart[grp]; jj < gstart[grp + 1]; ++jj) {
-      double xj = w[jj];
-      if (jj > gstart[grp]) {
-        const double pertol = 10.0 * fabs(eps * xj);
-        if (xj - xjm < pertol) xj = xjm + pertol;
-      }
-      xjm = xj;
-      // T - xj I = P L U (partial pivoting): row k holds (u0, u1, u2)
-      double a = d[0] - xj, c = (n > 1) ? e[0] : 0.0;
+  const double tol = fmax(eps * onenrm, DBL_MIN);
+  // the generator's step of 32 places, s <- a32 s + c32
+  constexpr unsigned long long kA = 6364136223846793005ULL, kC = 1442695040888963407ULL;
+  unsigned long long a32 = 1, c32 = 0;
+#pragma unroll
+  for (int q = 0; q < 32; ++q) {
+    c32 = c32 * kA + kC;
+    a32 *= kA;
+  }
+  double xjm = 0.0;
+  for (int jj = first; jj < nw && (jj == first || !(w[jj] - w[jj - 1] > ortol)); ++jj) {
+    double xj = w[jj];
+    if (jj > first) {
+      const double pertol = 10.0 * fabs(eps * xj);
+      if (xj - xjm < pertol) xj = xjm + pertol;
+    }
+    xjm = xj;
+    __syncwarp();
+    unsigned long long seed = 0x9E3779B97F4A7C15ULL * (unsigned long long)(m * 4096 + jj + 1);
+    for (int q = 0; q <= lane; ++q) seed = seed * kA + kC;
+    for (int i = lane; i < n; i += 32) {
+      u0[i] = d[i];
+      lm[i] = i < n - 1 ? e[i] : 0.0;
+      x[i] = lcg_uniform(seed);
+      seed = seed * a32 + c32;
+    }
+    __syncwarp();
+    // T - xj I = P L U (partial pivoting): row k holds (u0, u1, u2)
+    if (lane == 0) {
+      double a = u0[0] - xj, c = lm[0], b = c;  // b: subdiagonal (k + 1, k)
       for (int k = 0; k < n - 1; ++k) {
-        const double b = e[k];                     // subdiagonal (k+1, k)
-        const double an = d[k + 1] - xj;          // next row's diagonal
-        const double cn = (k + 1 < n - 1) ? e[k + 1] : 0.0;
-        if (fabs(a) >= fabs(b)) {
-          const double l = (a != 0.0) ? b / a : 0.0;
-          u0[k] = a;
-          u1[k] = c;
-          u2[k] = 0.0;
-          lm[k] = l;
-          piv[k] = 0;
-          a = an - l * c;
-          c = cn;
-        } else {
-          const double l = a / b;
-          u0[k] = b;
-          u1[k] = an;
-          u2[k] = cn;
-          lm[k] = l;
-          piv[k] = 1;
-          a = c - l * an;
-          c = -l * cn;
-        }
+        const double an = u0[k + 1] - xj;  // next row's diagonal
+        const double cn = lm[k + 1];       // 0 in the last row
+        const bool keep = fabs(a) >= fabs(b);
+        const double num = keep ? b : a, den = keep ? a : b;
+        const double l = den != 0.0 ? num / den : 0.0;
+        u0[k] = den;
+        u1[k] = keep ? c : an;
+        u2[k] = keep ? 0.0 : cn;
+        lm[k] = l;
+        piv[k] = !keep;
+        a = keep ? fma(-l, c, an) : fma(-l, an, c);
+        c = keep ? cn : -l * cn;
+        b = cn;
       }
       u0[n - 1] = a;
-      // small pivots are perturbed (dlagts with a tolerance)
-      const double tol = fmax(eps * onenrm, DBL_MIN);
-      for (int k = 0; k < n; ++k)
-        if (fabs(u0[k]) < tol) u0[k] = (u0[k] < 0.0) ? -tol : tol;
-      unsigned long long seed = 0x9E3779B97F4A7C15ULL * (unsigned long long)(m * 4096 + jj + 1);
-      for (int i = 0; i < n; ++i) x[i] = lcg_uniform(seed);
-      int nrmchk = 0;
-      for (int its = 0; its < 5; ++its) {
-        double asum = 0.0;
-        for (int i = 0; i < n; ++i) asum += fabs(x[i]);
-        const double scl = n * onenrm * fmax(eps, fabs(u0[n - 1])) / fmax(asum, DBL_MIN);
-        for (int i = 0; i < n; ++i) x[i] *= scl;
-        // solve P L U y = x: forward with the row interchanges, then U
-#pragma unroll 1
-        for (int k = 0; k < n - 1; ++k) {
-          if (piv[k]) {
-            const double t = x[k];
-            x[k] = x[k + 1];
-            x[k + 1] = t - lm[k] * x[k];
-          } else {
-            x[k + 1] -= lm[k] * x[k];
-          }
-        }
-#pragma unroll 1
-        for (int k = n - 1; k >= 0; --k) {
-          double s = x[k];
-          if (k + 1 < n) s -= u1[k] * x[k + 1];
-          if (k + 2 < n) s -= u2[k] * x[k + 2];
-          x[k] = s / u0[k];
-        }
-        // orthogonalise against the group's earlier vectors
-        for (int q = gstart[grp]; q < jj; ++q) {
-          const double* zq = Zm + (size_t)q * n;
-          double dot = 0.0;
-          for (int i = 0; i < n; ++i) dot += zq[i] * x[i];
-          for (int i = 0; i < n; ++i) x[i] -= dot * zq[i];
-        }
-        double nrm = 0.0;
-        for (int i = 0; i < n; ++i) nrm = fmax(nrm, fabs(x[i]));
-        if (nrm < dtpcrt) continue;
-        if (++nrmchk < 3) continue;
-        break;
-      }
-      if (nrmchk == 0 && info) atomicAdd(info + m, 1);  // no growth: not accepted by dstein
-      double s2 = 0.0;
-      int jmax = 0;
-      for (int i = 0; i < n; ++i) {
-        s2 += x[i] * x[i];
-        if (fabs(x[i]) > fabs(x[jmax])) jmax = i;
-      }
-      double scl = 1.0 / sqrt(s2);
-      if (x[jmax] < 0.0) scl = -scl;
-      double* zj = Zm + (size_t)jj * n;
-      for (int i = 0; i < n; ++i) zj[i] = x[i] * scl;
+      u1[n - 1] = u2[n - 1] = 0.0;
     }
+    __syncwarp();
+    // small pivots are perturbed (dlagts with a tolerance)
+    const double last = fmax(fabs(u0[n - 1]), tol);
+    __syncwarp();
+    for (int k = lane; k < n; k += 32) {
+      double u = u0[k];
+      if (fabs(u) < tol) u = u < 0.0 ? -tol : tol;
+      u0[k] = 1.0 / u;
+    }
+    int nrmchk = 0;
+    for (int its = 0; its < 5; ++its) {
+      double asum = 0.0;
+      for (int i = lane; i < n; i += 32) asum += fabs(x[i]);
+      asum = warp_sum(asum);
+      const double scl = n * onenrm * fmax(eps, last) / fmax(asum, DBL_MIN);
+      for (int i = lane; i < n; i += 32) x[i] *= scl;
+      __syncwarp();
+      // solve P L U y = x: forward with the row interchanges, then U; the next
+      // row's operands are read before this row's result is stored
+      if (lane == 0) {
+        double xk = x[0], xn = x[1], l = lm[0];
+        bool p = piv[0];
+        for (int k = 0; k < n - 1; ++k) {
+          const int k1 = min(k + 1, n - 2), k2 = min(k + 2, n - 1);
+          const double xn2 = x[k2], l2 = lm[k1];
+          const bool p2 = piv[k1];
+          const double keep = p ? xn : xk, other = p ? xk : xn;
+          x[k] = keep;
+          xk = fma(-l, keep, other);
+          xn = xn2;
+          l = l2;
+          p = p2;
+        }
+        double s = xk, y1 = 0.0, y2 = 0.0;
+        double r = u0[n - 1], v1 = 0.0, v2 = 0.0;
+        for (int k = n - 1; k >= 0; --k) {
+          const int kp = max(k - 1, 0);
+          const double sn = x[kp], rn = u0[kp], v1n = u1[kp], v2n = u2[kp];
+          const double y = fma(-v1, y1, fma(-v2, y2, s)) * r;
+          x[k] = y;
+          y2 = y1;
+          y1 = y;
+          s = sn;
+          r = rn;
+          v1 = v1n;
+          v2 = v2n;
+        }
+      }
+      __syncwarp();
+      // orthogonalise against the group's earlier vectors
+      for (int q = first; q < jj; ++q) {
+        const double* zq = Zm + (size_t)q * n;
+        double dot = 0.0;
+        for (int i = lane; i < n; i += 32) dot += zq[i] * x[i];
+        dot = warp_sum(dot);
+        for (int i = lane; i < n; i += 32) x[i] -= dot * zq[i];
+      }
+      unsigned long long big = 0;
+      int at = 0;
+      for (int i = lane; i < n; i += 32) {
+        // the bits of |x| order as |x| does
+        const unsigned long long v = (unsigned long long)__double_as_longlong(x[i]) << 1 >> 1;
+        big = v > big ? v : big;
+      }
+      warp_largest(big, at);
+      if (!(__longlong_as_double((long long)big) >= dtpcrt)) continue;
+      if (++nrmchk < 3) continue;
+      break;
+    }
+    if (nrmchk == 0 && lane == 0) atomicAdd(info + m, 1);  // no growth: not accepted by dstein
+    double s2 = 0.0;
+    unsigned long long big = 0;
+    int jmax = n;
+    for (int i = lane; i < n; i += 32) {
+      s2 += x[i] * x[i];
+      const unsigned long long v = (unsigned long long)__double_as_longlong(x[i]) << 1 >> 1;
+      if (v > big || jmax == n) {
+        big = v;
+        jmax = i;
+      }
+    }
+    s2 = warp_sum(s2);
+    warp_largest(big, jmax);
+    double scl = 1.0 / sqrt(s2);
+    if (x[jmax] < 0.0) scl = -scl;
+    double* zj = Zm + (size_t)jj * n;
+    for (int i = lane; i < n; i += 32) zj[i] = x[i] * scl;
+    __syncwarp();
   }
 }
 
@@ -656,8 +707,8 @@ cudaError_t run_all(Z* A, int n, int nmat, int nw, bool vectors, double* w, cons
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   if (!vectors) return cudaSuccess;
   if ((e = cudaMemsetAsync(wk.info, 0, sizeof(int) * nmat, s)) != cudaSuccess) return e;
-  k_stein<<<nmat, kSteinThreads, 0, s>>>(wk.d, wk.e, w, wk.tnorm, n, nw, wk.z, wk.scratch,
-                                         wk.info);
+  k_stein<<<dim3((unsigned)nmat, (unsigned)nw), 32, stein_smem(n), s>>>(wk.d, wk.e, w, wk.tnorm,
+                                                                        n, nw, wk.z, wk.info);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   k_unmtr<<<dim3((unsigned)nmat, (unsigned)((nw + kUnWarps - 1) / kUnWarps)), 32 * kUnWarps,
             (size_t)kUnWarps * n * sizeof(Z), s>>>(A, wk.tau, wk.z, n, nw, wk.x);
@@ -677,7 +728,7 @@ size_t work_bytes(int n, int nmat, int nw) {
          + nm * sizeof(int) + 64           // info
          + nm * n * nw * sizeof(double)    // tridiagonal eigenvectors
          + nm * n * nw * sizeof(Z)         // eigenvectors of A
-         + nm * kSteinThreads * 6 * n * sizeof(double) + 8 * 256;
+         + 8 * 256;
 }
 
 Work carve(void* base, int n, int nmat, int nw) {
@@ -696,7 +747,6 @@ Work carve(void* base, int n, int nmat, int nw) {
   wk.info = reinterpret_cast<int*>(take(nm * sizeof(int)));
   wk.z = reinterpret_cast<double*>(take(nm * n * nw * sizeof(double)));
   wk.x = reinterpret_cast<Z*>(take(nm * n * nw * sizeof(Z)));
-  wk.scratch = reinterpret_cast<double*>(take(nm * kSteinThreads * 6 * n * sizeof(double)));
   return wk;
 }
 

@@ -20,7 +20,6 @@ struct Work {
   int* info = nullptr;       // eigenvectors whose inverse iteration did not grow
   double* z = nullptr;       // eigenvectors of T (nmat x nw x n)
   double2* x = nullptr;      // eigenvectors of A (nmat x nw x n)
-  double* scratch = nullptr; // inverse-iteration rows and vectors
 };
 
 bool supported(int n, int nw);

@@ -119,3 +119,20 @@ def test_cluster_sizes(n, nmat):
         assert np.abs(w[m] - ref[:nw]).max() <= 1e-12 * scale
         r = a[m] @ v[m] - v[m] * w[m]
         assert np.abs(r).max() <= 1e-11 * scale
+
+
+@pytest.mark.parametrize("n,nw", [(2, 2), (3, 2), (31, 31), (32, 32), (33, 33), (65, 64),
+                                  (300, 64), (512, 64)])
+def test_inverse_iteration_groups(n, nw):
+    """One matrix with all wanted eigenvalues in one group (1e-6 apart: their
+    vectors are orthogonalised against each other), one with none in a group
+    (apart by more than 1e-3 of the norm, as far as nw allows) and one of both,
+    at sizes around a warp and the largest; bounds of the tests above."""
+    rng = np.random.default_rng(1000 + n)
+    far = np.linspace(-1.0, 1.0, n)
+    close = np.where(np.arange(n) < nw, -1.0 + 1e-6 * np.arange(n), np.linspace(0.5, 1.0, n))
+    mixed = np.sort(np.where(np.arange(n) % 3 == 0, far, np.roll(far, 1) + 1e-5))
+    a = np.stack([_with_spectrum(rng, lam) for lam in (close, far, mixed)])
+    w, v = sep.hermitian_lowest(a, nw)
+    for m in range(3):
+        _check(a[m], nw, w[m], v[m])
