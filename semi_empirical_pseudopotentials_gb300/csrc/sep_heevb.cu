@@ -80,6 +80,15 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
+// sums over the warp of two values per lane: a's in lanes 0-15, b's in 16-31
+__device__ __forceinline__ double warp_sum2(double a, double b, int lane) {
+  const bool up = lane & 16;
+  double c = (up ? b : a) + __shfl_xor_sync(0xffffffffu, up ? a : b, 16);
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+  return c;
+}
+
 // sums over the warp of 8 values per lane, with 9 additions a lane instead of
 // 40 (on this part an FP64 warp instruction holds its sub-partition for 64
 // clocks): value q's total ends in the lanes with lane / 4 == q
@@ -113,7 +122,7 @@ __device__ __forceinline__ double warp_sum8(const double (&x)[8], int lane) {
 //    their gather sums are reduced together (warp_sum8).  Bound by the FP64
 //    pipe (16 FMAs per element of the trailing triangle and step) and, for
 //    large G or small n, by the chain of each step (about 16 us).  42 matrices of
-//    377: 20.8 ms with clusters of 3, 55 ms with one block per matrix.
+//    377: 19.6 ms with clusters of 3, 55 ms with one block per matrix.
 //    shared memory: v, w, gather sums, this block's part (4 n complex) and the
 //    warps' scatter sums (kWarps x n complex)
 constexpr int kCols = 4;
@@ -128,8 +137,9 @@ __global__ void __launch_bounds__(kThreads, 1)
   Z* gs = w + n;                 // gather part of p per own column
   Z* part = gs + n;              // this block's part of A22 v
   Z* pw = part + n;              // scatter parts: kWarps x n
+  static_assert(kWarps == 16, "red: a warp reads it with one value per lane");
   __shared__ double red[2 * kWarps];
-  __shared__ Z sh_tau, sh_scale;
+  __shared__ double sh_q[4];  // tau, 1 / (alpha - beta)
   __shared__ int sh_skip;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int rank = blockIdx.x % G, m = blockIdx.x / G;
@@ -149,25 +159,23 @@ __global__ void __launch_bounds__(kThreads, 1)
         part2 = fma(x.x, x.x, fma(x.y, x.y, part2));
       }
       const double xn2 = warp_sum(part2);
-      if (lane == 0) {
-        const Z al = __ldcg(&A[(size_t)j * n + r0]);
-        double ej = al.x;
-        Z tj = zmk(0.0, 0.0);
-        if (xn2 == 0.0 && al.y == 0.0) {  // already reduced: H_j = I
-          sh_skip = 1;
-        } else {
-          const double beta = -copysign(sqrt(al.x * al.x + al.y * al.y + xn2), al.x);
-          tj = zmk((beta - al.x) / beta, -al.y / beta);
-          const double dx = al.x - beta, dy = al.y, dd = dx * dx + dy * dy;
-          sh_scale = zmk(dx / dd, -dy / dd);  // 1 / (alpha - beta)
-          sh_tau = tj;
-          sh_skip = 0;
-          ej = beta;
-        }
+      const Z al = __ldcg(&A[(size_t)j * n + r0]);
+      const bool skip = xn2 == 0.0 && al.y == 0.0;  // already reduced: H_j = I
+      double beta = al.x, q = 0.0;
+      if (!skip) {
+        beta = -copysign(sqrt(al.x * al.x + al.y * al.y + xn2), al.x);
+        const double dx = al.x - beta, dy = al.y, dd = dx * dx + dy * dy;
+        // the four quotients in four lanes: one division's instructions
+        const double num = lane == 0 ? -dx : lane == 2 ? dx : -dy;
+        q = num / (lane < 2 ? beta : dd);
+      }
+      if (lane < 4) {
+        sh_q[lane] = q;
+        if (lane == 0) sh_skip = skip;
         if (rank == 0) {
-          d[j] = __ldcg(&A[(size_t)j * n + j]).x;
-          e[j] = ej;
-          tau[j] = tj;
+          if (lane < 2) reinterpret_cast<double*>(tau + j)[lane] = q;
+          if (lane == 2) d[j] = __ldcg(&A[(size_t)j * n + j]).x;
+          if (lane == 3) e[j] = beta;
         }
       }
     }
@@ -176,7 +184,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       __syncthreads();
       continue;
     }
-    const Z sc = sh_scale, tj = sh_tau;
+    const Z tj = zmk(sh_q[0], sh_q[1]), sc = zmk(sh_q[2], sh_q[3]);
     for (int i = r0 + tid; i < n; i += kThreads)
       v[i] = i > r0 ? zmul(__ldcg(&A[(size_t)j * n + i]), sc) : zmk(1.0, 0.0);
     Z* mine = pw + (size_t)warp * n;
@@ -237,19 +245,13 @@ __global__ void __launch_bounds__(kThreads, 1)
       if (j % stride / kWarps == rank && i > r0)
         A[(size_t)j * n + i] = v[i];  // kept for the back-transformation
     }
-    px = warp_sum(px);
-    py = warp_sum(py);
-    if (lane == 0) {
-      red[warp] = px;
-      red[kWarps + warp] = py;
-    }
+    const double ps = warp_sum2(px, py, lane);
+    if ((lane & 15) == 0) red[lane + warp] = ps;  // 16 sums of px, 16 of py
     __syncthreads();
-    double dx = 0.0, dy = 0.0;
+    double pt = red[lane];
 #pragma unroll
-    for (int q = 0; q < kWarps; ++q) {
-      dx += red[q];
-      dy += red[kWarps + q];
-    }
+    for (int o = 8; o > 0; o >>= 1) pt += __shfl_xor_sync(0xffffffffu, pt, o);
+    const double dx = __shfl_sync(0xffffffffu, pt, 0), dy = __shfl_sync(0xffffffffu, pt, 16);
     // w = p + alpha v, alpha = -tau (p^H v) / 2
     const Z alpha = zmul(zmk(-0.5 * tj.x, -0.5 * tj.y), zmk(dx, dy));
     for (int i = r0 + tid; i < n; i += kThreads) w[i] = zfma(alpha, v[i], w[i]);
@@ -601,7 +603,7 @@ __global__ void __launch_bounds__(32)
 // 4. X = Q Z: warps on vectors, the vector in shared memory, lanes on the rows
 //    of each reflector.  Blocks of 4 vectors: bound by the FP64 pipe (8 FMAs
 //    per row and reflector) once a crystal's vectors cover every SM, which one
-//    block per matrix did not (42 matrices of 377, 32 vectors each: 2.7 ms, 7.3 ms
+//    block per matrix did not (42 matrices of 377, 32 vectors each: 2.5 ms, 7.3 ms
 //    with one block of 16 warps per matrix)
 constexpr int kUnWarps = 4;
 
@@ -625,8 +627,8 @@ __global__ void __launch_bounds__(32 * kUnWarps)
     Z s = zmk(0.0, 0.0);  // v^H x
     for (int i = j + 1 + lane; i < n; i += 32)
       s = zfmac(i == j + 1 ? zmk(1.0, 0.0) : col[i], x[i], s);
-    s.x = warp_sum(s.x);
-    s.y = warp_sum(s.y);
+    const double st = warp_sum2(s.x, s.y, lane);
+    s = zmk(__shfl_sync(0xffffffffu, st, 0), __shfl_sync(0xffffffffu, st, 16));
     const Z f = zmul(tj, s);
     for (int i = j + 1 + lane; i < n; i += 32) {
       const Z vi = (i == j + 1) ? zmk(1.0, 0.0) : col[i];
