@@ -16,7 +16,7 @@
 //     so the result does not depend on timing.  The reflectors stay below the
 //     subdiagonal for the back-transformation.
 //  2. k_stebz: the lowest nw eigenvalues of T by multisection on Sturm counts
-//     (four threads per eigenvalue; the counts by the division-free continuant
+//     (16 or four threads per eigenvalue; the counts by the division-free continuant
 //     recursion with exact power-of-two rescaling).
 //  3. k_stein: their eigenvectors by inverse iteration (LAPACK dstein's
 //     scheme): Gaussian elimination with partial pivoting of T - lambda I,
@@ -333,15 +333,15 @@ __device__ int sturm_count(const double* d, const double* e2, int n, double x) {
   return c;
 }
 
-// 2. lowest nw eigenvalues, kSect threads each; w[nw .. n-1] = NaN.  Every
-//    round the kSect threads count at the points that cut the interval into
-//    kSect + 1 parts, so an eigenvalue takes log2(kSect + 1) times fewer
-//    rounds of n dependent steps than bisection.  Bound by that chain: four
-//    points per round give a 377-row matrix's 32 eigenvalues one warp per
-//    sub-partition.  42 matrices of 377: 2.1 ms, 4.9 ms by bisection.
-constexpr int kSect = 4;
-
-__global__ void __launch_bounds__(kSect * kMaxWanted)
+// 2. lowest nw eigenvalues, S threads each; w[nw .. n-1] = NaN.  Every round
+//    the S threads count at the points that cut the interval into S + 1 parts,
+//    so an eigenvalue takes log2(S + 1) times fewer rounds of n dependent steps
+//    than bisection.  Bound by that chain as long as no sub-partition holds
+//    many warps; a block is one warp, so a matrix spreads over several SMs.
+//    42 matrices of 377, 32 eigenvalues: 1.24 ms with S = 16; 2.13 ms with S = 4
+//    and one block per matrix, 4.9 ms by bisection.
+template <int S>
+__global__ void __launch_bounds__(32)
     k_stebz(const double* __restrict__ dall, const double* __restrict__ eall, int n, int nw,
             double* __restrict__ wall, double* __restrict__ tnorm) {
   extern __shared__ double sb[];
@@ -351,12 +351,12 @@ __global__ void __launch_bounds__(kSect * kMaxWanted)
   const double* dg = dall + (size_t)blockIdx.x * n;
   const double* eg = eall + (size_t)blockIdx.x * n;
   double* w = wall + (size_t)blockIdx.x * n;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+  for (int i = threadIdx.x; i < n; i += 32) {
     d[i] = dg[i];
     e2[i] = (i < n - 1) ? eg[i] * eg[i] : 0.0;
   }
   __syncthreads();
-  if (threadIdx.x < 32) {  // Gershgorin interval, |T|_1 and the largest e^2
+  {  // Gershgorin interval, |T|_1 and the largest e^2
     double lo = d[0], hi = d[0], emax = 0.0, onenrm = 0.0;
     for (int i = threadIdx.x; i < n; i += 32) {
       const double r = (i > 0 ? fabs(eg[i - 1]) : 0.0) + (i < n - 1 ? fabs(eg[i]) : 0.0);
@@ -376,33 +376,35 @@ __global__ void __launch_bounds__(kSect * kMaxWanted)
       sh_lo = lo - 2.1 * DBL_EPSILON * span - 1e-300;
       sh_hi = hi + 2.1 * DBL_EPSILON * span + 1e-300;
       sh_piv = DBL_MIN * fmax(1.0, emax);
-      tnorm[blockIdx.x] = onenrm;
+      if (blockIdx.y == 0) tnorm[blockIdx.x] = onenrm;
     }
   }
   __syncthreads();
-  for (int t = nw + threadIdx.x; t < n; t += blockDim.x)
+  for (int t = nw + threadIdx.x; t < n && blockIdx.y == 0; t += 32)
     w[t] = __longlong_as_double(0x7ff8000000000000LL);  // NaN: not computed
-  const int t = threadIdx.x / kSect, q = threadIdx.x % kSect;
+  const int t = blockIdx.y * (32 / S) + threadIdx.x / S, q = threadIdx.x % S;
   double lo = sh_lo, hi = sh_hi;
   bool done = t >= nw;
   for (int it = 0; it < 200; ++it) {
     // this thread's point; the interval is done when it is as short as the
-    // eigenvalue's precision or a point no longer lies inside it
-    const double x = lo + (hi - lo) * ((q + 1) * (1.0 / (kSect + 1)));
-    const bool last = hi - lo <= 2.0 * DBL_EPSILON * fmax(fabs(lo), fabs(hi)) + sh_piv ||
-                      x <= lo || x >= hi;
-    const unsigned over = __ballot_sync(0xffffffffu, last);
-    const int base = threadIdx.x & 31 & ~(kSect - 1);
-    done = done || ((over >> base) & ((1u << kSect) - 1u)) != 0;
+    // eigenvalue's precision or no point lies inside it (towards the end some
+    // round to an end, whose count is known)
+    const double x = lo + (hi - lo) * ((q + 1) * (1.0 / (S + 1)));
+    const bool inside = x > lo && x < hi;
+    const int base = threadIdx.x & ~(S - 1);
+    const unsigned in = __ballot_sync(0xffffffffu, inside);
+    done = done || hi - lo <= 2.0 * DBL_EPSILON * fmax(fabs(lo), fabs(hi)) + sh_piv ||
+           ((in >> base) & ((1u << S) - 1u)) == 0;
     if (__all_sync(0xffffffffu, done)) break;
-    const bool above = !done && sturm_count(d, e2, n, x) > t;  // eigenvalue t lies below x
-    const unsigned ab = (__ballot_sync(0xffffffffu, above) >> base) & ((1u << kSect) - 1u);
-    const int first = ab ? __ffs(ab) - 1 : kSect;  // the lowest point above eigenvalue t
+    // eigenvalue t lies below x
+    const bool above = !done && (inside ? sturm_count(d, e2, n, x) > t : x >= hi);
+    const unsigned ab = (__ballot_sync(0xffffffffu, above) >> base) & ((1u << S) - 1u);
+    const int first = ab ? __ffs(ab) - 1 : S;  // the lowest point above eigenvalue t
     const double xl = __shfl_sync(0xffffffffu, x, base + max(first - 1, 0));
-    const double xh = __shfl_sync(0xffffffffu, x, base + min(first, kSect - 1));
+    const double xh = __shfl_sync(0xffffffffu, x, base + min(first, S - 1));
     if (!done) {
       if (first > 0) lo = xl;
-      if (first < kSect) hi = xh;
+      if (first < S) hi = xh;
     }
   }
   if (t < nw && q == 0) w[t] = 0.5 * (lo + hi);
@@ -705,7 +707,18 @@ cudaError_t run_all(Z* A, int n, int nmat, int nw, bool vectors, double* w, cons
                     cudaStream_t s) {
   cudaError_t e = launch_hetrd(A, n, nmat, wk, s);
   if (e != cudaSuccess) return e;
-  k_stebz<<<nmat, (kSect * nw + 31) / 32 * 32, 2 * n * sizeof(double), s>>>(wk.d, wk.e, n, nw, w, wk.tnorm);
+  const auto stebz = [&](auto kernel, int sect) {
+    const dim3 grid((unsigned)nmat, (unsigned)((sect * nw + 31) / 32));
+    kernel<<<grid, 32, 2 * n * sizeof(double), s>>>(wk.d, wk.e, n, nw, w, wk.tnorm);
+  };
+  // 16 points per round while that gives a sub-partition no more than two
+  // warps: a round then takes about as long as with four points, and 13 rounds
+  // do for 23.  Beyond it the FP64 pipe is full and the fewer counts of four
+  // points (4 x 23 per eigenvalue, not 16 x 13) are the faster.
+  if ((long)nmat * nw * 16 <= 2L * 4 * 152 * 32)
+    stebz(k_stebz<16>, 16);
+  else
+    stebz(k_stebz<4>, 4);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   if (!vectors) return cudaSuccess;
   if ((e = cudaMemsetAsync(wk.info, 0, sizeof(int) * nmat, s)) != cudaSuccess) return e;

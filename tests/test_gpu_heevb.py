@@ -136,3 +136,17 @@ def test_inverse_iteration_groups(n, nw):
     w, v = sep.hermitian_lowest(a, nw)
     for m in range(3):
         _check(a[m], nw, w[m], v[m])
+
+
+@pytest.mark.parametrize("nmat,nw", [(1, 1), (38, 64), (39, 64), (607, 4), (609, 4)])
+def test_multisection_point_counts(nmat, nw):
+    """16 or 4 points per round, by the number of eigenvalues wanted in all
+    (2,432 is the last that takes 16), against LAPACK to the bound above; a
+    matrix with a zero off-diagonal and equal eigenvalues among them."""
+    n = 66
+    rng = np.random.default_rng(nmat)
+    a = np.stack([_random_hermitian(rng, n) for _ in range(nmat)])
+    a[0] = np.diag(np.repeat([-2.0, 0.0, 1e-300, 3.0, 5.0, 5.5], n // 6)).astype(complex)
+    w, _ = sep.hermitian_lowest(a, nw, vectors=False)
+    ref = np.linalg.eigvalsh(a)
+    assert np.abs(w - ref[:, :nw]).max() <= 1e-12 * np.abs(ref).max()
