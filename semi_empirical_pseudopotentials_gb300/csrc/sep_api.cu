@@ -170,7 +170,7 @@ sep_ctx::~sep_ctx() {
   w_refine.release();
   for (DevBuf* b : {&w_hist, &w_fft, &w_acc, &w_coef, &w_steps, &w_start, &w_out, &w_red,
                     &w_small, &w_states, &w_states2, &w_tmp, &w_solver, &w_gemm, &w_hpsi,
-                    &w_ozA, &w_ozB, &w_ozP, &w_ozE, &w_sok, &w_sog, &w_soc, &w_nlc, &w_nl, &w_elkb, &w_so, &w_so2,
+                    &w_ozA, &w_ozB, &w_ozP, &w_ozE, &w_sok, &w_sog, &w_sot, &w_soc, &w_nlc, &w_nl, &w_elkb, &w_so, &w_so2,
                     &w_so3, &w_eigh})
     b->release();
   if (solver) cusolverDnDestroy(solver);

@@ -12,6 +12,7 @@
 #include "sep_engine.cuh"
 #include "sep_host.h"
 #include "sep_kernels.cuh"
+#include "sep_spinor.cuh"
 
 namespace sep {
 
@@ -106,6 +107,9 @@ struct sep_ctx {
   long so_kmax = 0, so_kld = 0;  // w_sok: natom x so_kmax x so_kld (0: K not kept)
   sep::DevBuf w_sok;  // the Gaussian form's kernel K(j1, j2) of every atom
   sep::DevBuf w_sog;  // with it: off[n + 1], idx: the list points of each grid point
+  sep::DevBuf w_sot;  // with it: K's digit planes and the tensor route's workspace
+  sep::VsoTensor so_tensor;
+  bool so_planes = false;  // so_tensor holds the operator's planes
   sep::DevBuf w_soc;  // the list points' contributions, 4 natom so_kmax doubles per spinor
   sep::DevBuf w_nlc, w_nl, w_elkb, w_so, w_so2, w_so3;
   sep::DevBuf w_eigh;  // workspace of the symmetric eigensolver

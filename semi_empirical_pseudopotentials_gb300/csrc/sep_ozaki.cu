@@ -32,6 +32,7 @@
 #include <type_traits>
 
 #include "sep_ozaki.cuh"
+#include "sep_ozaki_split.cuh"
 
 namespace sep {
 namespace oz {
@@ -194,70 +195,6 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
-// ---- splitting -------------------------------------------------------------
-// biased FP64 exponent field of x (0 for zero and denormals)
-__device__ __forceinline__ int exp_field(double x) {
-  return (int)((__double_as_longlong(x) >> 52) & 0x7FF);
-}
-
-// scale exponent of a row whose largest exponent field is ex: |x| < 2^e
-__device__ __forceinline__ int scale_of(int ex_max) { return ex_max - 1022; }
-
-// x 2^(55-e) rounded to an integer (|X| <= 2^55), split into kSlices balanced
-// base-256 digits, most significant first; integer operations only
-__device__ __forceinline__ void split7(double x, int e, int (&d)[kSlices]) {
-  const long long bits = __double_as_longlong(x);
-  const int ex = (int)((bits >> 52) & 0x7FF);
-  long long X = 0;
-  if (ex != 0) {
-    const long long m = (bits & 0xFFFFFFFFFFFFFLL) | (1LL << 52);
-    const int sh = 1020 + e - ex;  // X = m 2^-sh, sh >= -2
-    if (sh <= 0)
-      X = m << (-sh);
-    else if (sh < 62)
-      X = (m + (1LL << (sh - 1))) >> sh;
-    if (bits < 0) X = -X;
-  }
-#pragma unroll
-  for (int s = 0; s < kSlices - 1; ++s) {
-    const int w = 8 * (kSlices - 1 - s);
-    const long long q = (X + (1LL << (w - 1))) >> w;
-    d[s] = (int)q;
-    X -= q << w;
-  }
-  d[kSlices - 1] = (int)X;
-}
-
-__device__ __forceinline__ uint32_t bf16_pair(int lo, int hi) {
-  return (__float_as_uint((float)lo) >> 16) | (__float_as_uint((float)hi) & 0xFFFF0000u);
-}
-
-// element offset of (row block rb, K chunk kc, slice s) + position (rr, kk) in it
-__device__ __forceinline__ long long plane_off(int s, long long kc, long long rb, long long nkc,
-                                               long long nrb, int rr, int kk) {
-  (void)nrb;
-  return (rb * nkc + kc) * kBlockElems + ((s * 16 + (rr >> 3)) * 2 + (kk >> 3)) * 64 +
-         (rr & 7) * 8 + (kk & 7);
-}
-
-// eight consecutive K values of one row -> kSlices 16-byte stores
-__device__ __forceinline__ void store_digits8(const double (&x)[8], int e, uint16_t* planes,
-                                              long long kc, long long rb, long long nkc,
-                                              long long nrb, int rr, int k0) {
-  int d[8][kSlices];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) split7(x[i], e, d[i]);
-#pragma unroll
-  for (int s = 0; s < kSlices; ++s) {
-    uint4 v;
-    v.x = bf16_pair(d[0][s], d[1][s]);
-    v.y = bf16_pair(d[2][s], d[3][s]);
-    v.z = bf16_pair(d[4][s], d[5][s]);
-    v.w = bf16_pair(d[6][s], d[7][s]);
-    *reinterpret_cast<uint4*>(planes + plane_off(s, kc, rb, nkc, nrb, rr, k0)) = v;
-  }
-}
-
 // one block per (padded) row: the largest exponent field of the row
 __global__ void k_row_expo(const double* __restrict__ X, long long rows, long long k,
                            long long ld, int* __restrict__ expo) {
@@ -346,19 +283,20 @@ struct MmaArgs {
   long long ldc, m, n;
   double alpha;
   int acc;  // add into C instead of overwriting it
+  // Batch kernels: row blocks of A and 64-row tiles of B per member, tiles of B
+  // that hold columns of C, and C itself (integer sums, sum_value)
+  int batch_m, batch_n, cols_n, shift;
+  long long* S;
   int* err;
 };
 
-// v 2^k without overflow of the intermediate power (k = ea + eb - 38)
-__device__ __forceinline__ double pow2i(int k) {
-  return (k < -1022) ? 0.0 : __longlong_as_double((long long)(k + 1023) << 52);
-}
-__device__ __forceinline__ double scale2(double v, int k) {
-  const int k1 = k / 2;
-  return v * pow2i(k1) * pow2i(k - k1);
-}
-
+template <bool Batch>
 __device__ __forceinline__ void tile_of(const MmaArgs& a, int t, int& tm, int& tn) {
+  if constexpr (Batch) {
+    tm = t / a.cols_n;
+    tn = tm / a.batch_m * a.batch_n + (t - tm * a.cols_n);
+    return;
+  }
   if (!a.sym) {
     tm = t / a.tiles_n;
     tn = t - tm * a.tiles_n;
@@ -383,17 +321,19 @@ __device__ __forceinline__ bool drain_after(int c, int st, int nst) {
                               kStagesPerDrain - 1;
 }
 
+template <bool Batch>
 __device__ __forceinline__ void item_of(const MmaArgs& a, int item, int& split, int& tm, int& tn,
                                         long long& kc0, int& nst) {
   // split-major order: CTAs running together share K ranges (and L2 lines)
   split = item / a.ntiles;
-  tile_of(a, item - split * a.ntiles, tm, tn);
+  tile_of<Batch>(a, item - split * a.ntiles, tm, tn);
   kc0 = split * a.kc_per_split;
   long long kc1 = kc0 + a.kc_per_split;
   if (kc1 > a.nkc) kc1 = a.nkc;
   nst = (int)(kc1 > kc0 ? kc1 - kc0 : 0);  // the host leaves no split empty
 }
 
+template <bool Batch>
 __global__ void __maxnreg__(96) k_oz_mma(const MmaArgs a, const __grid_constant__ CUtensorMap tmb) {
   extern __shared__ __align__(1024) uint8_t stage_mem[];
   __shared__ __align__(8) uint64_t bar_load[kStages];   // copies of a stage landed
@@ -436,7 +376,7 @@ __global__ void __maxnreg__(96) k_oz_mma(const MmaArgs a, const __grid_constant_
       for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
         int split, tm, tn, nst;
         long long kc0;
-        item_of(a, item, split, tm, tn, kc0, nst);
+        item_of<Batch>(a, item, split, tm, tn, kc0, nst);
         const uint16_t* ablk = a.A + (long long)tm * a.nkc * kBlockElems;
         const uint16_t* bblk = a.B + (long long)(tn >> 1) * a.nkc * kBlockElems;
         // B pieces: 1 KB piece (tn & 1) * kSets + c of every digit of block
@@ -490,7 +430,7 @@ __global__ void __maxnreg__(96) k_oz_mma(const MmaArgs a, const __grid_constant_
       for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
         int split, tm, tn, nst;
         long long kc0;
-        item_of(a, item, split, tm, tn, kc0, nst);
+        item_of<Batch>(a, item, split, tm, tn, kc0, nst);
         for (int st = 0; st < nst; ++st) {
           const bool fresh = st == 0 || drain_after(c, st - 1, nst);
           if (fresh && nd < nf) {
@@ -540,7 +480,7 @@ __global__ void __maxnreg__(96) k_oz_mma(const MmaArgs a, const __grid_constant_
     for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
       int split, tm, tn, nst;
       long long kc0;
-      item_of(a, item, split, tm, tn, kc0, nst);
+      item_of<Batch>(a, item, split, tm, tn, kc0, nst);
       long long Rh[kDrainCols], Rl[kDrainCols];
 #pragma unroll
       for (int j = 0; j < kDrainCols; ++j) Rh[j] = Rl[j] = 0;
@@ -592,6 +532,16 @@ __global__ void __maxnreg__(96) k_oz_mma(const MmaArgs a, const __grid_constant_
           *reinterpret_cast<longlong2*>(dh + j) = make_longlong2(Rh[j], Rh[j + 1]);
           *reinterpret_cast<longlong2*>(dl + j) = make_longlong2(Rl[j], Rl[j + 1]);
         }
+      } else if constexpr (Batch) {
+        // one 64-bit sum per output, level 3's unit times 2^-shift: no FP64
+        // instruction here, where 16 columns a lane cost 10 us per tile
+        const long long jb = j0 - (long long)(tm / a.batch_m) * a.batch_n * kTileN;
+        const int sh = a.shift;
+#pragma unroll
+        for (int jj = 0; jj < kDrainCols; ++jj)
+          if (jb + jj < a.n)
+            a.S[i * a.ldc + jb + jj] =
+                (Rh[jj] << sh) + ((Rl[jj] + ((1LL << (24 - sh)) >> 1)) >> (24 - sh));
       } else if (i < a.m) {
         const int ei = a.ea[i];
 #pragma unroll
@@ -754,21 +704,69 @@ int choose_splits(long long m, long long n, long long k, bool sym) {
   return (int)best;
 }
 
-cudaError_t gemm_nt(const Planes& A, const Planes& B, double alpha, bool sym, bool accumulate,
-                    double* C, long long ldc, long long* part, int nsplit, int* err,
-                    cudaStream_t s) {
-  if (A.nkc != B.nkc || A.k != B.k) return cudaErrorInvalidValue;
-  if (nsplit > 1 && !part) return cudaErrorInvalidValue;
+namespace {
+template <bool Batch>
+cudaError_t launch_mma(const MmaArgs& a, const Planes& B, cudaStream_t s) {
   static bool attr_set[64] = {};
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-    e = cudaFuncSetAttribute(k_oz_mma, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    e = cudaFuncSetAttribute(k_oz_mma<Batch>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              kStages * kStageBytes);
     if (e != cudaSuccess) return e;
     attr_set[dev] = true;
   }
+  const long long items = (long long)a.ntiles * a.nsplit;
+  if (items < 1) return cudaSuccess;
+  CUtensorMap tmb;
+  e = b_pieces_map(B, &tmb);
+  if (e != cudaSuccess) return e;
+  const unsigned grid = (unsigned)std::min<long long>(items, sm_count());
+  k_oz_mma<Batch><<<grid, kThreads, kStages * kStageBytes, s>>>(a, tmb);
+  return cudaGetLastError();
+}
+}  // namespace
+
+int batch_shift(long long nkc) {
+  // a sum's high part is below 1.02 K 2^38: shifted, below 2^63
+  int s = 24;
+  while (s > 0 && (nkc * kChunkK) >> (24 - s)) --s;
+  return s;
+}
+
+cudaError_t gemm_nt_batched(const Planes& A, const Planes& B, int batches, long long n,
+                            long long* S, long long ldc, int* err, cudaStream_t s) {
+  if (A.nkc != B.nkc || A.k != B.k || batches < 1 || A.nrb % batches || B.nrb % batches ||
+      n < 1 || n > B.nrb / batches * kBlockRows || A.nrb * cdiv(n, kTileN) > 0x7fffffffLL)
+    return cudaErrorInvalidValue;
+  MmaArgs a{};
+  a.A = A.d;
+  a.a_nrb = A.nrb;
+  a.B = B.d;
+  a.b_nrb = B.nrb;
+  a.nkc = a.kc_per_split = A.nkc;
+  a.ea = A.expo;
+  a.eb = B.expo;
+  a.m = A.nrb * kBlockRows;
+  a.n = n;
+  a.batch_m = (int)(A.nrb / batches);
+  a.batch_n = (int)(B.nrb / batches) * (kBlockRows / kTileN);
+  a.cols_n = (int)cdiv(n, kTileN);
+  a.ntiles = (int)(A.nrb * a.cols_n);
+  a.nsplit = 1;
+  a.shift = batch_shift(A.nkc);
+  a.S = S;
+  a.ldc = ldc;
+  a.err = err;
+  return launch_mma<true>(a, B, s);
+}
+
+cudaError_t gemm_nt(const Planes& A, const Planes& B, double alpha, bool sym, bool accumulate,
+                    double* C, long long ldc, long long* part, int nsplit, int* err,
+                    cudaStream_t s) {
+  if (A.nkc != B.nkc || A.k != B.k) return cudaErrorInvalidValue;
+  if (nsplit > 1 && !part) return cudaErrorInvalidValue;
   MmaArgs a{};
   a.A = A.d;
   a.a_nrb = A.nrb;
@@ -795,15 +793,8 @@ cudaError_t gemm_nt(const Planes& A, const Planes& B, double alpha, bool sym, bo
   a.alpha = alpha;
   a.acc = accumulate ? 1 : 0;
   a.err = err;
-  const long long items = (long long)a.ntiles * a.nsplit;
-  if (items < 1) return cudaSuccess;
-  CUtensorMap tmb;
-  e = b_pieces_map(B, &tmb);
-  if (e != cudaSuccess) return e;
-  const unsigned grid = (unsigned)std::min<long long>(items, sm_count());
-  k_oz_mma<<<grid, kThreads, kStages * kStageBytes, s>>>(a, tmb);
-  e = cudaGetLastError();
-  if (e != cudaSuccess || a.nsplit == 1) return e;
+  const cudaError_t e = launch_mma<false>(a, B, s);
+  if (e != cudaSuccess || a.nsplit == 1 || a.ntiles < 1) return e;
   const long long mn = A.rows * B.rows;
   k_oz_reduce<<<(unsigned)std::min<long long>(cdiv(mn, 256), 152LL * 8), 256, 0, s>>>(
       part, a.nsplit, a.prow, a.pcol, A.expo, B.expo, A.rows, B.rows, alpha, a.sym, a.acc, C, ldc);

@@ -77,6 +77,16 @@ cudaError_t gemm_nt(const Planes& A, const Planes& B, double alpha, bool sym, bo
                     double* C, long long ldc, long long* part, int nsplit, int* err,
                     cudaStream_t s);
 
+// batches products at once, C_b = A_b B_b^T: A and B hold the members' row
+// blocks one after another (the same number each, zero beyond a member's rows
+// and K), C_b (A's rows of b x n, n columns kept of each B_b) begins at row b *
+// (A.nrb / batches) * 128 of S.  S holds integer sums, for the reader to scale
+// (sum_value of sep_ozaki_split.cuh with batch_shift(A.nkc)): the 39 bits below
+// level 0's unit and more, where the dropped levels err by the 37th.
+int batch_shift(long long nkc);
+cudaError_t gemm_nt_batched(const Planes& A, const Planes& B, int batches, long long n,
+                            long long* S, long long ldc, int* err, cudaStream_t s);
+
 // Launch-level check of the kernel's device-side status word (err).
 cudaError_t check_status(const int* err, cudaStream_t s, int* host_status);
 

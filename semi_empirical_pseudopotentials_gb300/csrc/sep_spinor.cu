@@ -14,9 +14,10 @@
 // atom; the j2 points are staged through shared memory in tiles of 256 with
 // conj(Y) psi already formed, so each pair costs one exp and 12 FMAs.  K
 // depends on the operator alone: a context that applies it many times keeps
-// K(j1, j2) of every atom (k_vso_kernel, k_vso_stored), and each pair costs
-// the 12 FMAs; there each list point's contribution is stored and a grid
-// point sums its own in list order (k_vso_gather).
+// K(j1, j2) of every atom (k_vso_kernel), and the sums are matrix products on
+// the tensor cores (k_vso_x_slice, k_vso_combine) or, for short lists, 12 FMAs
+// per pair (k_vso_stored); there each list point's contribution is stored and
+// a grid point sums its own in list order (k_vso_gather).
 // Kleinman-Bylander form (filterSpinors/hamiltonian.c:193-401): twelve
 // projections per atom (block reduction), scaled by Elkb dv, then spread back
 // over the atom's points with the reference's coefficients, term by term.
@@ -24,11 +25,14 @@
 // Kleinman-Bylander form and where K is formed in place.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <string>
 
 #include "../../include/sep_gb300.h"
+#include "sep_ozaki_split.cuh"
+#include "sep_spinor.cuh"
 
 namespace sep {
 void set_error(const std::string& msg);
@@ -170,7 +174,9 @@ __global__ void __launch_bounds__(kT) k_vso_kernel(long nnlc, const sep_nlc* __r
   }
 }
 
-// The Gaussian form with K read back: block (atom, 64 points j1, spinor).
+// The Gaussian form with K read back: block (atom, 64 points j1, spinor).  For
+// lists below 64 points, and where the tensor cores are switched off or K has
+// a value that is not finite.
 // Bound by the FP64 pipe: 12 FMAs per pair and spinor, where forming K costs
 // about 45 more FP64 operations.  Two warps a block, so that the points of an
 // atom spread over several SMs (one block per atom and spinor left most of
@@ -231,6 +237,140 @@ __global__ void __launch_bounds__(kTS)
     o[0] = make_double2(up.re, up.im);
     o[1] = make_double2(dn.re, dn.im);
   }
+}
+
+// ---- the sums on the tensor cores -----------------------------------------
+// Per atom the sums are a matrix product, (K: n x n) times (conj(Y) psi: n x
+// 12 per spinor, the real and imaginary parts of the six products), done for
+// all atoms at once by the digit-split contraction of sep_ozaki.cu: K's digit
+// planes are kept with the operator, the products' are written per apply.
+// 64 atoms x 340 points, 4 spinors: digits of the products 27 us, contraction
+// 63 us (two waves of tiles, K's digits read once: 121 MB), contributions 18 us,
+// where the FMAs took 736 us.  Sums agree with the FP64 kernel's to 1e-15 of
+// the largest and with 64-bit references as well as they do.
+
+// scale exponent of every row of every K (mpad rows per atom); *bad: some
+// value is not finite
+__global__ void k_vso_k_expo(const long* __restrict__ nl, const double* __restrict__ km,
+                             long nmax, long ld, long mpad, int* __restrict__ expo,
+                             int* __restrict__ bad) {
+  const long a = blockIdx.x / mpad, j1 = blockIdx.x % mpad, n = nl[a];
+  int mx = 0;
+  if (j1 < n)  // K is symmetric
+    for (long j2 = threadIdx.x; j2 < n; j2 += 32)
+      mx = max(mx, sep::oz::exp_field(km[((size_t)a * nmax + j1) * ld + j2]));
+  for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if (threadIdx.x == 0) {
+    expo[blockIdx.x] = j1 < n ? sep::oz::scale_of(mx) : 0;
+    if (mx == 0x7ff) *bad = 1;
+  }
+}
+
+// digit planes of every K: block (16 values of j2, 128 rows)
+constexpr int kSliceT = sep::oz::kBlockRows * sep::oz::kChunkK / 8;
+__global__ void __launch_bounds__(kSliceT)
+    k_vso_k_slice(const long* __restrict__ nl, const double* __restrict__ km, long nmax, long ld,
+                  long mb, const int* __restrict__ expo, uint16_t* __restrict__ planes,
+                  long nkc) {
+  const long kc = blockIdx.x, rb = blockIdx.y, a = rb / mb, n = nl[a];
+  const int rr = threadIdx.x / 2, k0 = threadIdx.x % 2 * 8;
+  const long j1 = rb % mb * sep::oz::kBlockRows + rr, j2 = kc * sep::oz::kChunkK + k0;
+  double x[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+    x[i] = j1 < n && j2 + i < n ? km[((size_t)a * nmax + j1) * ld + j2 + i] : 0.0;
+  sep::oz::store_digits8(x, expo[rb * sep::oz::kBlockRows + rr], planes, kc, rb, nkc, 0, rr, k0);
+}
+
+// product m of a list point, in the order of the sums above
+__device__ __forceinline__ C2 vso_product(const double* __restrict__ psi, long ngrid,
+                                          const sep_nlc& e, int m) {
+  const C2 p = ld2(psi + 2 * (m < 3 ? e.jxyz : ngrid + e.jxyz));
+  const int q = m % 3;
+  return conj_mul(ld2(q == 0 ? e.y11 : q == 1 ? e.y10 : e.y1_1), p);
+}
+
+// exponents and digit planes of the products: block (atom, spinor) writes the
+// 12 rows 12 s .. of the atom's nb row blocks, zero from the list's end to the
+// last chunk's.  A thread takes one product of eight points; where that covers
+// the list (up to 680 points) they stay in registers between the exponents and
+// the digits, beyond it they are formed again.
+constexpr int kSliceX = 512;
+__global__ void __launch_bounds__(kSliceX)
+    k_vso_x_slice(const double* __restrict__ psi, long ngrid, long nnlc,
+                  const sep_nlc* __restrict__ nlc, const long* __restrict__ nl, long nb, long nkc,
+                  int* __restrict__ expo, uint16_t* __restrict__ planes) {
+  __shared__ int top[12];
+  const long a = blockIdx.x, n = nl[a];
+  const int row0 = 12 * blockIdx.y, nt = blockDim.x;
+  psi += (size_t)blockIdx.y * 4 * (size_t)ngrid;
+  const sep_nlc* base = nlc + a * nnlc;
+  if (threadIdx.x < 12) top[threadIdx.x] = 0;
+  __syncthreads();
+  const int groups = (int)nkc * (sep::oz::kChunkK / 8), items = 6 * groups;
+  double x[8], y[8];
+  auto form = [&](int t) {
+    const int m = t / groups;
+    const long j0 = 8 * (t - m * groups);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      C2 v = {0.0, 0.0};
+      if (j0 + i < n) v = vso_product(psi, ngrid, base[j0 + i], m);
+      x[i] = v.re;
+      y[i] = v.im;
+    }
+    return m;
+  };
+  for (int t = threadIdx.x; t < items; t += nt) {
+    const int m = form(t);
+    int ex = 0, ey = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      ex = max(ex, sep::oz::exp_field(x[i]));
+      ey = max(ey, sep::oz::exp_field(y[i]));
+    }
+    atomicMax(&top[2 * m], ex);
+    atomicMax(&top[2 * m + 1], ey);
+  }
+  __syncthreads();
+  if (threadIdx.x < 12)
+    expo[a * nb * sep::oz::kBlockRows + row0 + threadIdx.x] = sep::oz::scale_of(top[threadIdx.x]);
+  for (int t = threadIdx.x; t < items; t += nt) {
+    if (items > nt) form(t);
+    const int m = t / groups, g = t - m * groups;
+    const int r = row0 + 2 * m;  // even: both rows are in one block
+    const long rb = a * nb + r / sep::oz::kBlockRows;
+    const int rr = r % sep::oz::kBlockRows;
+    sep::oz::store_digits8(x, sep::oz::scale_of(top[2 * m]), planes, g / 2, rb, nkc, 0, rr,
+                           g % 2 * 8);
+    sep::oz::store_digits8(y, sep::oz::scale_of(top[2 * m + 1]), planes, g / 2, rb, nkc, 0, rr + 1,
+                           g % 2 * 8);
+  }
+}
+
+// contributions from the sums: sums[(a mpad + j) ldc + 12 s + 2 m] (re, im),
+// scaled by the exponents of K's row and of the product's (e0: the rest)
+__global__ void __launch_bounds__(kT)
+    k_vso_combine(const long long* __restrict__ sums, const int* __restrict__ ea,
+                  const int* __restrict__ eb, long xpad, int e0, long ldc, long natom, long mpad,
+                  long nnlc,
+                  const sep_nlc* __restrict__ nlc, const long* __restrict__ nl, long nmax,
+                  double tmp, double2* __restrict__ contrib) {
+  const long t = (long)blockIdx.x * kT + threadIdx.x, a = t / nmax, j = t - a * nmax;
+  if (a >= natom || j >= nl[a]) return;
+  const long long* row = sums + (size_t)(a * mpad + j) * ldc + 12 * blockIdx.y;
+  const int e = ea[a * mpad + j] + e0;
+  eb += a * xpad + 12 * blockIdx.y;
+  C2 acc[6], up, dn;
+#pragma unroll
+  for (int m = 0; m < 6; ++m) {
+    const longlong2 v = *reinterpret_cast<const longlong2*>(row + 2 * m);
+    acc[m] = {sep::oz::sum_value(v.x, e + eb[2 * m]), sep::oz::sum_value(v.y, e + eb[2 * m + 1])};
+  }
+  vso_gauss_point(nlc[a * nnlc + j], tmp, acc, up, dn);
+  double2* o = contrib + (size_t)blockIdx.y * 2 * (size_t)(natom * nmax) + 2 * (size_t)t;
+  o[0] = make_double2(up.re, up.im);
+  o[1] = make_double2(dn.re, dn.im);
 }
 
 // Vso psi of every grid point from the list points' contributions: point g
@@ -359,18 +499,88 @@ cudaError_t spinor_vso_kernel(long natom, long nnlc, const sep_nlc* nlc, const l
       nnlc, nlc, nl, sqrt(0.5) / sigma, nmax, ld, km);  // init.c:97
   return cudaGetLastError();
 }
-// The Gaussian form on nsp spinors (4 ngrid doubles apart) into psinl with the
-// operator's K (spinor_vso_kernel), on st.  off, idx: the list points of each
-// grid point (k_vso_gather); contrib: 4 natom nmax doubles per spinor.
-// 1 <= nsp <= 65535, natom, nmax >= 1.
+
+bool VsoTensor::fits(long natom, long nmax) {
+  const double mb = (double)((nmax + oz::kBlockRows - 1) / oz::kBlockRows);
+  return natom > 0 && nmax > 0 && (double)natom * mb <= 65535.0;
+}
+
+size_t VsoTensor::carve(void* base, long natom_, long nmax_) {
+  natom = natom_;
+  nmax = nmax_;
+  mb = (nmax + oz::kBlockRows - 1) / oz::kBlockRows;
+  nkc = (nmax + oz::kChunkK - 1) / oz::kChunkK;
+  // 128 columns of products at a time per block of B: as many blocks as stay
+  // below half a gigabyte, at most 4 (42 spinors)
+  const double per = (double)natom * ((double)nkc * oz::kBlockElems * 2 + mb * 128.0 * 1024.0);
+  nb = (long)std::max(1.0, std::min(4.0, 536870912.0 / per));
+  char* p = static_cast<char*>(base);
+  auto take = [&](size_t bytes) {
+    char* q = p;
+    p += (bytes + 255) & ~(size_t)255;
+    return q;
+  };
+  const size_t blk = sizeof(uint16_t) * (size_t)nkc * oz::kBlockElems;
+  ka = reinterpret_cast<uint16_t*>(take(blk * natom * mb));
+  xb = reinterpret_cast<uint16_t*>(take(blk * natom * nb));
+  ea = reinterpret_cast<int*>(take(sizeof(int) * natom * mb * oz::kBlockRows));
+  eb = reinterpret_cast<int*>(take(sizeof(int) * natom * nb * oz::kBlockRows));
+  sums = reinterpret_cast<long long*>(
+      take(sizeof(long long) * (size_t)(natom * mb * oz::kBlockRows) * nb * oz::kBlockRows));
+  err = reinterpret_cast<int*>(take(2 * sizeof(int)));
+  return (size_t)(p - static_cast<char*>(base));
+}
+
+cudaError_t spinor_vso_planes(const VsoTensor& v, const long* nl, const double* km, long ld,
+                              int* bad, cudaStream_t st) {
+  const long mpad = v.mb * oz::kBlockRows;
+  cudaError_t e = cudaMemsetAsync(v.err, 0, 2 * sizeof(int), st);
+  if (e != cudaSuccess) return e;
+  k_vso_k_expo<<<(unsigned)(v.natom * mpad), 32, 0, st>>>(nl, km, v.nmax, ld, mpad, v.ea,
+                                                          v.err + 1);
+  k_vso_k_slice<<<dim3((unsigned)v.nkc, (unsigned)(v.natom * v.mb)), kSliceT, 0, st>>>(
+      nl, km, v.nmax, ld, v.mb, v.ea, v.ka, v.nkc);
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  e = cudaMemcpyAsync(bad, v.err + 1, sizeof(int), cudaMemcpyDeviceToHost, st);
+  return e != cudaSuccess ? e : cudaStreamSynchronize(st);
+}
+
 cudaError_t spinor_vso_kept(const double* psi, long ngrid, long nsp, long natom, long nnlc,
                             const sep_nlc* nlc, const long* nl, double sigma, double dv,
-                            const double* km, long nmax, long ld, const int* off, const int* idx,
-                            double* contrib, double* psinl, cudaStream_t st) {
+                            const double* km, long nmax, long ld, const VsoTensor* tensor,
+                            const int* off, const int* idx, double* contrib, double* psinl,
+                            cudaStream_t st) {
   const double tmp = 0.5 / sqrt(kTwoPi * (sigma * sigma)) * dv;  // hamiltonian.c:89
-  const dim3 g((unsigned)natom, (unsigned)((nmax + kTS - 1) / kTS), (unsigned)nsp);
   double2* cb = reinterpret_cast<double2*>(contrib);
-  k_vso_stored<<<g, kTS, 0, st>>>(psi, ngrid, nnlc, nlc, nl, km, nmax, ld, tmp, cb);
+  if (tensor) {
+    const VsoTensor& v = *tensor;
+    const long most = v.nb * oz::kBlockRows / 12;
+    for (long s0 = 0; s0 < nsp; s0 += most) {
+      const long k = std::min(most, nsp - s0), nb = (12 * k + oz::kBlockRows - 1) / oz::kBlockRows;
+      const int items = (int)(6 * v.nkc * (oz::kChunkK / 8));
+      k_vso_x_slice<<<dim3((unsigned)natom, (unsigned)k), std::min(kSliceX, (items + 31) / 32 * 32),
+                      0, st>>>(
+          psi + (size_t)s0 * 4 * ngrid, ngrid, nnlc, nlc, nl, nb, v.nkc, v.eb, v.xb);
+      oz::Planes A, B;
+      A.d = v.ka;
+      A.expo = v.ea;
+      B.d = v.xb;
+      B.expo = v.eb;
+      A.k = B.k = nmax;
+      A.nkc = B.nkc = v.nkc;
+      A.nrb = natom * v.mb;
+      B.nrb = natom * nb;
+      const cudaError_t e =
+          oz::gemm_nt_batched(A, B, (int)natom, 12 * k, v.sums, 12 * k, v.err, st);
+      if (e != cudaSuccess) return e;
+      k_vso_combine<<<dim3((unsigned)((natom * nmax + kT - 1) / kT), (unsigned)k), kT, 0, st>>>(
+          v.sums, v.ea, v.eb, nb * oz::kBlockRows, -38 - oz::batch_shift(v.nkc), 12 * k, natom, v.mb * oz::kBlockRows, nnlc, nlc, nl, nmax, tmp,
+          cb + (size_t)s0 * 2 * (size_t)(natom * nmax));
+    }
+  } else {
+    const dim3 g((unsigned)natom, (unsigned)((nmax + kTS - 1) / kTS), (unsigned)nsp);
+    k_vso_stored<<<g, kTS, 0, st>>>(psi, ngrid, nnlc, nlc, nl, km, nmax, ld, tmp, cb);
+  }
   const dim3 gg((unsigned)((ngrid + kT - 1) / kT), (unsigned)nsp);
   k_vso_gather<<<gg, kT, 0, st>>>(cb, off, idx, ngrid, natom * nmax,
                                   reinterpret_cast<double2*>(psinl));

@@ -39,18 +39,10 @@
 #include "sep_ctx.cuh"
 #include "sep_ctx_detail.cuh"
 #include "sep_eigh.cuh"
+#include "sep_ozaki.cuh"
+#include "sep_spinor.cuh"
 
 namespace sep {
-
-cudaError_t spinor_vso_launch(const double* psi, long ngrid, long nsp, long natom, long nnlc,
-                              const sep_nlc* nlc, const long* nl, double sigma, double dv,
-                              int flagkb, const double* elkb, double* psinl, cudaStream_t st);
-cudaError_t spinor_vso_kept(const double* psi, long ngrid, long nsp, long natom, long nnlc,
-                            const sep_nlc* nlc, const long* nl, double sigma, double dv,
-                            const double* km, long nmax, long ld, const int* off, const int* idx,
-                            double* contrib, double* psinl, cudaStream_t st);
-cudaError_t spinor_vso_kernel(long natom, long nnlc, const sep_nlc* nlc, const long* nl,
-                              double sigma, long nmax, long ld, double* km, cudaStream_t st);
 
 namespace {
 
@@ -169,6 +161,31 @@ size_t vso_scratch(const sep_ctx* c) {
   return sizeof(double) * 4 * (size_t)c->so_natom * (size_t)c->so_kmax;
 }
 
+// The kept operator's sums go to the tensor cores from lists of 64 points on:
+// there both routes take about 40 us (8 atoms, 4 spinors: 39.3 us on the tensor
+// cores, 40.2 us by FP64 FMAs).  The FP64 kernel's time grows with the list
+// (0.7 us per point, and with the pairs once they fill the chip) from 13 us at 10
+// points, the tensor route's stays near 35 us up to 100 points: 64 atoms x 80
+// points 42 against 64 us, x 340 points 109 against 736.
+bool vso_on_tensor_cores(const sep_ctx* c) {
+  return c->so_planes && c->subspace_tc && c->so_kmax >= 64;
+}
+
+// the status of the contractions since the last check
+int vso_check(sep_ctx* c) {
+  if (!c->so_planes) return kOk;
+  int h = 0;
+  CK(oz::check_status(c->so_tensor.err, c->stream, &h));
+  if (h != 0) {
+    char b[160];
+    snprintf(b, sizeof b, "spinor path: a bounded wait in the contraction kernel ran out (%d)", h);
+    set_error(b);
+    CK(cudaMemsetAsync(c->so_tensor.err, 0, sizeof(int), c->stream));
+    return kErrCuda;
+  }
+  return kOk;
+}
+
 // Vso applied to nsp spinors into out
 int vso(sep_ctx* c, const double* psi, long long nsp, double* out) {
   if (nsp > 65535) return arg_fail("spinor path: more than 65535 spinors in one call");
@@ -177,7 +194,8 @@ int vso(sep_ctx* c, const double* psi, long long nsp, double* out) {
     const int* off = c->w_sog.as<int>();
     CK(spinor_vso_kept(psi, (long)c->n, (long)nsp, c->so_natom, c->so_nnlc,
                        c->w_nlc.as<sep_nlc>(), c->w_nl.as<long>(), c->so_sigma, c->dv,
-                       c->w_sok.as<double>(), c->so_kmax, c->so_kld, off, off + c->n + 1,
+                       c->w_sok.as<double>(), c->so_kmax, c->so_kld,
+                       vso_on_tensor_cores(c) ? &c->so_tensor : nullptr, off, off + c->n + 1,
                        c->w_soc.as<double>(), out, c->stream));
     return kOk;
   }
@@ -498,9 +516,10 @@ int spinor_set_operator(sep_ctx* c, long natom, long nnlc, const sep_nlc* nlc, c
   // the Gaussian form's K(j1, j2) of every atom, kept while the operator is
   // set: an apply of 64 atoms x 340 points to 4 spinors takes 0.73 ms with it
   // and 2.83 ms forming K in place.  nmax^2 doubles per atom (2.9 MB at 600
-  // points); left out where that is more than an eighth of the free memory,
+  // points) and 1.8 times that for its digits; left out where that is more than an eighth of the free memory,
   // which the filter's history needs more.
   c->so_kmax = 0;
+  c->so_planes = false;
   if (!flagkb && natom > 0) {
     long nmax = 0, points = 0;
     for (long a = 0; a < natom; ++a) {
@@ -531,6 +550,17 @@ int spinor_set_operator(sep_ctx* c, long natom, long nnlc, const sep_nlc* nlc, c
                              ld, c->w_sok.as<double>(), c->stream));
         c->so_kmax = nmax;
         c->so_kld = ld;
+        VsoTensor& v = c->so_tensor;
+        const size_t tb = nmax >= 64 && VsoTensor::fits(natom, nmax) ? v.carve(nullptr, natom, nmax) : 0;
+        if (tb > 0 && (double)tb <= 0.125 * (double)(free_device_bytes() + c->w_sot.bytes) &&
+            c->w_sot.ensure(tb) == cudaSuccess) {
+          v.carve(c->w_sot.p, natom, nmax);
+          int bad = 0;
+          CK(spinor_vso_planes(v, c->w_nl.as<long>(), c->w_sok.as<double>(), ld, &bad, c->stream));
+          c->so_planes = !bad;
+        } else {
+          cudaGetLastError();
+        }
       } else {
         cudaGetLastError();  // formed in place then
       }
@@ -541,6 +571,7 @@ int spinor_set_operator(sep_ctx* c, long natom, long nnlc, const sep_nlc* nlc, c
     c->w_sog.release();
     c->w_soc.release();
   }
+  if (!c->so_planes) c->w_sot.release();
   c->so_natom = natom;
   c->so_nnlc = nnlc;
   c->so_sigma = sigma;
@@ -551,7 +582,8 @@ int spinor_set_operator(sep_ctx* c, long natom, long nnlc, const sep_nlc* nlc, c
 
 int spinor_hamiltonian_device(sep_ctx* c, const double* psi, double* hpsi, long nsp) {
   if (!c->so_ready) return arg_fail("spinor path: no spin-orbit operator set");
-  return spinor_h(c, psi, hpsi, nsp);
+  RET(spinor_h(c, psi, hpsi, nsp));
+  return vso_check(c);
 }
 
 // filterSpinors/energy.c:49-109.  starts: 4 component grids (real, n each):
@@ -619,6 +651,7 @@ int spinor_energy_range_device(sep_ctx* c, const double* starts_host, double tau
     ++i;
   }
   it_total += i;
+  RET(vso_check(c));
   emax *= 1.2;
   emin -= 0.2 * std::fabs(emin);
   if (!std::isfinite(emin) || !std::isfinite(emax)) {
@@ -715,7 +748,7 @@ int spinor_filter_device(sep_ctx* c, const double* d_start, long ns, const doubl
                                                                     d_out + s0 * ms * L);
     CK(cudaGetLastError());
   }
-  return kOk;
+  return vso_check(c);
 }
 
 // filterSpinors/ortho.c:5-40: orthonormalise m spinors in place, keeping the
@@ -785,6 +818,7 @@ int spinor_rr_device(sep_ctx* c, double* psi, long m, double* eval, double* hpsi
   RET(grow(c, c->w_so3, sizeof(double) * (size_t)(m * L)));
   double* S = c->w_so3.as<double>();
   RET(spinor_h(c, psi, hpsi, m));
+  RET(vso_check(c));
   RET(cgram(w, psi, m, hpsi, m, c->dv));
   k_hermitize<<<blocks((long long)m * m), kT, 0, c->stream>>>(w.A, m);
   CK(cudaGetLastError());

@@ -212,3 +212,55 @@ def test_kept_kernel_equals_the_operator_applied_alone(counts):
         assert np.abs(ref).max() > 0.0
         for got in (full, again):
             assert np.abs(got[s] - bare[s] - ref).max() <= 1e-13 * np.abs(full[s]).max()
+
+
+@pytest.mark.parametrize("counts,nsp", [((64, 5, 0, 63), 1), ((129, 128), 45), ((681, 40), 2),
+                                        ((700,), 1)])
+def test_operator_on_the_tensor_cores(counts, nsp):
+    """Lists of 64 points on take the digit-split contraction: against the
+    operator applied alone (FP64 FMAs) to 1e-13 of the largest value of H psi
+    (a term is good to 2^-53 of its row's largest K and its product's largest
+    value, and 700 of them add up), as with the contraction switched off; over
+    more spinors than one chunk takes (42), above 680 points, where products
+    are formed twice, and around a tile of 128 rows."""
+    rng = np.random.default_rng(sum(counts) + nsp)
+    dims, h = (16, 16, 20), 0.5
+    ngrid = int(np.prod(dims))
+    nlc = np.zeros((len(counts), max(counts)), dtype=spinor.NLC_DTYPE)
+    for a, n in enumerate(counts):
+        nlc[a, :n] = _list_entries(rng, n, ngrid)
+    nl = np.array(counts, dtype=np.int64)
+    psi = rng.normal(size=(nsp, 2 * ngrid)) + 1j * rng.normal(size=(nsp, 2 * ngrid))
+    psi[:, :ngrid] *= np.logspace(-9, 0, ngrid)  # products of many magnitudes in a list
+    out = {}
+    ctx = binding.Context(dims, (h, h, h), potl=np.zeros(ngrid), precision="f64", ekinmax=20.0)
+    for tc in (1, 0):
+        ctx.set_subspace("tc" if tc else "f64")
+        out[tc] = spinor.SpinorPath(ctx, nlc, nl, sigma=h).hamiltonian(psi)
+    bare = spinor.SpinorPath(ctx, nlc, np.zeros_like(nl), sigma=h).hamiltonian(psi)
+    ctx.close()
+    for s in range(nsp):
+        ref = spinor.nonlocal_potential(psi[s], nlc, nl, h, h ** 3)
+        for tc in (1, 0):
+            assert np.abs(out[tc][s] - bare[s] - ref).max() <= 1e-13 * np.abs(out[0][s]).max()
+
+
+def test_operator_with_values_that_are_not_finite():
+    """A list point at its atom (r = 0) makes K infinite there: the sums stay
+    with the FP64 kernel, and the same points are not finite as with the
+    operator applied alone."""
+    rng = np.random.default_rng(5)
+    dims, h = (16, 16, 20), 0.5
+    ngrid = int(np.prod(dims))
+    nlc = np.zeros((2, 100), dtype=spinor.NLC_DTYPE)
+    for a in range(2):
+        nlc[a] = _list_entries(rng, 100, ngrid)
+    nlc["r"][1, 7] = nlc["r2"][1, 7] = 0.0
+    nl = np.array([100, 100], dtype=np.int64)
+    psi = rng.normal(size=(1, 2 * ngrid)) + 1j * rng.normal(size=(1, 2 * ngrid))
+    ctx = binding.Context(dims, (h, h, h), potl=np.zeros(ngrid), precision="f64", ekinmax=20.0)
+    got = spinor.SpinorPath(ctx, nlc, nl, sigma=h).hamiltonian(psi)
+    ctx.close()
+    ref = spinor.nonlocal_potential(psi[0], nlc, nl, h, h ** 3)
+    assert not np.isfinite(ref).all()
+    assert np.array_equal(np.isfinite(got[0]), np.isfinite(ref))
