@@ -54,6 +54,16 @@ __device__ __forceinline__ cx<T> newton_epi(cx<T> t, T v, cx<T> p, T alpha, T be
   const T hx = fma_t(v, p.x, t.x), hy = fma_t(v, p.y, t.y);
   return mk<T>(fma_t(alpha, hx, beta * p.x), fma_t(alpha, hy, beta * p.y));
 }
+// min(k, cap) for k >= 0; in FP64 the bits are compared, on the integer pipe, and
+// not the values, on the FP64 pipe that bounds these passes (64^3 filter 225.7 ->
+// 223.5 ms, the same bits)
+template <typename T>
+__device__ __forceinline__ T capped(T k, T cap) {
+  return k > cap ? cap : k;
+}
+__device__ __forceinline__ double capped(double k, double cap) {
+  return __double_as_longlong(k) > __double_as_longlong(cap) ? cap : k;
+}
 template <typename T> __device__ __forceinline__ cx<T> scale(cx<T> a, T s) {
   return mk<T>(a.x * s, a.y * s);
 }

@@ -348,7 +348,7 @@ line_pass(PassArgs<T> a) {
 #pragma unroll
       for (int k1 = 0; k1 < N1; ++k1) {
         T k = kxy + a.kz[k2 + N2 * k1];
-        k = (k > a.kcap) ? a.kcap : k;
+        k = capped(k, a.kcap);
         if constexpr (PRECOND) k = T(1) / (a.pc_a * k + a.pc_b);
         vb[r][k1] = scale<T>(vb[r][k1], k);
       }
