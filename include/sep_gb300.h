@@ -303,7 +303,8 @@ int sep_ctx_set_tiles(sep_ctx *ctx, const int *choices);
  * The Gram, projection and rotation products of sep_ortho (filter/ortho.c:11-52)
  * and sep_rayleigh_ritz (filter/Hmat.c:11-86).  mode 1 (default): on the
  * tcgen05 tensor cores by exact splitting into bf16 digits with exact integer
- * accumulation, FP64-accurate; mode 0: on the FP64 pipe. */
+ * accumulation, FP64-accurate; mode 0: on the FP64 pipe.  The spinor path's
+ * Gaussian spin-orbit operator, a product per atom, follows the same mode. */
 int sep_ctx_set_subspace(sep_ctx *ctx, int mode);
 /* C (m x n) = alpha A B^T, A m x k, B n x k (host, row-major); sym: B = A
  * (B may be NULL) and C is symmetric.  Uses the context's mode. */
