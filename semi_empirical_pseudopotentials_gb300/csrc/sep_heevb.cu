@@ -659,9 +659,9 @@ size_t hetrd_smem(int n) { return (size_t)(4 + kWarps) * n * sizeof(Z); }
 // number of rounds that nmat clusters need (the clusters of G that the device
 // holds at once, one block per SM) times the time of one, which falls as
 // 1 / G + 64 / n (measured, 42 or 20 matrices, whole band solve without
-// vectors: n = 377 G = 1 52.4 ms, 2 32.3, 3 25.8, 6 19.3, and 42 clusters of 4
-// need a second round: 40.2; n = 219 14.6, 10.3, 8.9, 7.8; n = 73 2.33, 2.13,
-// 2.08, 1.97).
+// vectors: n = 377 G = 1 48.5 ms, 2 28.4, 3 21.9, 6 15.6, and 42 clusters of 4
+// need a second round: 35.1; n = 219 12.5, 8.2, 6.9, 5.7; n = 73 1.63, 1.43,
+// 1.37, 1.30).
 cudaError_t cluster_size(cudaLaunchConfig_t cfg, int n, int nmat, int* size) {
   double best = 0.0;
   *size = 1;
