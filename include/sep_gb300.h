@@ -160,7 +160,8 @@ int sep_hnorm(sep_ctx *ctx, const double *psim1, double *psin, long nstates, dou
  * start: ns x N real states; an_re: ms x nc (real parts of the reference's
  * zomplex an[nc*e + j]); zn: nc points; out: ns x ms x N, block s holding
  * psi0[e][g] = sum_j an_re[e][j] Re psi_j[g] as filter.c computes it.
- * In SEP_PREC_MIXED the recursion and the sums run in complex64 / FP32. */
+ * In SEP_PREC_MIXED the recursion and the sums run in complex64 / FP32.
+ * sep_filter_dev: start and out are device arrays that may begin at any double. */
 int sep_filter(sep_ctx *ctx, const double *start, long ns, const double *an_re,
                const double *zn, long ms, long nc, double dE_1, double vmin, double *out);
 int sep_filter_dev(sep_ctx *ctx, const double *start, long ns, const double *an_re,

@@ -3,6 +3,7 @@
 #include "sep_kernels.cuh"
 
 #include <algorithm>
+#include <cstdint>
 #include <type_traits>
 
 namespace sep {
@@ -233,10 +234,12 @@ cudaError_t launch_x2(dim3 g, const cx<float>* hist, int slots, int B, long long
 }
 
 // k_accumulate_x2's sums -> out[(2b + c) ms + e][g] (state-major, double): a
-// thread takes the two points of one thread of that kernel, so both the
-// 16-byte loads and the 16-byte stores of a warp are adjacent.  Bound by HBM:
-// 48 states x 20 targets of 80 x 64 x 64 in 0.59 ms (6.4 TB/s), 0.73 ms with a
-// point's sums adjacent.
+// thread takes the two points of one thread of that kernel, so a warp reads
+// adjacent quads and its 16-byte stores are adjacent.  Bound by HBM: 48 states x
+// 20 targets of 80 x 64 x 64 in 0.59 ms (6.4 TB/s), 0.73 ms with a point's sums
+// adjacent.  out is the caller's (sep_filter_dev) and may begin at any double:
+// WIDE where it is on a 16-byte boundary (each row then is, n being even).
+template <bool WIDE>
 __global__ void k_unpack_x2(const float4* __restrict__ acc, long long B, long long n2, int ms,
                             long long nstates, double* __restrict__ out) {
   const long long chunks = (n2 + 31) / 32;
@@ -246,12 +249,18 @@ __global__ void k_unpack_x2(const float4* __restrict__ acc, long long B, long lo
     if (g2 >= n2) continue;
     const float* p = reinterpret_cast<const float*>(
         acc + ((b * chunks + g2 / 32) * ms * 32 + (g2 & 31)));
-    double2* o = reinterpret_cast<double2*>(out) + 2 * b * ms * n2 + g2;
+    double* o = out + 2 * (2 * b * ms * n2 + g2);
     const int count = 2 * b + 1 < nstates ? 2 * ms : ms;
     for (int k = 0; k < count; ++k) {  // k = c ms + e; point 2 g2 + 1 is 2 ms values on
       const int k1 = k + 2 * ms;
       const float x = p[(k / 4) * 128 + k % 4], y = p[(k1 / 4) * 128 + k1 % 4];
-      o[(long long)k * n2] = make_double2((double)x, (double)y);
+      double* q = o + 2 * (long long)k * n2;
+      if constexpr (WIDE) {
+        *reinterpret_cast<double2*>(q) = make_double2((double)x, (double)y);
+      } else {
+        q[0] = (double)x;
+        q[1] = (double)y;
+      }
     }
   }
 }
@@ -644,7 +653,9 @@ cudaError_t unpack_accumulators(const TA* acc, long long B, long long n, int ms,
                                 long long nstates, double* out, cudaStream_t s) {
   if constexpr (std::is_same<TA, float>::value) {
     if (n % 2 != 0) return cudaErrorInvalidValue;
-    k_unpack_x2<<<blocks_for(B * n / 2, kThreads, 152LL * 16), kThreads, 0, s>>>(
+    const auto kernel =
+        reinterpret_cast<uintptr_t>(out) % sizeof(double2) == 0 ? k_unpack_x2<true> : k_unpack_x2<false>;
+    kernel<<<blocks_for(B * n / 2, kThreads, 152LL * 16), kThreads, 0, s>>>(
         reinterpret_cast<const float4*>(acc), B, n / 2, ms, nstates, out);
   } else {
     k_unpack_acc<TA><<<blocks_for(B * n, kThreads, 152LL * 16), kThreads, 0, s>>>(

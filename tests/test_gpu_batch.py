@@ -176,3 +176,34 @@ def test_plane_pass_of_rectangles_and_short_lengths(dims):
     ctx.close()
     assert np.abs(lines).max() > 0.0
     assert np.array_equal(fused, lines)
+
+
+@pytest.mark.parametrize("precision", ["mixed", "f64"])
+@pytest.mark.parametrize("ns", [1, 4])
+def test_filter_into_a_buffer_at_any_double(precision, ns):
+    """The device-pointer filter reads and writes the caller's buffers, which may
+    begin at any double (a view of a larger array): one double past a 16-byte
+    boundary the results are the same, bit for bit, and nothing beside them is
+    written."""
+    torch = pytest.importorskip("torch")
+    dims = (14, 18, 20)
+    ctx, pot, dv, npts = _job(dims, 6, precision)
+    vmin = float(pot.min())
+    nc, dE, ms = 40, 40.0, 5
+    ar, ai, zn = sep.coefficients(np.linspace(-1.2, -0.2, ms), nc, dE, vmin,
+                                  (nc / (2.5 * dE)) ** 2)
+    start = torch.as_tensor(sep.start_states(-15, ns, npts, dv), dtype=torch.float64)
+    got = []
+    for off in (0, 1):
+        src = torch.zeros(ns * npts + 2, dtype=torch.float64, device="cuda")
+        out = torch.full((ns * ms * npts + 2,), 7.5, dtype=torch.float64, device="cuda")
+        src[off:off + ns * npts] = start.reshape(-1).to(src)
+        assert src[off:].data_ptr() % 16 == 8 * off and out[off:].data_ptr() % 16 == 8 * off
+        torch.cuda.synchronize()
+        ctx.filter_dev(src[off:].data_ptr(), ns, ar, zn, 4.0 / dE, vmin, out[off:].data_ptr())
+        torch.cuda.synchronize()
+        got.append(out[off:off + ns * ms * npts].cpu().numpy())
+        assert (out[:off] == 7.5).all() and (out[off + ns * ms * npts:] == 7.5).all()
+    ctx.close()
+    assert np.abs(got[0]).max() > 0.0
+    assert np.array_equal(got[0], got[1])
