@@ -26,7 +26,13 @@ namespace {
 thread_local std::string g_err;
 }
 
-void set_error(const std::string& msg) { g_err = msg; }
+// The runtime keeps the error of a failed call (an allocation, say) until it is
+// read: once reported it is taken away, or the check behind the next launch, of
+// a call that has nothing to do with it, would return it again.
+void set_error(const std::string& msg) {
+  g_err = msg;
+  cudaGetLastError();
+}
 const char* last_error() { return g_err.c_str(); }
 
 int cuda_fail(cudaError_t e, const char* what, int line) {

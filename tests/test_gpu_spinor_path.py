@@ -8,6 +8,8 @@ Tolerances: H psi and the filter output as the CPU oracle's pins (samples
 to 1e-12 of the largest, row sums and sums of squares to 1e-11); Vmin and
 dE to 1e-9; the kept count exactly; Ritz values to 1e-9 (relative) and
 sigma to 1e-7 (relative)."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -264,3 +266,29 @@ def test_operator_with_values_that_are_not_finite():
     ref = spinor.nonlocal_potential(psi[0], nlc, nl, h, h ** 3)
     assert not np.isfinite(ref).all()
     assert np.array_equal(np.isfinite(got[0]), np.isfinite(ref))
+
+
+def _set_operator_of(ctx, nnlc, entries):
+    """sep_spinor_set_operator for one atom with the given entries in a list that
+    claims room for nnlc; returns the status."""
+    nlc = np.ascontiguousarray(entries, dtype=spinor.NLC_DTYPE)
+    nl = np.array([len(nlc)], dtype=np.int64)
+    f = binding.lib().sep_spinor_set_operator
+    f.argtypes = [C.c_void_p, C.c_long, C.c_long, C.c_void_p, C.c_void_p, C.c_double, C.c_int,
+                  C.c_void_p]
+    return f(ctx.h, 1, nnlc, nlc.ctypes.data, nl.ctypes.data, 0.5, 0, None)
+
+
+def test_call_after_one_that_ran_out_of_memory():
+    """A list with room for 2^34 entries (1.8 TB) cannot be allocated: the call
+    says so, and the next call, which needs nothing of it, succeeds."""
+    rng = np.random.default_rng(8)
+    dims, h = (16, 16, 20), 0.5
+    ngrid = int(np.prod(dims))
+    psi = rng.normal(size=(1, ngrid)) + 1j * rng.normal(size=(1, ngrid))
+    ctx = binding.Context(dims, (h, h, h), potl=rng.normal(size=ngrid), ekinmax=20.0)
+    before = ctx.hamiltonian(psi)
+    assert _set_operator_of(ctx, 2 ** 34, _list_entries(rng, 10, ngrid)) == -3  # SEP_ERR_NOMEM
+    after = ctx.hamiltonian(psi)
+    ctx.close()
+    assert np.array_equal(after, before)
