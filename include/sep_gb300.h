@@ -536,6 +536,8 @@ int sep_spinor_neighbour_lists(long nx, long ny, long nz, const double *vx, cons
  *   the context until set again.  The Gaussian form also keeps its kernel
  *   K(j1, j2) of every atom (8 nl^2 bytes each) when that is at most an
  *   eighth of the free device memory, and forms it on each apply otherwise.
+ *   Refused arguments leave the operator set before as it was; a call that
+ *   fails after that (out of memory) leaves the context without one.
  * sep_spinor_hamiltonian: hpsi = H psi for nspinors spinors
  *   (filterSpinors/hamiltonian.c:8-46).
  * sep_spinor_energy_range: filterSpinors/energy.c:49-109 from four

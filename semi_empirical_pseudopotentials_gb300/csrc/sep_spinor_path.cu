@@ -498,6 +498,11 @@ int spinor_set_operator(sep_ctx* c, long natom, long nnlc, const sep_nlc* nlc, c
         return arg_fail("sep_spinor_set_operator: a neighbour-list point lies outside the grid");
     }
   }
+  // from here to the end the context has no operator: its buffers are taken over
+  // one after another, and a call that fails on the way leaves none half set
+  c->so_ready = false;
+  c->so_kmax = 0;
+  c->so_planes = false;
   CK(cudaStreamSynchronize(c->stream));
   RET(grow(c, c->w_nlc, sizeof(sep_nlc) * (size_t)std::max<long>(1, natom * nnlc)));
   RET(grow(c, c->w_nl, sizeof(long) * (size_t)std::max<long>(1, natom)));
@@ -518,8 +523,6 @@ int spinor_set_operator(sep_ctx* c, long natom, long nnlc, const sep_nlc* nlc, c
   // and 2.83 ms forming K in place.  nmax^2 doubles per atom (2.9 MB at 600
   // points) and 1.8 times that for its digits; left out where that is more than an eighth of the free memory,
   // which the filter's history needs more.
-  c->so_kmax = 0;
-  c->so_planes = false;
   if (!flagkb && natom > 0) {
     long nmax = 0, points = 0;
     for (long a = 0; a < natom; ++a) {

@@ -292,3 +292,33 @@ def test_call_after_one_that_ran_out_of_memory():
     after = ctx.hamiltonian(psi)
     ctx.close()
     assert np.array_equal(after, before)
+
+
+def test_operator_that_could_not_be_set():
+    """A set call that fails after its arguments were checked has begun to take
+    over the buffers of the operator before it: the context has no operator then
+    (every spinor call says so), and takes a new one as a fresh context does.  One
+    that is refused for its arguments leaves the operator as it was."""
+    rng = np.random.default_rng(9)
+    dims, h = (16, 16, 20), 0.5
+    ngrid = int(np.prod(dims))
+    nlc = np.stack([_list_entries(rng, 90, ngrid) for _ in range(3)])
+    nl = np.array([90, 70, 5], dtype=np.int64)
+    psi = rng.normal(size=(2, 2 * ngrid)) + 1j * rng.normal(size=(2, 2 * ngrid))
+    ctx = binding.Context(dims, (h, h, h), potl=rng.normal(size=ngrid), ekinmax=20.0)
+    path = spinor.SpinorPath(ctx, nlc, nl, sigma=h)
+    first = path.hamiltonian(psi)
+    bad = nlc.copy()
+    bad["jxyz"][0, 0] = ngrid
+    with pytest.raises(binding.SepError, match="outside the grid"):
+        spinor.SpinorPath(ctx, bad, nl, sigma=h)
+    assert np.array_equal(path.hamiltonian(psi), first)
+    assert _set_operator_of(ctx, 2 ** 34, _list_entries(rng, 10, ngrid)) == -3  # SEP_ERR_NOMEM
+    for call in (lambda: path.hamiltonian(psi), path.energy_range,
+                 lambda: path.filter(psi, np.ones((1, 2)), np.zeros(2), 0.1, -1.0),
+                 lambda: path.pipeline(psi, [-0.5], 8)):
+        with pytest.raises(binding.SepError, match="no spin-orbit operator set"):
+            call()
+    again = spinor.SpinorPath(ctx, nlc, nl, sigma=h).hamiltonian(psi)
+    ctx.close()
+    assert np.array_equal(again, first)
