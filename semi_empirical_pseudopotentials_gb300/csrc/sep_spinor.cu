@@ -174,32 +174,14 @@ __global__ void __launch_bounds__(kT) k_vso_kernel(long nnlc, const sep_nlc* __r
   }
 }
 
-// The Gaussian form with K read back: block (atom, 64 points j1, spinor).  For
-// lists below 64 points, and where the tensor cores are switched off or K has
-// a value that is not finite.
-// Bound by the FP64 pipe: 12 FMAs per pair and spinor, where forming K costs
-// about 45 more FP64 operations.  Two warps a block, so that the points of an
-// atom spread over several SMs (one block per atom and spinor left most of
-// them with one or two blocks).  64 atoms x 340 points,
-// 4 spinors: 0.73 ms (12 FMAs per pair at the pipe's rate: 0.57 ms), 2.83 ms
-// forming K in place; K itself 0.79 ms once.
+// The six sums of point j1 of a list of n points (act: there is one), with K read
+// back: FP64 FMAs over tiles of kTS points, which the block's kTS threads share.
 constexpr int kTS = 64;
-__global__ void __launch_bounds__(kTS)
-    k_vso_stored(const double* __restrict__ psi, long ngrid, long nnlc,
-                 const sep_nlc* __restrict__ nlc, const long* __restrict__ nl,
-                 const double* __restrict__ km, long nmax, long ld, double tmp,
-                 double2* __restrict__ contrib) {
-  __shared__ C2 sx[kTS][6];
-  const long a = blockIdx.x, n = nl[a];
-  if ((long)blockIdx.y * kTS >= n) return;
-  psi += (size_t)blockIdx.z * 4 * (size_t)ngrid;
-  contrib += (size_t)blockIdx.z * 2 * (size_t)gridDim.x * (size_t)nmax;
-  const sep_nlc* base = nlc + a * nnlc;
+__device__ __forceinline__ void vso_stored_sums(const double* __restrict__ psi, long ngrid,
+                                                const sep_nlc* __restrict__ base, long n,
+                                                const double* __restrict__ kc, long ld, bool act,
+                                                C2 (&sx)[kTS][6], C2 (&acc)[6]) {
   const int tid = threadIdx.x;
-  const long j1 = (long)blockIdx.y * kTS + tid;
-  const bool act = j1 < n;
-  const double* kc = km + (size_t)a * nmax * ld + j1;
-  C2 acc[6];
 #pragma unroll
   for (int m = 0; m < 6; ++m) acc[m] = {0.0, 0.0};
   for (long t0 = 0; t0 < n; t0 += kTS) {
@@ -230,6 +212,32 @@ __global__ void __launch_bounds__(kTS)
       }
     }
   }
+}
+
+// The Gaussian form with K read back: block (atom, 64 points j1, spinor).  For
+// lists below 64 points, and where the tensor cores are switched off or K has
+// a value that is not finite.
+// Bound by the FP64 pipe: 12 FMAs per pair and spinor, where forming K costs
+// about 45 more FP64 operations.  Two warps a block, so that the points of an
+// atom spread over several SMs (one block per atom and spinor left most of
+// them with one or two blocks).  64 atoms x 340 points,
+// 4 spinors: 0.73 ms (12 FMAs per pair at the pipe's rate: 0.57 ms), 2.83 ms
+// forming K in place; K itself 0.79 ms once.
+__global__ void __launch_bounds__(kTS)
+    k_vso_stored(const double* __restrict__ psi, long ngrid, long nnlc,
+                 const sep_nlc* __restrict__ nlc, const long* __restrict__ nl,
+                 const double* __restrict__ km, long nmax, long ld, double tmp,
+                 double2* __restrict__ contrib) {
+  __shared__ C2 sx[kTS][6];
+  const long a = blockIdx.x, n = nl[a];
+  if ((long)blockIdx.y * kTS >= n) return;
+  psi += (size_t)blockIdx.z * 4 * (size_t)ngrid;
+  contrib += (size_t)blockIdx.z * 2 * (size_t)gridDim.x * (size_t)nmax;
+  const sep_nlc* base = nlc + a * nnlc;
+  const long j1 = (long)blockIdx.y * kTS + threadIdx.x;
+  const bool act = j1 < n;
+  C2 acc[6];
+  vso_stored_sums(psi, ngrid, base, n, km + (size_t)a * nmax * ld + j1, ld, act, sx, acc);
   if (act) {
     C2 up, dn;
     vso_gauss_point(base[j1], tmp, acc, up, dn);
@@ -348,29 +356,48 @@ __global__ void __launch_bounds__(kSliceX)
   }
 }
 
-// contributions from the sums: sums[(a mpad + j) ldc + 12 s + 2 m] (re, im),
-// scaled by the exponents of K's row and of the product's (e0: the rest)
-__global__ void __launch_bounds__(kT)
+// contributions from the sums: block (atom, 64 points j, spinor s); sums[(a mpad
+// + j) ldc + 12 s + 2 m] (re, im), scaled by the exponents of K's row and of the
+// product's (e0: the rest).  Products with an infinite or NaN value have no
+// digits: an (atom, spinor) that holds one takes the FP64 sums, which pass it on.
+__global__ void __launch_bounds__(kTS)
     k_vso_combine(const long long* __restrict__ sums, const int* __restrict__ ea,
-                  const int* __restrict__ eb, long xpad, int e0, long ldc, long natom, long mpad,
-                  long nnlc,
-                  const sep_nlc* __restrict__ nlc, const long* __restrict__ nl, long nmax,
-                  double tmp, double2* __restrict__ contrib) {
-  const long t = (long)blockIdx.x * kT + threadIdx.x, a = t / nmax, j = t - a * nmax;
-  if (a >= natom || j >= nl[a]) return;
-  const long long* row = sums + (size_t)(a * mpad + j) * ldc + 12 * blockIdx.y;
-  const int e = ea[a * mpad + j] + e0;
-  eb += a * xpad + 12 * blockIdx.y;
-  C2 acc[6], up, dn;
+                  const int* __restrict__ eb, long xpad, int e0, long ldc, long mpad,
+                  const double* __restrict__ psi, long ngrid, long nnlc,
+                  const sep_nlc* __restrict__ nlc, const long* __restrict__ nl,
+                  const double* __restrict__ km, long nmax, long ld, double tmp,
+                  double2* __restrict__ contrib) {
+  __shared__ C2 sx[kTS][6];
+  const long a = blockIdx.x, n = nl[a];
+  if ((long)blockIdx.y * kTS >= n) return;
+  const sep_nlc* base = nlc + a * nnlc;
+  const long j = (long)blockIdx.y * kTS + threadIdx.x;
+  const bool act = j < n;
+  eb += a * xpad + 12 * blockIdx.z;
+  C2 acc[6];
+  bool finite = true;
 #pragma unroll
-  for (int m = 0; m < 6; ++m) {
-    const longlong2 v = *reinterpret_cast<const longlong2*>(row + 2 * m);
-    acc[m] = {sep::oz::sum_value(v.x, e + eb[2 * m]), sep::oz::sum_value(v.y, e + eb[2 * m + 1])};
+  for (int m = 0; m < 12; ++m) finite = finite && eb[m] != sep::oz::scale_of(0x7ff);
+  if (!finite) {  // the same in the whole block
+    vso_stored_sums(psi + (size_t)blockIdx.z * 4 * (size_t)ngrid, ngrid, base, n,
+                    km + (size_t)a * nmax * ld + j, ld, act, sx, acc);
+  } else if (act) {
+    const long long* row = sums + (size_t)(a * mpad + j) * ldc + 12 * blockIdx.z;
+    const int e = ea[a * mpad + j] + e0;
+#pragma unroll
+    for (int m = 0; m < 6; ++m) {
+      const longlong2 v = *reinterpret_cast<const longlong2*>(row + 2 * m);
+      acc[m] = {sep::oz::sum_value(v.x, e + eb[2 * m]),
+                sep::oz::sum_value(v.y, e + eb[2 * m + 1])};
+    }
   }
-  vso_gauss_point(nlc[a * nnlc + j], tmp, acc, up, dn);
-  double2* o = contrib + (size_t)blockIdx.y * 2 * (size_t)(natom * nmax) + 2 * (size_t)t;
-  o[0] = make_double2(up.re, up.im);
-  o[1] = make_double2(dn.re, dn.im);
+  if (act) {
+    C2 up, dn;
+    vso_gauss_point(base[j], tmp, acc, up, dn);
+    double2* o = contrib + 2 * (((size_t)blockIdx.z * gridDim.x + a) * nmax + j);
+    o[0] = make_double2(up.re, up.im);
+    o[1] = make_double2(dn.re, dn.im);
+  }
 }
 
 // Vso psi of every grid point from the list points' contributions: point g
@@ -573,9 +600,10 @@ cudaError_t spinor_vso_kept(const double* psi, long ngrid, long nsp, long natom,
       const cudaError_t e =
           oz::gemm_nt_batched(A, B, (int)natom, 12 * k, v.sums, 12 * k, v.err, st);
       if (e != cudaSuccess) return e;
-      k_vso_combine<<<dim3((unsigned)((natom * nmax + kT - 1) / kT), (unsigned)k), kT, 0, st>>>(
-          v.sums, v.ea, v.eb, nb * oz::kBlockRows, -38 - oz::batch_shift(v.nkc), 12 * k, natom, v.mb * oz::kBlockRows, nnlc, nlc, nl, nmax, tmp,
-          cb + (size_t)s0 * 2 * (size_t)(natom * nmax));
+      k_vso_combine<<<dim3((unsigned)natom, (unsigned)((nmax + kTS - 1) / kTS), (unsigned)k), kTS, 0,
+                      st>>>(v.sums, v.ea, v.eb, nb * oz::kBlockRows, -38 - oz::batch_shift(v.nkc),
+                            12 * k, v.mb * oz::kBlockRows, psi + (size_t)s0 * 4 * ngrid, ngrid, nnlc,
+                            nlc, nl, km, nmax, ld, tmp, cb + (size_t)s0 * 2 * (size_t)(natom * nmax));
     }
   } else {
     const dim3 g((unsigned)natom, (unsigned)((nmax + kTS - 1) / kTS), (unsigned)nsp);

@@ -322,3 +322,31 @@ def test_operator_that_could_not_be_set():
     again = spinor.SpinorPath(ctx, nlc, nl, sigma=h).hamiltonian(psi)
     ctx.close()
     assert np.array_equal(again, first)
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf, complex(0.0, np.inf)])
+def test_states_with_values_that_are_not_finite(bad):
+    """One value of a spinor's up grid, a point of the first atom's list, is not
+    finite: the other component is not finite on that list, through the operator
+    alone, exactly where it is with the operator applied by itself, and has its
+    values elsewhere; the other spinors of the call do not notice."""
+    rng = np.random.default_rng(6)
+    dims, h = (16, 16, 20), 0.5
+    ngrid = int(np.prod(dims))
+    points = rng.permutation(ngrid)
+    nlc = np.stack([_list_entries(rng, 150, ngrid) for _ in range(2)])
+    nlc["jxyz"] = points[:300].reshape(2, 150)
+    nl = np.array([150, 100], dtype=np.int64)
+    psi = rng.normal(size=(3, 2 * ngrid)) + 1j * rng.normal(size=(3, 2 * ngrid))
+    ctx = binding.Context(dims, (h, h, h), potl=np.zeros(ngrid), precision="f64", ekinmax=20.0)
+    path = spinor.SpinorPath(ctx, nlc, nl, sigma=h)
+    clean = path.hamiltonian(psi)
+    psi[1, nlc["jxyz"][0, 70]] = bad
+    got = path.hamiltonian(psi)
+    ctx.close()
+    ref = spinor.nonlocal_potential(psi[1], nlc, nl, h, h ** 3)
+    lost = ~np.isfinite(ref[ngrid:])
+    assert lost.sum() == 150
+    assert np.array_equal(~np.isfinite(got[1, ngrid:]), lost)
+    assert np.array_equal(got[1, ngrid:][~lost], clean[1, ngrid:][~lost])
+    assert np.array_equal(got[[0, 2]], clean[[0, 2]])
