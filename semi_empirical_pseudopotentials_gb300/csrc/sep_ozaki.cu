@@ -19,7 +19,8 @@
 //    read them back with tcgen05.ld (warp w: lanes 32 (w % 4) .. + 31, 16 of
 //    the set's columns, two levels per wait) and add them into two int64
 //    fixed-point registers per output element: levels 0-3 in units of 2^-24
-//    of level 0, levels 4-6 in units of 2^-48.
+//    of level 0, levels 4-6 in units of 2^-48 (the batched form has one digit
+//    and level more, in units of 2^-56 from level 4 on).
 // The two sets drain kDrainK / 2 of K apart; while one set is drained the
 // other set's thread keeps issuing, up to kStages - 1 stages ahead, so the
 // tensor cores do not wait for the drains.
@@ -45,20 +46,28 @@ constexpr int kDrainCols = kSetN / 2;                      // columns per drain 
 constexpr int kMmaWarp = kDrainWarps, kLoadWarp = kDrainWarps + kSets;  // a MMA warp per set
 constexpr int kThreads = 32 * (kDrainWarps + kSets + 1);   // + the MMA and copy warps
 constexpr int kStages = 4;
-constexpr int kStageA = kSlices * kTileM * kChunkK * 2;    // 28672 bytes: one block
-constexpr int kStageB = kSlices * kTileN * kChunkK * 2;    // 14336 bytes: 64 rows
-constexpr int kStageBytes = kStageA + kStageB;             // 43008 bytes
+// digits, elements of a block and bytes of a stage of the kernel's two forms
+template <bool Batch> struct Form {
+  static constexpr int slices = Batch ? kBatchSlices : kSlices;
+  static constexpr int block = block_elems(slices);
+  static constexpr int stage_a = slices * kTileM * kChunkK * 2;  // 28672 or 32768 bytes: one block
+  static constexpr int stage_b = slices * kTileN * kChunkK * 2;  // 14336 or 16384 bytes: 64 rows
+  static constexpr int stage = stage_a + stage_b;                // 43008 or 49152 bytes
+};
 constexpr uint32_t kRowGroupStride = 256;                  // bytes between 8-row groups
 constexpr uint32_t kSliceBytes = 16 * 256;                 // one digit of a 128-row block
 constexpr uint32_t kSetSliceBytes = (kSetN / 8) * 256;     // one digit of a set's 32 rows
-constexpr int kTmemCols = 512;                              // set c: 256 c .. + 7 * 32
+constexpr int kTmemCols = 512;                  // set c: 256 c .. + 7 * 32, Batch + 8 * 32
 constexpr int kSetCols = 256;
 constexpr int kStagesPerDrain = kDrainK / kChunkK;          // 8
 constexpr long long kSpin = 1LL << 26;                      // bounded waits
 constexpr int kL2Ahead = 8;  // stages between an operand block's L2 prefetch and its copy
-static_assert(kSlices * kSetN <= kSetCols && kSets * kSetCols <= kTmemCols, "TMEM columns");
-static_assert((kSlices * kSetN) % 16 == 0, "one MMA per digit of A and set");
-static_assert((kSlices) * kDrainK * 16384LL < (1LL << 24), "exact FP32 level sums");
+static_assert(kSlices <= kBatchSlices && kBatchSlices * kSetN <= kSetCols &&
+                  kSets * kSetCols <= kTmemCols,
+              "TMEM columns");
+static_assert(kSetN % 16 == 0 && kBatchSlices * kSetN <= 256, "one MMA per digit of A and set");
+static_assert(kBatchSlices * kDrainK * 16384LL <= (1LL << 24), "exact FP32 level sums");
+static_assert(kStages * Form<true>::stage <= 227 * 1024 - 1024, "shared memory");
 
 // ---- PTX wrappers ----------------------------------------------------------
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -283,10 +292,9 @@ struct MmaArgs {
   long long ldc, m, n;
   double alpha;
   int acc;  // add into C instead of overwriting it
-  // Batch kernels: row blocks of A and 64-row tiles of B per member, tiles of B
-  // that hold columns of C, and C itself (integer sums, sum_value)
-  int batch_m, batch_n, cols_n, shift;
-  long long* S;
+  // Batch kernels: row blocks of A and 64-row tiles of B per member, and tiles of
+  // B that hold columns of C; C holds the sums without their scales (kBatchUnit)
+  int batch_m, batch_n, cols_n;
   int* err;
 };
 
@@ -335,6 +343,8 @@ __device__ __forceinline__ void item_of(const MmaArgs& a, int item, int& split, 
 
 template <bool Batch>
 __global__ void __maxnreg__(96) k_oz_mma(const MmaArgs a, const __grid_constant__ CUtensorMap tmb) {
+  using F = Form<Batch>;
+  constexpr int kS = F::slices;
   extern __shared__ __align__(1024) uint8_t stage_mem[];
   __shared__ __align__(8) uint64_t bar_load[kStages];   // copies of a stage landed
   __shared__ __align__(8) uint64_t bar_free[kStages];   // both sets' products of a stage done
@@ -377,32 +387,32 @@ __global__ void __maxnreg__(96) k_oz_mma(const MmaArgs a, const __grid_constant_
         int split, tm, tn, nst;
         long long kc0;
         item_of<Batch>(a, item, split, tm, tn, kc0, nst);
-        const uint16_t* ablk = a.A + (long long)tm * a.nkc * kBlockElems;
-        const uint16_t* bblk = a.B + (long long)(tn >> 1) * a.nkc * kBlockElems;
+        const uint16_t* ablk = a.A + (long long)tm * a.nkc * F::block;
+        const uint16_t* bblk = a.B + (long long)(tn >> 1) * a.nkc * F::block;
         // B pieces: 1 KB piece (tn & 1) * kSets + c of every digit of block
         // ((tn >> 1) nkc + kc), the tensor's third coordinate counting digits
         const int piece0 = (tn & 1) * kSets;
-        const long long dig0 = (long long)(tn >> 1) * a.nkc * kSlices;
+        const long long dig0 = (long long)(tn >> 1) * a.nkc * kS;
         for (int st = 0; st < nst && ok; ++st, ++gs) {
           const int b = (int)(gs % kStages);
           const long long kc = kc0 + st;
           if (kL2Ahead > 0 && st + kL2Ahead < nst) {  // warm L2 for a later stage
-            prefetch_l2(ablk + (kc + kL2Ahead) * kBlockElems, (uint32_t)(kBlockElems * 2));
-            prefetch_l2(bblk + (kc + kL2Ahead) * kBlockElems, (uint32_t)(kBlockElems * 2));
+            prefetch_l2(ablk + (kc + kL2Ahead) * F::block, (uint32_t)(F::block * 2));
+            prefetch_l2(bblk + (kc + kL2Ahead) * F::block, (uint32_t)(F::block * 2));
           }
           // the buffer's previous stage: both sets' products done
           if (gs >= kStages)
             ok = mbar_wait(smem_u32(&bar_free[b]), (uint32_t)((gs / kStages - 1) & 1), a.err, 2);
           if (!ok) break;
-          const uint32_t base = smem0 + b * kStageBytes, bar = smem_u32(&bar_load[b]);
-          mbar_expect_tx(bar, kStageBytes);
-          bulk_g2s(base, ablk + kc * kBlockElems, kStageA, bar);
+          const uint32_t base = smem0 + b * F::stage, bar = smem_u32(&bar_load[b]);
+          mbar_expect_tx(bar, F::stage);
+          bulk_g2s(base, ablk + kc * F::block, F::stage_a, bar);
           // set c's 32 rows of every digit, digits consecutive: any run of
           // digits of one set is one operand of 32 rows per digit
 #pragma unroll
           for (int c = 0; c < kSets; ++c)
-            tensor3_g2s(base + kStageA + c * kSlices * kSetSliceBytes, &tmb, 0, piece0 + c,
-                        (int)(dig0 + kc * kSlices), bar);
+            tensor3_g2s(base + F::stage_a + c * kS * kSetSliceBytes, &tmb, 0, piece0 + c,
+                        (int)(dig0 + kc * kS), bar);
         }
       }
       // the last copies of every buffer land before the shared memory is released
@@ -412,7 +422,7 @@ __global__ void __maxnreg__(96) k_oz_mma(const MmaArgs a, const __grid_constant_
   } else if (warp == kMmaWarp || warp == kMmaWarp + 1) {
     // ---------------- products: one thread per set ----------------
     // Each set's thread walks the stages in order: it waits for the stage's
-    // copies, issues the set's kSlices MMAs and commits them to the stage
+    // copies, issues the set's kS MMAs and commits them to the stage
     // buffer's barrier (which the copy thread waits on, for both sets,
     // before it reuses the buffer, so a set runs at most kStages - 1 stages
     // ahead of the other).  Before the first stage of a period it waits for
@@ -423,7 +433,7 @@ __global__ void __maxnreg__(96) k_oz_mma(const MmaArgs a, const __grid_constant_
       // and a digit are fixed byte offsets added to the start-address field
       // (shared addresses < 2^18, so the 14-bit field never carries)
       const uint64_t da0 = smem_desc(smem0, 128, kRowGroupStride);
-      const uint64_t db0 = smem_desc(smem0 + kStageA + c * kSlices * kSetSliceBytes, 128, kRowGroupStride);
+      const uint64_t db0 = smem_desc(smem0 + F::stage_a + c * kS * kSetSliceBytes, 128, kRowGroupStride);
       const uint32_t dt = tmem + (uint32_t)(c * kSetCols);
       long long g0 = 0;        // global stage index of the item's first stage
       uint32_t nf = 0, nd = 0;  // periods ended (bar_full commits), drains seen complete
@@ -443,13 +453,13 @@ __global__ void __maxnreg__(96) k_oz_mma(const MmaArgs a, const __grid_constant_
           ok = mbar_wait(smem_u32(&bar_load[b]), (uint32_t)((gs / kStages) & 1), a.err, 1);
           if (!ok) break;
           tc_fence_after();
-          const uint64_t so = (uint64_t)((b * (uint32_t)kStageBytes) >> 4);
-          // digit s of A times digits 0 .. kSlices-1-s of B: the accumulators
-          // of levels s .. kSlices-1, adjacent in TMEM
+          const uint64_t so = (uint64_t)((b * (uint32_t)F::stage) >> 4);
+          // digit s of A times digits 0 .. kS-1-s of B: the accumulators
+          // of levels s .. kS-1, adjacent in TMEM
 #pragma unroll
-          for (int s = 0; s < kSlices; ++s)
+          for (int s = 0; s < kS; ++s)
             mma_bf16(dt + (uint32_t)(s * kSetN), da0 + so + (uint64_t)((s * kSliceBytes) >> 4),
-                     db0 + so, idesc_bf16(kTileM, (kSlices - s) * kSetN),
+                     db0 + so, idesc_bf16(kTileM, (kS - s) * kSetN),
                      (fresh && s == 0) ? 0u : 1u);
           mma_commit(smem_u32(&bar_free[b]));
           if (drain_after(c, st, nst)) {
@@ -493,9 +503,9 @@ __global__ void __maxnreg__(96) k_oz_mma(const MmaArgs a, const __grid_constant_
         const uint32_t t0 = tmem + lane_base + (uint32_t)(c * kSetCols + h * kDrainCols);
         // levels in pairs, two loads in flight per wait
 #pragma unroll
-        for (int l0 = 0; l0 < kSlices; l0 += 2) {
+        for (int l0 = 0; l0 < kS; l0 += 2) {
           uint32_t v[2 * kDrainCols];
-          if (l0 + 1 < kSlices) {
+          if (l0 + 1 < kS) {
             tmem_ld16x2(t0 + (uint32_t)(l0 * kSetN), t0 + (uint32_t)((l0 + 1) * kSetN), v);
           } else {
             uint32_t (&v0)[kDrainCols] = *reinterpret_cast<uint32_t(*)[kDrainCols]>(v);
@@ -504,7 +514,7 @@ __global__ void __maxnreg__(96) k_oz_mma(const MmaArgs a, const __grid_constant_
 #pragma unroll
           for (int q = 0; q < 2; ++q) {
             const int l = l0 + q;
-            if (l < kSlices) {
+            if (l < kS) {
 #pragma unroll
               for (int j = 0; j < kDrainCols; ++j) {
                 const long long w =
@@ -512,7 +522,7 @@ __global__ void __maxnreg__(96) k_oz_mma(const MmaArgs a, const __grid_constant_
                 if (l <= 3)
                   Rh[j] += w << (24 - 8 * l);
                 else
-                  Rl[j] += w << (48 - 8 * l);
+                  Rl[j] += w << (8 * (kS - 1) - 8 * l);
               }
             }
           }
@@ -533,15 +543,12 @@ __global__ void __maxnreg__(96) k_oz_mma(const MmaArgs a, const __grid_constant_
           *reinterpret_cast<longlong2*>(dl + j) = make_longlong2(Rl[j], Rl[j + 1]);
         }
       } else if constexpr (Batch) {
-        // one 64-bit sum per output, level 3's unit times 2^-shift: no FP64
-        // instruction here, where 16 columns a lane cost 10 us per tile
+        // the sums without their scales: no FP64 instruction here, where 16
+        // columns a lane cost 10 us per tile
         const long long jb = j0 - (long long)(tm / a.batch_m) * a.batch_n * kTileN;
-        const int sh = a.shift;
 #pragma unroll
         for (int jj = 0; jj < kDrainCols; ++jj)
-          if (jb + jj < a.n)
-            a.S[i * a.ldc + jb + jj] =
-                (Rh[jj] << sh) + ((Rl[jj] + ((1LL << (24 - sh)) >> 1)) >> (24 - sh));
+          if (jb + jj < a.n) a.C[i * a.ldc + jb + jj] = round_sum(Rh[jj], Rl[jj]);
       } else if (i < a.m) {
         const int ei = a.ea[i];
 #pragma unroll
@@ -619,9 +626,9 @@ int tile_count(long long m, long long n, bool sym) {
 // Tensor map of B's digit planes as 1 KB pieces (32 rows x 16 K of one
 // digit): dimension 0 the 128 8-byte words of a piece, dimension 1 the four
 // pieces of a digit's 128 rows (1 KB apart), dimension 2 the digits of all
-// blocks in order (4 KB apart).  A box {128, 1, kSlices} is the run of one
+// blocks in order (4 KB apart).  A box {128, 1, slices} is the run of one
 // set's pieces over all digits of a block.
-cudaError_t b_pieces_map(const Planes& B, CUtensorMap* map) {
+cudaError_t b_pieces_map(const Planes& B, int slices, CUtensorMap* map) {
   static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
   if (!encode) {
     cudaDriverEntryPointQueryResult q;
@@ -632,9 +639,9 @@ cudaError_t b_pieces_map(const Planes& B, CUtensorMap* map) {
       return cudaErrorNotSupported;
     encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
   }
-  const cuuint64_t dims[3] = {128, 4, (cuuint64_t)(B.nrb * B.nkc * kSlices)};
+  const cuuint64_t dims[3] = {128, 4, (cuuint64_t)(B.nrb * B.nkc * slices)};
   const cuuint64_t strides[2] = {1024, 4096};
-  const cuuint32_t box[3] = {128, 1, (cuuint32_t)kSlices};
+  const cuuint32_t box[3] = {128, 1, (cuuint32_t)slices};
   const cuuint32_t estr[3] = {1, 1, 1};
   const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT64, 3, B.d, dims, strides, box, estr,
                             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
@@ -713,30 +720,23 @@ cudaError_t launch_mma(const MmaArgs& a, const Planes& B, cudaStream_t s) {
   if (e != cudaSuccess) return e;
   if (dev >= 0 && dev < 64 && !attr_set[dev]) {
     e = cudaFuncSetAttribute(k_oz_mma<Batch>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             kStages * kStageBytes);
+                             kStages * Form<Batch>::stage);
     if (e != cudaSuccess) return e;
     attr_set[dev] = true;
   }
   const long long items = (long long)a.ntiles * a.nsplit;
   if (items < 1) return cudaSuccess;
   CUtensorMap tmb;
-  e = b_pieces_map(B, &tmb);
+  e = b_pieces_map(B, Form<Batch>::slices, &tmb);
   if (e != cudaSuccess) return e;
   const unsigned grid = (unsigned)std::min<long long>(items, sm_count());
-  k_oz_mma<Batch><<<grid, kThreads, kStages * kStageBytes, s>>>(a, tmb);
+  k_oz_mma<Batch><<<grid, kThreads, kStages * Form<Batch>::stage, s>>>(a, tmb);
   return cudaGetLastError();
 }
 }  // namespace
 
-int batch_shift(long long nkc) {
-  // a sum's high part is below 1.02 K 2^38: shifted, below 2^63
-  int s = 24;
-  while (s > 0 && (nkc * kChunkK) >> (24 - s)) --s;
-  return s;
-}
-
 cudaError_t gemm_nt_batched(const Planes& A, const Planes& B, int batches, long long n,
-                            long long* S, long long ldc, int* err, cudaStream_t s) {
+                            double* S, long long ldc, int* err, cudaStream_t s) {
   if (A.nkc != B.nkc || A.k != B.k || batches < 1 || A.nrb % batches || B.nrb % batches ||
       n < 1 || n > B.nrb / batches * kBlockRows || A.nrb * cdiv(n, kTileN) > 0x7fffffffLL)
     return cudaErrorInvalidValue;
@@ -755,8 +755,7 @@ cudaError_t gemm_nt_batched(const Planes& A, const Planes& B, int batches, long 
   a.cols_n = (int)cdiv(n, kTileN);
   a.ntiles = (int)(A.nrb * a.cols_n);
   a.nsplit = 1;
-  a.shift = batch_shift(A.nkc);
-  a.S = S;
+  a.C = S;
   a.ldc = ldc;
   a.err = err;
   return launch_mma<true>(a, B, s);

@@ -22,6 +22,11 @@
 //    integers: the result does not depend on the order of the additions.
 //  * Levels l >= kSlices are dropped: the error is below 2^-53 of the
 //    product of the two row maxima, per term, like an FP64 product.
+//
+// The batched products (gemm_nt_batched) hold values as 62-bit integers in
+// kBatchSlices digits: the error is below 2^-60 of the product of the two row
+// maxima, per term, and what bounds a sum is its rounding to FP64 unless its
+// terms are far below that product (sep_spinor.cu tests for that).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -32,12 +37,14 @@ namespace sep {
 namespace oz {
 
 constexpr int kSlices = 7;          // digits per value (55 bits)
+constexpr int kBatchSlices = 8;     // of the batched products (62 bits)
 constexpr int kTileM = 128;         // rows of A per tile (TMEM lanes)
 constexpr int kTileN = 64;          // rows of B per tile (two sets of 32 TMEM columns per level)
 constexpr int kChunkK = 16;         // K per pipeline stage (one MMA per digit pair)
 constexpr int kBlockRows = 128;     // rows per pre-tiled block in global memory
 constexpr int kDrainK = 128;        // K accumulated per level before a drain
-constexpr int kBlockElems = kSlices * kBlockRows * kChunkK;  // 14336 bf16: all digits of a block
+constexpr int block_elems(int slices) { return slices * kBlockRows * kChunkK; }
+constexpr int kBlockElems = block_elems(kSlices);  // 14336 bf16: all digits of a block
 
 // Pre-tiled digit planes of one operand.  Row block rb (128 rows) and K chunk
 // kc (16 values) hold all kSlices digits in one 28,672-byte block, in the
@@ -48,6 +55,7 @@ constexpr int kBlockElems = kSlices * kBlockRows * kChunkK;  // 14336 bf16: all 
 // bytes in, and each 32 rows of a digit one 1024-byte piece.
 // Element offset (uint16) of (row rr of the block, k, digit s):
 //   (rb * nkc + kc) * 14336 + ((s * 16 + i) * 2 + j) * 64 + r * 8 + (k % 8).
+// The batched products' operands have blocks of block_elems(kBatchSlices).
 struct Planes {
   uint16_t* d = nullptr;  // nrb * nkc * 14336 values
   int* expo = nullptr;    // scale exponent per row (nrb * 128 entries)
@@ -80,12 +88,12 @@ cudaError_t gemm_nt(const Planes& A, const Planes& B, double alpha, bool sym, bo
 // batches products at once, C_b = A_b B_b^T: A and B hold the members' row
 // blocks one after another (the same number each, zero beyond a member's rows
 // and K), C_b (A's rows of b x n, n columns kept of each B_b) begins at row b *
-// (A.nrb / batches) * 128 of S.  S holds integer sums, for the reader to scale
-// (sum_value of sep_ozaki_split.cuh with batch_shift(A.nkc)): the 39 bits below
-// level 0's unit and more, where the dropped levels err by the 37th.
-int batch_shift(long long nkc);
-cudaError_t gemm_nt_batched(const Planes& A, const Planes& B, int batches, long long n,
-                            long long* S, long long ldc, int* err, cudaStream_t s);
+// (A.nrb / batches) * 128 of S.  S holds the sums without their scales, for the
+// reader to apply: C = S 2^(ea + eb - kBatchUnit), each the integer sum of the
+// kept levels rounded once to FP64.
+constexpr int kBatchUnit = 68;
+cudaError_t gemm_nt_batched(const Planes& A, const Planes& B, int batches, long long n, double* S,
+                            long long ldc, int* err, cudaStream_t s);
 
 // Launch-level check of the kernel's device-side status word (err).
 cudaError_t check_status(const int* err, cudaStream_t s, int* host_status);

@@ -15,31 +15,38 @@ __device__ __forceinline__ int exp_field(double x) {
 }
 
 // scale exponent of a row whose largest exponent field is ex: |x| < 2^e
-__device__ __forceinline__ int scale_of(int ex_max) { return ex_max - 1022; }
+__host__ __device__ constexpr int scale_of(int ex_max) { return ex_max - 1022; }
 
-// x 2^(55-e) rounded to an integer (|X| <= 2^55), split into kSlices balanced
-// base-256 digits, most significant first; integer operations only
-__device__ __forceinline__ void split7(double x, int e, int (&d)[kSlices]) {
+// x 2^(B-e) rounded to an integer, B = 55 bits in 7 digits (|X| <= 2^55) or 62 in
+// 8 (|X| <= 2^62); integer operations only
+template <int S> __device__ __forceinline__ long long fixed_point(double x, int e) {
+  static_assert(S == kSlices || S == kBatchSlices, "bits of the fixed point");
+  constexpr int bits_of_x = S == kSlices ? 55 : 62;
   const long long bits = __double_as_longlong(x);
   const int ex = (int)((bits >> 52) & 0x7FF);
   long long X = 0;
   if (ex != 0) {
     const long long m = (bits & 0xFFFFFFFFFFFFFLL) | (1LL << 52);
-    const int sh = 1020 + e - ex;  // X = m 2^-sh, sh >= -2
+    const int sh = 1075 - bits_of_x + e - ex;  // X = m 2^-sh, sh >= 53 - 1 - bits_of_x
     if (sh <= 0)
       X = m << (-sh);
     else if (sh < 62)
       X = (m + (1LL << (sh - 1))) >> sh;
     if (bits < 0) X = -X;
   }
+  return X;
+}
+
+// X split into S balanced base-256 digits, most significant first
+template <int S> __device__ __forceinline__ void digits(long long X, int (&d)[S]) {
 #pragma unroll
-  for (int s = 0; s < kSlices - 1; ++s) {
-    const int w = 8 * (kSlices - 1 - s);
+  for (int s = 0; s < S - 1; ++s) {
+    const int w = 8 * (S - 1 - s);
     const long long q = (X + (1LL << (w - 1))) >> w;
     d[s] = (int)q;
     X -= q << w;
   }
-  d[kSlices - 1] = (int)X;
+  d[S - 1] = (int)X;
 }
 
 __device__ __forceinline__ uint32_t bf16_pair(int lo, int hi) {
@@ -47,28 +54,30 @@ __device__ __forceinline__ uint32_t bf16_pair(int lo, int hi) {
 }
 
 // element offset of (row block rb, K chunk kc, slice s) + position (rr, kk) in it
+template <int S = kSlices>
 __device__ __forceinline__ long long plane_off(int s, long long kc, long long rb, long long nkc,
                                                long long nrb, int rr, int kk) {
   (void)nrb;
-  return (rb * nkc + kc) * kBlockElems + ((s * 16 + (rr >> 3)) * 2 + (kk >> 3)) * 64 +
+  return (rb * nkc + kc) * block_elems(S) + ((s * 16 + (rr >> 3)) * 2 + (kk >> 3)) * 64 +
          (rr & 7) * 8 + (kk & 7);
 }
 
-// eight consecutive K values of one row -> kSlices 16-byte stores
+// eight consecutive K values of one row -> S 16-byte stores
+template <int S = kSlices>
 __device__ __forceinline__ void store_digits8(const double (&x)[8], int e, uint16_t* planes,
                                               long long kc, long long rb, long long nkc,
                                               long long nrb, int rr, int k0) {
-  int d[8][kSlices];
+  int d[8][S];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) split7(x[i], e, d[i]);
+  for (int i = 0; i < 8; ++i) digits<S>(fixed_point<S>(x[i], e), d[i]);
 #pragma unroll
-  for (int s = 0; s < kSlices; ++s) {
+  for (int s = 0; s < S; ++s) {
     uint4 v;
     v.x = bf16_pair(d[0][s], d[1][s]);
     v.y = bf16_pair(d[2][s], d[3][s]);
     v.z = bf16_pair(d[4][s], d[5][s]);
     v.w = bf16_pair(d[6][s], d[7][s]);
-    *reinterpret_cast<uint4*>(planes + plane_off(s, kc, rb, nkc, nrb, rr, k0)) = v;
+    *reinterpret_cast<uint4*>(planes + plane_off<S>(s, kc, rb, nkc, nrb, rr, k0)) = v;
   }
 }
 
@@ -81,15 +90,43 @@ __device__ __forceinline__ double scale2(double v, int k) {
   return v * pow2i(k1) * pow2i(k - k1);
 }
 
-// the value of a batched product's integer sum (gemm_nt_batched), e = the two
-// rows' scale exponents - 38 - batch_shift: one FP64 conversion, the scale added
-// to the exponent field while the result stays normal
-__device__ __forceinline__ double sum_value(long long v, int e) {
-  const double d = (double)v;
+// h 2^32 + l rounded to the nearest double (ties to even), by integer operations
+__device__ __forceinline__ double round_sum(long long h, long long l) {
+  h += l >> 32;
+  uint32_t lo = (uint32_t)l;  // the value is h 2^32 + lo
+  const bool neg = h < 0;
+  if (neg) {
+    h = -h - (lo != 0u);
+    lo = 0u - lo;
+  }
+  unsigned long long m;  // the leading 64 bits; lost: some bit below them is set
+  int top;               // exponent of the leading bit
+  bool lost = false;
+  if (h != 0) {
+    const int z = __clzll(h);  // >= 1
+    m = ((unsigned long long)h << z) | (((unsigned long long)lo << 32) >> (64 - z));
+    lost = z < 32 && (lo << z) != 0u;
+    top = 95 - z;
+  } else {
+    if (lo == 0u) return 0.0;
+    const int z = __clz((int)lo);
+    m = (unsigned long long)lo << (32 + z);
+    top = 31 - z;
+  }
+  const unsigned rest = (unsigned)m & 0x7FFu;
+  unsigned long long r = m >> 11;  // 53 bits
+  r += rest > 0x400u || (rest == 0x400u && (lost || (r & 1)));
+  // r's leading bit adds one to the exponent field
+  const unsigned long long bits = ((unsigned long long)(top + 1022) << 52) + r;
+  return __longlong_as_double((long long)(bits | (neg ? 1ULL << 63 : 0ULL)));
+}
+
+// d 2^e: the scale is added to the exponent field while the result stays normal
+__device__ __forceinline__ double scaled(double d, int e) {
   const long long bits = __double_as_longlong(d);
-  const int ex = (int)((bits >> 52) & 0x7FF) + e;
-  if (v == 0) return 0.0;
-  if (ex > 0 && ex < 0x7FF) return __longlong_as_double(bits + ((long long)e << 52));
+  const int ex = (int)((bits >> 52) & 0x7FF);
+  if (ex == 0) return d;  // a sum of integers: zero
+  if (ex + e > 0 && ex + e < 0x7FF) return __longlong_as_double(bits + ((long long)e << 52));
   return scale2(d, e);
 }
 

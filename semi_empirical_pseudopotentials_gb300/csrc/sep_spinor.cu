@@ -250,13 +250,13 @@ __global__ void __launch_bounds__(kTS)
 // ---- the sums on the tensor cores -----------------------------------------
 // Per atom the sums are a matrix product, (K: n x n) times (conj(Y) psi: n x
 // 12 per spinor, the real and imaginary parts of the six products), done for
-// all atoms at once by the digit-split contraction of sep_ozaki.cu: K's digit
+// all atoms at once by the batched contraction of sep_ozaki.cu: K's digit
 // planes are kept with the operator, the products' are written per apply.
-// 64 atoms x 340 points, 4 spinors: digits of the products 27 us, contraction
-// 63 us (two waves of tiles, K's digits read once: 121 MB), contributions 18 us,
-// where the FMAs took 736 us.  Sums agree with the FP64 kernel's to 1e-15 of
-// the largest and with 64-bit references as well as they do.
-
+// Accuracy: a term's error is below 2^-60 of the product of the largest K of its
+// row and the largest of its product over the list, so a row's sums are no worse
+// than by FP64 FMAs unless every one of its terms lies far below that product:
+// K grows towards the atom, so that is where psi falls towards it by orders of
+// magnitude.  vso_row_covered finds such rows, and they take the FP64 sums.
 // scale exponent of every row of every K (mpad rows per atom); *bad: some
 // value is not finite
 __global__ void k_vso_k_expo(const long* __restrict__ nl, const double* __restrict__ km,
@@ -274,6 +274,35 @@ __global__ void k_vso_k_expo(const long* __restrict__ nl, const double* __restri
   }
 }
 
+// the four largest values of every row of every K: columns and exponent fields
+__global__ void __launch_bounds__(kTS)
+    k_vso_k_top(const long* __restrict__ nl, const double* __restrict__ km, long nmax, long ld,
+                long mpad, int4* __restrict__ top, ushort4* __restrict__ top_exp) {
+  const long a = blockIdx.x, n = nl[a], j1 = (long)blockIdx.y * kTS + threadIdx.x;
+  if (j1 >= n) return;
+  const double* col = km + (size_t)a * nmax * ld + j1;
+  unsigned long long v[4] = {};  // the bits of |K| order as |K| does
+  int at[4] = {};
+  for (long j2 = 0; j2 < n; ++j2) {
+    unsigned long long x = (unsigned long long)__double_as_longlong(col[(size_t)j2 * ld]) << 1 >> 1;
+    int c = (int)j2;
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (x > v[q]) {
+        const unsigned long long y = v[q];
+        const int d = at[q];
+        v[q] = x;
+        at[q] = c;
+        x = y;
+        c = d;
+      }
+  }
+  top[a * mpad + j1] = make_int4(at[0], at[1], at[2], at[3]);
+  top_exp[a * mpad + j1] =
+      make_ushort4((unsigned short)(v[0] >> 52), (unsigned short)(v[1] >> 52),
+                   (unsigned short)(v[2] >> 52), (unsigned short)(v[3] >> 52));
+}
+
 // digit planes of every K: block (16 values of j2, 128 rows)
 constexpr int kSliceT = sep::oz::kBlockRows * sep::oz::kChunkK / 8;
 __global__ void __launch_bounds__(kSliceT)
@@ -287,7 +316,8 @@ __global__ void __launch_bounds__(kSliceT)
 #pragma unroll
   for (int i = 0; i < 8; ++i)
     x[i] = j1 < n && j2 + i < n ? km[((size_t)a * nmax + j1) * ld + j2 + i] : 0.0;
-  sep::oz::store_digits8(x, expo[rb * sep::oz::kBlockRows + rr], planes, kc, rb, nkc, 0, rr, k0);
+  sep::oz::store_digits8<sep::oz::kBatchSlices>(x, expo[rb * sep::oz::kBlockRows + rr], planes, kc,
+                                                rb, nkc, 0, rr, k0);
 }
 
 // product m of a list point, in the order of the sums above
@@ -300,18 +330,21 @@ __device__ __forceinline__ C2 vso_product(const double* __restrict__ psi, long n
 
 // exponents and digit planes of the products: block (atom, spinor) writes the
 // 12 rows 12 s .. of the atom's nb row blocks, zero from the list's end to the
-// last chunk's.  A thread takes one product of eight points; where that covers
-// the list (up to 680 points) they stay in registers between the exponents and
+// last chunk's, and the exponent field of every product (xe, `most` spinors per
+// atom).  A thread takes one product of eight points; where that covers
+// the list (up to 672 points) they stay in registers between the exponents and
 // the digits, beyond it they are formed again.
 constexpr int kSliceX = 512;
 __global__ void __launch_bounds__(kSliceX)
     k_vso_x_slice(const double* __restrict__ psi, long ngrid, long nnlc,
                   const sep_nlc* __restrict__ nlc, const long* __restrict__ nl, long nb, long nkc,
-                  int* __restrict__ expo, uint16_t* __restrict__ planes) {
+                  long most, int* __restrict__ expo, uint16_t* __restrict__ xe,
+                  uint16_t* __restrict__ planes) {
   __shared__ int top[12];
   const long a = blockIdx.x, n = nl[a];
   const int row0 = 12 * blockIdx.y, nt = blockDim.x;
   psi += (size_t)blockIdx.y * 4 * (size_t)ngrid;
+  xe += ((size_t)a * most + blockIdx.y) * (size_t)nkc * sep::oz::kChunkK * 8;
   const sep_nlc* base = nlc + a * nnlc;
   if (threadIdx.x < 12) top[threadIdx.x] = 0;
   __syncthreads();
@@ -334,8 +367,10 @@ __global__ void __launch_bounds__(kSliceX)
     int ex = 0, ey = 0;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      ex = max(ex, sep::oz::exp_field(x[i]));
-      ey = max(ey, sep::oz::exp_field(y[i]));
+      const int fx = sep::oz::exp_field(x[i]), fy = sep::oz::exp_field(y[i]);
+      ex = max(ex, fx);
+      ey = max(ey, fy);
+      xe[(8 * (t - m * groups) + i) * 8 + m] = (uint16_t)max(fx, fy);
     }
     atomicMax(&top[2 * m], ex);
     atomicMax(&top[2 * m + 1], ey);
@@ -349,24 +384,66 @@ __global__ void __launch_bounds__(kSliceX)
     const int r = row0 + 2 * m;  // even: both rows are in one block
     const long rb = a * nb + r / sep::oz::kBlockRows;
     const int rr = r % sep::oz::kBlockRows;
-    sep::oz::store_digits8(x, sep::oz::scale_of(top[2 * m]), planes, g / 2, rb, nkc, 0, rr,
-                           g % 2 * 8);
-    sep::oz::store_digits8(y, sep::oz::scale_of(top[2 * m + 1]), planes, g / 2, rb, nkc, 0, rr + 1,
-                           g % 2 * 8);
+    constexpr int kS = sep::oz::kBatchSlices;
+    sep::oz::store_digits8<kS>(x, sep::oz::scale_of(top[2 * m]), planes, g / 2, rb, nkc, 0, rr,
+                               g % 2 * 8);
+    sep::oz::store_digits8<kS>(y, sep::oz::scale_of(top[2 * m + 1]), planes, g / 2, rb, nkc, 0,
+                               rr + 1, g % 2 * 8);
   }
+}
+
+// whether the digits hold the terms of a row (K's scale exponent ea) well enough:
+// for either component (products 0-2, 3-5; eb: their scale exponents) one of the
+// terms of the row's four largest K is at least 2^-kCover of the bound 2^(ea +
+// eb) that the digits' error is measured by, or the component is zero.
+// Error of Vso psi against extended precision, relative to the sum of the
+// absolute values added up, root mean square over a list of 590 points (FP64
+// FMAs): normally distributed psi 6e-18 (1.8e-17), constant 4e-18 (2.6e-17), psi
+// falling by nine decades away from the atom 6e-17 (8e-17), by three towards it
+// 4.9e-18 (6.9e-18, some rows not covered), by nine towards it the FP64 sums for
+// every row.  With kCover 8 a point of the fourth erred by 1.6 times the FP64
+// sums' worst; without the test a list near a grid point errs by 1e-9.
+constexpr int kCover = 6;
+__device__ __forceinline__ bool vso_row_covered(const uint16_t* __restrict__ xe, int4 at, ushort4 k,
+                                                int ea, const int* __restrict__ eb) {
+  constexpr int zero = sep::oz::scale_of(0);
+  if (ea == zero) return true;
+  const int col[4] = {at.x, at.y, at.z, at.w};
+  const int kf[4] = {k.x, k.y, k.z, k.w};
+  int best[2] = {-4096, -4096};
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const uint4 f = *reinterpret_cast<const uint4*>(xe + (size_t)col[q] * 8);
+    const int x[2] = {(int)max(max(f.x & 0xFFFFu, f.x >> 16), f.y & 0xFFFFu),
+                      (int)max(max(f.y >> 16, f.z & 0xFFFFu), f.z >> 16)};
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+      if (x[c] > 0 && kf[q] > 0) best[c] = max(best[c], x[c] + kf[q] - 2044);
+  }
+  bool ok = true;
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    int e = eb[6 * c];
+#pragma unroll
+    for (int m = 1; m < 6; ++m) e = max(e, eb[6 * c + m]);
+    ok = ok && (e == zero || best[c] >= ea + e - kCover);
+  }
+  return ok;
 }
 
 // contributions from the sums: block (atom, 64 points j, spinor s); sums[(a mpad
 // + j) ldc + 12 s + 2 m] (re, im), scaled by the exponents of K's row and of the
-// product's (e0: the rest).  Products with an infinite or NaN value have no
-// digits: an (atom, spinor) that holds one takes the FP64 sums, which pass it on.
+// product's.  Products with an infinite or NaN value have no digits: an (atom,
+// spinor) that holds one takes the FP64 sums, which pass it on, and so do the
+// rows whose terms the digits do not cover.
 __global__ void __launch_bounds__(kTS)
-    k_vso_combine(const long long* __restrict__ sums, const int* __restrict__ ea,
-                  const int* __restrict__ eb, long xpad, int e0, long ldc, long mpad,
-                  const double* __restrict__ psi, long ngrid, long nnlc,
-                  const sep_nlc* __restrict__ nlc, const long* __restrict__ nl,
-                  const double* __restrict__ km, long nmax, long ld, double tmp,
-                  double2* __restrict__ contrib) {
+    k_vso_combine(const double* __restrict__ sums, const int* __restrict__ ea,
+                  const int* __restrict__ eb, long xpad, const int4* __restrict__ top,
+                  const ushort4* __restrict__ top_exp, const uint16_t* __restrict__ xe,
+                  long xe_spinor, long most, long ldc, long mpad, const double* __restrict__ psi,
+                  long ngrid, long nnlc, const sep_nlc* __restrict__ nlc,
+                  const long* __restrict__ nl, const double* __restrict__ km, long nmax, long ld,
+                  double tmp, double2* __restrict__ contrib) {
   __shared__ C2 sx[kTS][6];
   const long a = blockIdx.x, n = nl[a];
   if ((long)blockIdx.y * kTS >= n) return;
@@ -374,30 +451,31 @@ __global__ void __launch_bounds__(kTS)
   const long j = (long)blockIdx.y * kTS + threadIdx.x;
   const bool act = j < n;
   eb += a * xpad + 12 * blockIdx.z;
-  C2 acc[6];
-  bool finite = true;
+  xe += ((size_t)a * most + blockIdx.z) * (size_t)xe_spinor;
+  bool ok = true;
 #pragma unroll
-  for (int m = 0; m < 12; ++m) finite = finite && eb[m] != sep::oz::scale_of(0x7ff);
-  if (!finite) {  // the same in the whole block
+  for (int m = 0; m < 12; ++m) ok = ok && eb[m] != sep::oz::scale_of(0x7ff);
+  const long r = a * mpad + j;
+  if (ok && act) ok = vso_row_covered(xe, top[r], top_exp[r], ea[r], eb);
+  C2 acc[6];
+  if (__syncthreads_or(!ok))
     vso_stored_sums(psi + (size_t)blockIdx.z * 4 * (size_t)ngrid, ngrid, base, n,
                     km + (size_t)a * nmax * ld + j, ld, act, sx, acc);
-  } else if (act) {
-    const long long* row = sums + (size_t)(a * mpad + j) * ldc + 12 * blockIdx.z;
-    const int e = ea[a * mpad + j] + e0;
+  if (!act) return;
+  if (ok) {
+    const double* row = sums + (size_t)r * ldc + 12 * blockIdx.z;
+    const int e = ea[r] - sep::oz::kBatchUnit;
 #pragma unroll
     for (int m = 0; m < 6; ++m) {
-      const longlong2 v = *reinterpret_cast<const longlong2*>(row + 2 * m);
-      acc[m] = {sep::oz::sum_value(v.x, e + eb[2 * m]),
-                sep::oz::sum_value(v.y, e + eb[2 * m + 1])};
+      const double2 v = *reinterpret_cast<const double2*>(row + 2 * m);
+      acc[m] = {sep::oz::scaled(v.x, e + eb[2 * m]), sep::oz::scaled(v.y, e + eb[2 * m + 1])};
     }
   }
-  if (act) {
-    C2 up, dn;
-    vso_gauss_point(base[j], tmp, acc, up, dn);
-    double2* o = contrib + 2 * (((size_t)blockIdx.z * gridDim.x + a) * nmax + j);
-    o[0] = make_double2(up.re, up.im);
-    o[1] = make_double2(dn.re, dn.im);
-  }
+  C2 up, dn;
+  vso_gauss_point(base[j], tmp, acc, up, dn);
+  double2* o = contrib + 2 * (((size_t)blockIdx.z * gridDim.x + a) * nmax + j);
+  o[0] = make_double2(up.re, up.im);
+  o[1] = make_double2(dn.re, dn.im);
 }
 
 // Vso psi of every grid point from the list points' contributions: point g
@@ -532,6 +610,8 @@ bool VsoTensor::fits(long natom, long nmax) {
   return natom > 0 && nmax > 0 && (double)natom * mb <= 65535.0;
 }
 
+long VsoTensor::spinors() const { return nb * oz::kBlockRows / 12; }
+
 size_t VsoTensor::carve(void* base, long natom_, long nmax_) {
   natom = natom_;
   nmax = nmax_;
@@ -539,7 +619,8 @@ size_t VsoTensor::carve(void* base, long natom_, long nmax_) {
   nkc = (nmax + oz::kChunkK - 1) / oz::kChunkK;
   // 128 columns of products at a time per block of B: as many blocks as stay
   // below half a gigabyte, at most 4 (42 spinors)
-  const double per = (double)natom * ((double)nkc * oz::kBlockElems * 2 + mb * 128.0 * 1024.0);
+  constexpr int elems = oz::block_elems(oz::kBatchSlices);
+  const double per = (double)natom * ((double)nkc * elems * 2 + mb * 128.0 * 1024.0);
   nb = (long)std::max(1.0, std::min(4.0, 536870912.0 / per));
   char* p = static_cast<char*>(base);
   auto take = [&](size_t bytes) {
@@ -547,13 +628,17 @@ size_t VsoTensor::carve(void* base, long natom_, long nmax_) {
     p += (bytes + 255) & ~(size_t)255;
     return q;
   };
-  const size_t blk = sizeof(uint16_t) * (size_t)nkc * oz::kBlockElems;
+  const size_t blk = sizeof(uint16_t) * (size_t)nkc * elems;
   ka = reinterpret_cast<uint16_t*>(take(blk * natom * mb));
   xb = reinterpret_cast<uint16_t*>(take(blk * natom * nb));
   ea = reinterpret_cast<int*>(take(sizeof(int) * natom * mb * oz::kBlockRows));
   eb = reinterpret_cast<int*>(take(sizeof(int) * natom * nb * oz::kBlockRows));
-  sums = reinterpret_cast<long long*>(
-      take(sizeof(long long) * (size_t)(natom * mb * oz::kBlockRows) * nb * oz::kBlockRows));
+  top = reinterpret_cast<int4*>(take(sizeof(int4) * natom * mb * oz::kBlockRows));
+  top_exp = reinterpret_cast<ushort4*>(take(sizeof(ushort4) * natom * mb * oz::kBlockRows));
+  xe = reinterpret_cast<uint16_t*>(
+      take(sizeof(uint16_t) * 8 * (size_t)natom * spinors() * nkc * oz::kChunkK));
+  sums = reinterpret_cast<double*>(
+      take(sizeof(double) * (size_t)(natom * mb * oz::kBlockRows) * nb * oz::kBlockRows));
   err = reinterpret_cast<int*>(take(2 * sizeof(int)));
   return (size_t)(p - static_cast<char*>(base));
 }
@@ -565,6 +650,8 @@ cudaError_t spinor_vso_planes(const VsoTensor& v, const long* nl, const double* 
   if (e != cudaSuccess) return e;
   k_vso_k_expo<<<(unsigned)(v.natom * mpad), 32, 0, st>>>(nl, km, v.nmax, ld, mpad, v.ea,
                                                           v.err + 1);
+  k_vso_k_top<<<dim3((unsigned)v.natom, (unsigned)((v.nmax + kTS - 1) / kTS)), kTS, 0, st>>>(
+      nl, km, v.nmax, ld, mpad, v.top, v.top_exp);
   k_vso_k_slice<<<dim3((unsigned)v.nkc, (unsigned)(v.natom * v.mb)), kSliceT, 0, st>>>(
       nl, km, v.nmax, ld, v.mb, v.ea, v.ka, v.nkc);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
@@ -581,13 +668,14 @@ cudaError_t spinor_vso_kept(const double* psi, long ngrid, long nsp, long natom,
   double2* cb = reinterpret_cast<double2*>(contrib);
   if (tensor) {
     const VsoTensor& v = *tensor;
-    const long most = v.nb * oz::kBlockRows / 12;
+    const long most = v.spinors();
     for (long s0 = 0; s0 < nsp; s0 += most) {
       const long k = std::min(most, nsp - s0), nb = (12 * k + oz::kBlockRows - 1) / oz::kBlockRows;
       const int items = (int)(6 * v.nkc * (oz::kChunkK / 8));
       k_vso_x_slice<<<dim3((unsigned)natom, (unsigned)k), std::min(kSliceX, (items + 31) / 32 * 32),
                       0, st>>>(
-          psi + (size_t)s0 * 4 * ngrid, ngrid, nnlc, nlc, nl, nb, v.nkc, v.eb, v.xb);
+          psi + (size_t)s0 * 4 * ngrid, ngrid, nnlc, nlc, nl, nb, v.nkc, most, v.eb, v.xe,
+          v.xb);
       oz::Planes A, B;
       A.d = v.ka;
       A.expo = v.ea;
@@ -601,9 +689,10 @@ cudaError_t spinor_vso_kept(const double* psi, long ngrid, long nsp, long natom,
           oz::gemm_nt_batched(A, B, (int)natom, 12 * k, v.sums, 12 * k, v.err, st);
       if (e != cudaSuccess) return e;
       k_vso_combine<<<dim3((unsigned)natom, (unsigned)((nmax + kTS - 1) / kTS), (unsigned)k), kTS, 0,
-                      st>>>(v.sums, v.ea, v.eb, nb * oz::kBlockRows, -38 - oz::batch_shift(v.nkc),
-                            12 * k, v.mb * oz::kBlockRows, psi + (size_t)s0 * 4 * ngrid, ngrid, nnlc,
-                            nlc, nl, km, nmax, ld, tmp, cb + (size_t)s0 * 2 * (size_t)(natom * nmax));
+                      st>>>(v.sums, v.ea, v.eb, nb * oz::kBlockRows, v.top, v.top_exp, v.xe,
+                            v.nkc * oz::kChunkK * 8, most, 12 * k, v.mb * oz::kBlockRows,
+                            psi + (size_t)s0 * 4 * ngrid, ngrid, nnlc, nlc, nl, km, nmax, ld, tmp,
+                            cb + (size_t)s0 * 2 * (size_t)(natom * nmax));
     }
   } else {
     const dim3 g((unsigned)natom, (unsigned)((nmax + kTS - 1) / kTS), (unsigned)nsp);

@@ -19,9 +19,13 @@ struct VsoTensor {
   uint16_t* ka = nullptr;        // K's planes
   uint16_t* xb = nullptr;        // the products' planes
   int *ea = nullptr, *eb = nullptr;
-  long long* sums = nullptr;  // natom mb 128 x (nb 128)
+  int4* top = nullptr;       // per row of K: its four largest values' columns
+  ushort4* top_exp = nullptr;  // and their exponent fields
+  uint16_t* xe = nullptr;    // exponent field of every product: [atom][spinor][point][8]
+  double* sums = nullptr;    // natom mb 128 x (nb 128)
   int* err = nullptr;      // the contraction's status word, and one more
   static bool fits(long natom, long nmax);  // within the launches' limits
+  long spinors() const;  // that one contraction takes: nb 128 / 12
   // sets the sizes and the parts of base; returns the bytes
   size_t carve(void* base, long natom, long nmax);
 };

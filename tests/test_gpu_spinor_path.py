@@ -350,3 +350,106 @@ def test_states_with_values_that_are_not_finite(bad):
     assert np.array_equal(~np.isfinite(got[1, ngrid:]), lost)
     assert np.array_equal(got[1, ngrid:][~lost], clean[1, ngrid:][~lost])
     assert np.array_equal(got[[0, 2]], clean[[0, 2]])
+
+
+def _list_states(rng, kind, r, ngrid, points):
+    """A spinor over the grid whose values on a list's points (radii r) are normal,
+    constant, falling by nine or three decades towards or away from the atom,
+    zero on the inner half, or of random magnitude."""
+    psi = rng.normal(size=2 * ngrid) + 1j * rng.normal(size=2 * ngrid)
+    out = r / r.max()
+    f = {"normal": np.ones_like(r), "smooth": None, "towards9": 10.0 ** (9 * (out - 1)),
+         "towards3": 10.0 ** (3 * (out - 1)), "away9": 10.0 ** (-9 * out),
+         "node": np.where(out < 0.5, 0.0, 1.0), "any9": 10.0 ** rng.uniform(-9, 0, len(r))}[kind]
+    for c in range(2):
+        at = c * ngrid + points
+        psi[at] = (1.0 + 0.3j) * (1 - 2 * c) if f is None else psi[at] * f
+    return psi
+
+
+def _row_errors(got, e, k, psi, ngrid, sigma, dv, held=None):
+    """Per list point: the error of Vso psi against extended precision over the sum
+    of the absolute values of what it adds up.  held: K's rows and the products
+    rounded to that many bits below their largest, and summed exactly, instead."""
+    LD = np.longdouble
+    j, n = e["jxyz"], len(e)
+    tmp = 0.5 / np.sqrt(2 * np.pi * sigma ** 2) * dv
+    y = [e[f] for f in ("y11", "y10", "y1_1")]
+    kl = k.astype(LD)
+    if held:
+        unit = np.ldexp(LD(1), np.frexp(k.max(1))[1] - held)
+        kl = np.rint(kl / unit[:, None]) * unit[:, None]
+    s, a = {}, {}
+    for c in range(2):
+        p = psi[c * ngrid + j]
+        for m in range(3):
+            yr, yi, pr, pi = (v.astype(LD) for v in (y[m].real, y[m].imag, p.real, p.imag))
+            x = [yr * pr + yi * pi, yr * pi - yi * pr]
+            a[m, c] = kl @ (np.abs(yr * pr) + np.abs(yi * pi) + np.abs(yr * pi) + np.abs(yi * pr))
+            if held:
+                for q in range(2):
+                    u = np.ldexp(LD(1), int(np.frexp(np.abs(x[q]).max())[1]) - held)
+                    x[q] = np.rint(x[q] / u) * u
+            s[m, c] = [kl @ v for v in x]
+    w = {(0, 0): [(0, (0, 0), 1), (2, (2, 0), -1), (1, (0, 1), 2 ** 0.5), (2, (1, 1), 2 ** 0.5)],
+         (1, 0): [(0, (0, 1), -1), (2, (2, 1), -1), (1, (2, 0), 2 ** 0.5), (0, (1, 0), 2 ** 0.5)]}
+    err, size = np.zeros(n, LD), np.zeros(n, LD)
+    for (c, _), terms in w.items():
+        re, im = np.zeros(n, LD), np.zeros(n, LD)
+        for m, at, f in terms:
+            yr, yi = y[m].real.astype(LD), y[m].imag.astype(LD)
+            sr, si = s[at]
+            g = LD(np.sqrt(LD(2))) if abs(f) > 1 else LD(f)
+            re += g * tmp * (yr * sr - yi * si)
+            im += g * tmp * (yr * si + yi * sr)
+            size += abs(g) * tmp * (np.abs(yr) + np.abs(yi)) * a[at]
+        if held:
+            return re, im, size
+        v = got[c * ngrid + j]
+        err = np.maximum(err, np.maximum(np.abs(v.real - re), np.abs(v.imag - im)))
+    return (err / size).astype(float)
+
+
+@pytest.mark.parametrize("at,rc,take", [((0.13, -0.2, 0.07), 2.6, None), ((0.005, 0.0, 0.0), 2.6, None),
+                                        ((0.0, 0.0, 0.0), 2.6, None), ((0.2, 0.2, 0.1), 3.0, 672),
+                                        ((0.2, 0.2, 0.1), 3.0, 673), ((0.1, 0.2, 0.25), 1.4, None)])
+def test_tensor_core_sums_are_as_accurate_as_the_fp64_ones(at, rc, take):
+    """Vso psi of one atom (no potential, no kinetic energy to speak of) against
+    extended precision, point by point, relative to the sum of the absolute
+    values added up there: on the tensor cores it errs no more than by FP64 FMAs
+    (root mean square over the points, a tenth for chance where nearly every row
+    takes the FP64 sums; half as much again for the worst point).
+    Atoms between grid points, near one and on one; lists of 92 to 673 points;
+    states that are steep towards the atom, where K is largest and a split that
+    is relative to the list's largest value alone loses their digits."""
+    rng = np.random.default_rng(11)
+    dims, h = (20, 20, 20), 0.5
+    ngrid = int(np.prod(dims))
+    ax = [(np.arange(d) - d // 2) * h for d in dims]
+    nlc, nl = spinor.neighbour_lists(*ax, [at], [0.1], rc ** 2)
+    nl = np.minimum(nl, take or nl)
+    e = nlc[0, :nl[0]]
+    assert len(e) == (take or len(e)) and len(e) >= 64
+    r = np.where(e["r2"] > 1e10, 0.0, e["r"])
+    k = (0.5 * (e["Vr"][:, None] + e["Vr"]) * np.exp(-((e["r"][:, None] - e["r"]) / h) ** 2 / 2)
+         / (0.5 * (e["r2"][:, None] + e["r2"])))
+    kinds = ["normal", "smooth", "towards9", "towards3", "away9", "node", "any9"]
+    psi = np.stack([_list_states(rng, q, r, ngrid, e["jxyz"]) for q in kinds])
+    ctx = binding.Context(dims, (h, h, h), potl=np.zeros(ngrid), ekinmax=1e-200)
+    out = {}
+    for route in ("tc", "f64"):
+        ctx.set_subspace(route)
+        out[route] = spinor.SpinorPath(ctx, nlc, nl, sigma=h).hamiltonian(psi)
+    ctx.close()
+    for q in range(len(kinds)):
+        err = {t: _row_errors(out[t][q], e, k, psi[q], ngrid, h, h ** 3) for t in out}
+        rms = {t: np.sqrt((v ** 2).mean()) for t, v in err.items()}
+        assert rms["tc"] <= 1.1 * rms["f64"]
+        assert err["tc"].max() <= 1.5 * err["f64"].max()
+        assert err["f64"].max() <= (len(e) + 20) * 2.0 ** -53
+    # the comparison sees a digit less in each value
+    re, im, size = _row_errors(None, e, k, psi[0], ngrid, h, h ** 3, held=47)
+    full = _row_errors(None, e, k, psi[0], ngrid, h, h ** 3, held=63)
+    lost = np.maximum(np.abs(re - full[0]), np.abs(im - full[1])) / size
+    err = _row_errors(out["f64"][0], e, k, psi[0], ngrid, h, h ** 3)
+    assert np.sqrt((lost ** 2).mean()) > np.sqrt((err ** 2).mean())
