@@ -610,6 +610,21 @@ bool VsoTensor::fits(long natom, long nmax) {
   return natom > 0 && nmax > 0 && (double)natom * mb <= 65535.0;
 }
 
+// Below 64 points both take about as long (8 atoms, 4 spinors: 39 and 40 us at 64).
+// From there on, in us for 4 spinors, fitted to 64 and 1000 atoms with longest
+// lists of 67 to 356 points, of which all to one in fifty lists were long and the
+// rest had 10 points: the FMAs wait for the longest list and then take the pairs
+// (64 atoms x 346 points 743, one such list among 64 175, 20 of them among 1000
+// 587); the contraction takes every list as long as the longest (129, 113, 913).
+// The rule misses the faster of the two by a tenth at most there.
+bool VsoTensor::pays(long natom, long nmax, double pairs) {
+  const double na = (double)natom;
+  const double mb = (double)((nmax + oz::kBlockRows - 1) / oz::kBlockRows);
+  const double nkc = (double)((nmax + oz::kChunkK - 1) / oz::kChunkK);
+  return nmax >= 64 &&
+         0.5 * (double)nmax + 8.8e-5 * pairs > 25.0 + 0.12 * na + 0.0095 * na * mb * nkc;
+}
+
 long VsoTensor::spinors() const { return nb * oz::kBlockRows / 12; }
 
 size_t VsoTensor::carve(void* base, long natom_, long nmax_) {

@@ -25,6 +25,8 @@ struct VsoTensor {
   double* sums = nullptr;    // natom mb 128 x (nb 128)
   int* err = nullptr;      // the contraction's status word, and one more
   static bool fits(long natom, long nmax);  // within the launches' limits
+  // whether an apply takes less time so than by FP64 FMAs (pairs: sum of nl^2)
+  static bool pays(long natom, long nmax, double pairs);
   long spinors() const;  // that one contraction takes: nb 128 / 12
   // sets the sizes and the parts of base; returns the bytes
   size_t carve(void* base, long natom, long nmax);

@@ -161,14 +161,10 @@ size_t vso_scratch(const sep_ctx* c) {
   return sizeof(double) * 4 * (size_t)c->so_natom * (size_t)c->so_kmax;
 }
 
-// The kept operator's sums go to the tensor cores from lists of 64 points on:
-// there both routes take about 40 us (8 atoms, 4 spinors: 39.3 us on the tensor
-// cores, 40.2 us by FP64 FMAs).  The FP64 kernel's time grows with the list
-// (0.7 us per point, and with the pairs once they fill the chip) from 13 us at 10
-// points, the tensor route's stays near 35 us up to 100 points: 64 atoms x 80
-// points 42 against 64 us, x 340 points 109 against 736.
+// The kept operator's sums go to the tensor cores where that takes less time
+// (VsoTensor::pays), the planes fit, and the subspace contractions do.
 bool vso_on_tensor_cores(const sep_ctx* c) {
-  return c->so_planes && c->subspace_tc && c->so_kmax >= 64;
+  return c->so_planes && c->subspace_tc;
 }
 
 // the status of the contractions since the last check
@@ -525,9 +521,11 @@ int spinor_set_operator(sep_ctx* c, long natom, long nnlc, const sep_nlc* nlc, c
   // which the filter's history needs more.
   if (!flagkb && natom > 0) {
     long nmax = 0, points = 0;
+    double pairs = 0.0;
     for (long a = 0; a < natom; ++a) {
       nmax = std::max(nmax, nl[a]);
       points += nl[a];
+      pairs += (double)nl[a] * (double)nl[a];
     }
     const long ld = (nmax + 31) / 32 * 32;
     const double bytes = 8.0 * (double)natom * (double)nmax * (double)ld;
@@ -554,7 +552,9 @@ int spinor_set_operator(sep_ctx* c, long natom, long nnlc, const sep_nlc* nlc, c
         c->so_kmax = nmax;
         c->so_kld = ld;
         VsoTensor& v = c->so_tensor;
-        const size_t tb = nmax >= 64 && VsoTensor::fits(natom, nmax) ? v.carve(nullptr, natom, nmax) : 0;
+        const size_t tb = VsoTensor::fits(natom, nmax) && VsoTensor::pays(natom, nmax, pairs)
+                              ? v.carve(nullptr, natom, nmax)
+                              : 0;
         if (tb > 0 && (double)tb <= 0.125 * (double)(free_device_bytes() + c->w_sot.bytes) &&
             c->w_sot.ensure(tb) == cudaSuccess) {
           v.carve(c->w_sot.p, natom, nmax);

@@ -453,3 +453,27 @@ def test_tensor_core_sums_are_as_accurate_as_the_fp64_ones(at, rc, take):
     lost = np.maximum(np.abs(re - full[0]), np.abs(im - full[1])) / size
     err = _row_errors(out["f64"][0], e, k, psi[0], ngrid, h, h ** 3)
     assert np.sqrt((lost ** 2).mean()) > np.sqrt((err ** 2).mean())
+
+
+def test_one_long_list_among_many_short_ones():
+    """The contraction takes every list as long as the longest, so an operator with
+    one long list among a thousand short ones stays with the FP64 sums: the same
+    bits with the tensor cores switched on and off, where lists that are all long
+    differ in the last ones."""
+    rng = np.random.default_rng(12)
+    dims, h = (16, 16, 20), 0.5
+    ngrid = int(np.prod(dims))
+    psi = rng.normal(size=(2, 2 * ngrid)) + 1j * rng.normal(size=(2, 2 * ngrid))
+    ctx = binding.Context(dims, (h, h, h), potl=np.zeros(ngrid), ekinmax=20.0)
+    for counts, same in (((300,) + (5,) * 999, True), ((300,) * 20, False)):
+        nlc = np.zeros((len(counts), 300), dtype=spinor.NLC_DTYPE)
+        for a, n in enumerate(counts):
+            nlc[a, :n] = _list_entries(rng, n, ngrid)
+        path = spinor.SpinorPath(ctx, nlc, np.array(counts, dtype=np.int64), sigma=h)
+        out = []
+        for route in ("tc", "f64"):
+            ctx.set_subspace(route)
+            out.append(path.hamiltonian(psi))
+        assert np.array_equal(*out) == same
+        assert np.abs(out[0] - out[1]).max() <= 1e-13 * np.abs(out[0]).max()
+    ctx.close()
