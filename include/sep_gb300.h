@@ -533,9 +533,14 @@ int sep_spinor_neighbour_lists(long nx, long ny, long nz, const double *vx, cons
  * sep_spinor_set_operator: the neighbour lists (natom x nnlc sep_nlc, nl[a]
  *   used per atom, every jxyz on the grid), sigma (Gaussian form) or
  *   flagkb = 1 with elkb (2 natom energies); copied to the device, kept by
- *   the context until set again.  The Gaussian form also keeps its kernel
- *   K(j1, j2) of every atom (8 nl^2 bytes each) when that is at most an
- *   eighth of the free device memory, and forms it on each apply otherwise.
+ *   the context until set again.  For speed the Gaussian form also keeps its
+ *   kernel K(j1, j2), 8 natom nmax^2 bytes with nmax the longest list rounded
+ *   up to 32, when that is at most an eighth of the free device memory; where
+ *   the tensor cores do the sums (lists of 64 points on, unless one long list
+ *   stands among many short ones), K's digits and their workspace, two to
+ *   three times that and at most another eighth; and per spinor of a call 32 natom
+ *   nmax bytes.  A call of this context that would run out of device memory
+ *   gives all of it back first; K is then formed on each apply, more slowly.
  *   Refused arguments leave the operator set before as it was; a call that
  *   fails after that (out of memory) leaves the context without one.
  * sep_spinor_hamiltonian: hpsi = H psi for nspinors spinors

@@ -142,7 +142,7 @@ int to_device(sep_ctx* c, DevBuf& b, const double* h, size_t count) {
     for (auto& g : c->graphs)
       if (g.exec) cudaGraphExecDestroy(g.exec);
     c->graphs.clear();
-    CK(b.ensure(count * sizeof(double)));
+    CK(ensure_or_release(c, b, count * sizeof(double)));
   }
   CK(cudaMemcpyAsync(b.p, h, count * sizeof(double), cudaMemcpyHostToDevice, c->stream));
   return kOk;
@@ -153,7 +153,7 @@ int ensure_buf(sep_ctx* c, DevBuf& b, size_t bytes) {
     for (auto& g : c->graphs)
       if (g.exec) cudaGraphExecDestroy(g.exec);
     c->graphs.clear();
-    CK(b.ensure(bytes));
+    CK(ensure_or_release(c, b, bytes));
   }
   return kOk;
 }

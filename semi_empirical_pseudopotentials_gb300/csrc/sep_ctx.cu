@@ -12,6 +12,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <initializer_list>
 #include <type_traits>
 #include <utility>
 #include <vector>
@@ -114,7 +115,7 @@ int grow(sep_ctx* c, DevBuf& b, size_t bytes) {
                     "use sizes that fit it");
   cudaStreamSynchronize(c->stream);
   drop_graphs(c);
-  cudaError_t e = b.ensure(bytes);
+  cudaError_t e = ensure_or_release(c, b, bytes);
   if (e != cudaSuccess) return cuda_fail(e, "workspace allocation", __LINE__);
   return kOk;
 }
@@ -243,9 +244,13 @@ int filter_impl(sep_ctx* c, const double* d_start, long ns, const double* an_re,
       sizeof(T) * accumulator_values<T>(n, ms) * Bc > c->w_acc.bytes) {
     // the workspace has to grow: as many pairs as the free memory holds
     const size_t have = c->w_hist.bytes + c->w_fft.bytes + c->w_acc.bytes;
-    const size_t budget = (size_t)(0.6 * (double)free_device_bytes()) + have;
-    Bc = std::min(Bc, (long long)(budget / per_pair));
+    const auto fit = [&] {
+      return (long long)(((size_t)(0.6 * (double)free_device_bytes()) + have) / per_pair);
+    };
+    Bc = std::min(Bc, fit());
+    if (Bc < 1 && release_kept_operator(c)) Bc = std::min(B, fit());
     if (Bc < 1) return arg_fail("filter: not enough device memory for one pair of states");
+    Bc = std::min<long long>(Bc, 65535);
   }
   RET(grow(c, c->w_hist, sizeof(cx<T>) * (size_t)n * K * Bc));
   RET(grow(c, c->w_fft, sizeof(cx<T>) * (size_t)n * Bc));
@@ -393,10 +398,14 @@ int apply_h_chunked_t(sep_ctx* c, const cx<T>* in, cx<T>* out, long long nst) {
   // the free memory is asked for only where the scratch has to grow: the query
   // costs more than a small grid's passes
   if (sizeof(cx<T>) * (size_t)n * chunk > c->w_fft.bytes) {
-    const long long fit = (long long)((0.25 * (double)free_device_bytes() + c->w_fft.bytes) /
-                                      (sizeof(cx<T>) * (double)n));
-    if (fit < 1) return arg_fail("hamiltonian: not enough device memory");
-    chunk = std::min(chunk, fit);
+    const auto fit = [&] {
+      return (long long)((0.25 * (double)free_device_bytes() + c->w_fft.bytes) /
+                         (sizeof(cx<T>) * (double)n));
+    };
+    long long most = fit();
+    if (most < 1 && release_kept_operator(c)) most = fit();
+    if (most < 1) return arg_fail("hamiltonian: not enough device memory");
+    chunk = std::min(chunk, most);
   }
   RET(grow(c, c->w_fft, sizeof(cx<T>) * (size_t)n * chunk));
   for (long long b0 = 0; b0 < nst; b0 += chunk) {
@@ -439,8 +448,12 @@ int precond_real(sep_ctx* c, double* d_x, long long m, double shift) {
   RET(grow(c, c->w_states, sizeof(cx<double>) * (size_t)n * B));
   RET(grow(c, c->w_states2, sizeof(cx<double>) * (size_t)n * B));
   CK(pack_pairs<double, double>(d_x, m, n, c->w_states.as<cx<double>>(), c->stream));
-  long long chunk = (long long)((0.25 * (double)free_device_bytes() + c->w_fft.bytes) /
-                                (sizeof(cx<double>) * (double)n));
+  const auto fit = [&] {
+    return (long long)((0.25 * (double)free_device_bytes() + c->w_fft.bytes) /
+                       (sizeof(cx<double>) * (double)n));
+  };
+  long long chunk = fit();
+  if (chunk < 1 && release_kept_operator(c)) chunk = fit();
   if (chunk < 1) return arg_fail("preconditioner: not enough device memory");
   chunk = std::min<long long>(chunk, std::min<long long>(B, 4096));
   RET(grow(c, c->w_fft, sizeof(cx<double>) * (size_t)n * chunk));
@@ -595,6 +608,28 @@ int rotate_rows(sep_ctx* c, double* d_psi, long long m, long long k, const doubl
 
 }  // namespace detail
 using namespace detail;
+
+bool release_kept_operator(sep_ctx* c) {
+  const std::initializer_list<DevBuf*> kept = {&c->w_sok, &c->w_sog, &c->w_sot, &c->w_soc};
+  if (std::all_of(kept.begin(), kept.end(), [](DevBuf* b) { return b->bytes == 0; })) return false;
+  cudaStreamSynchronize(c->stream);
+  int err = 0;
+  if (c->so_planes && oz::check_status(c->so_tensor.err, c->stream, &err) == cudaSuccess && err)
+    c->so_err = err;
+  c->so_kmax = 0;
+  c->so_planes = false;
+  for (DevBuf* b : kept) b->release();
+  return true;
+}
+
+cudaError_t ensure_or_release(sep_ctx* c, DevBuf& b, size_t bytes) {
+  cudaError_t e = b.ensure(bytes);
+  if (e == cudaErrorMemoryAllocation && release_kept_operator(c)) {
+    cudaGetLastError();
+    e = b.ensure(bytes);
+  }
+  return e;
+}
 
 int release_filter_workspace_if_short(sep_ctx* c, size_t need) {
   if (free_device_bytes() >= need || c->batch_holds > 0) return kOk;

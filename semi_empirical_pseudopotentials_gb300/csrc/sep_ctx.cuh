@@ -110,6 +110,7 @@ struct sep_ctx {
   sep::DevBuf w_sot;  // with it: K's digit planes and the tensor route's workspace
   sep::VsoTensor so_tensor;
   bool so_planes = false;  // so_tensor holds the operator's planes
+  int so_err = 0;          // status of the contractions before the planes were released
   sep::DevBuf w_soc;  // the list points' contributions, 4 natom so_kmax doubles per spinor
   sep::DevBuf w_nlc, w_nl, w_elkb, w_so, w_so2, w_so3;
   sep::DevBuf w_eigh;  // workspace of the symmetric eigensolver
@@ -141,6 +142,12 @@ int ortho_device(sep_ctx* c, double* d_psi, long m, long* mkept);
 // accumulator grids) and the start states when fewer than `need` bytes of
 // device memory are free; the next filter call allocates them again.
 int release_filter_workspace_if_short(sep_ctx* c, size_t need);
+// Gives back what a spin-orbit operator keeps for speed alone (K, its digits, the
+// contributions); its applies form K in place from then on.  false: nothing kept.
+// For callers whose memory does not suffice: they look again after it.
+bool release_kept_operator(sep_ctx* c);
+// b holds at least bytes, after release_kept_operator if need be
+cudaError_t ensure_or_release(sep_ctx* c, DevBuf& b, size_t bytes);
 // keep_hpsi: also return H psi of the rotated states (rotated with them) in
 // *hpsi when the device has room for it, else *hpsi = nullptr
 int rayleigh_ritz_device(sep_ctx* c, double* d_psi, long m, double* eval_host,

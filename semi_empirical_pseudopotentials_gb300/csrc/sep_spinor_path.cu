@@ -169,14 +169,20 @@ bool vso_on_tensor_cores(const sep_ctx* c) {
 
 // the status of the contractions since the last check
 int vso_check(sep_ctx* c) {
-  if (!c->so_planes) return kOk;
-  int h = 0;
-  CK(oz::check_status(c->so_tensor.err, c->stream, &h));
+  int h = c->so_err;
+  c->so_err = 0;
+  if (c->so_planes) {
+    int now = 0;
+    CK(oz::check_status(c->so_tensor.err, c->stream, &now));
+    if (now != 0) {
+      CK(cudaMemsetAsync(c->so_tensor.err, 0, sizeof(int), c->stream));
+      h = now;
+    }
+  }
   if (h != 0) {
     char b[160];
     snprintf(b, sizeof b, "spinor path: a bounded wait in the contraction kernel ran out (%d)", h);
     set_error(b);
-    CK(cudaMemsetAsync(c->so_tensor.err, 0, sizeof(int), c->stream));
     return kErrCuda;
   }
   return kOk;
@@ -186,7 +192,16 @@ int vso_check(sep_ctx* c) {
 int vso(sep_ctx* c, const double* psi, long long nsp, double* out) {
   if (nsp > 65535) return arg_fail("spinor path: more than 65535 spinors in one call");
   if (c->so_kmax > 0) {
-    RET(grow(c, c->w_soc, vso_scratch(c) * (size_t)nsp));
+    const size_t need = vso_scratch(c) * (size_t)nsp;
+    if (need > c->w_soc.bytes) {
+      cudaStreamSynchronize(c->stream);
+      if (c->w_soc.ensure(need) != cudaSuccess) {  // no room: K formed in place from now on
+        release_kept_operator(c);
+        cudaGetLastError();
+      }
+    }
+  }
+  if (c->so_kmax > 0) {
     const int* off = c->w_sog.as<int>();
     CK(spinor_vso_kept(psi, (long)c->n, (long)nsp, c->so_natom, c->so_nnlc,
                        c->w_nlc.as<sep_nlc>(), c->w_nl.as<long>(), c->so_sigma, c->dv,
@@ -499,6 +514,7 @@ int spinor_set_operator(sep_ctx* c, long natom, long nnlc, const sep_nlc* nlc, c
   c->so_ready = false;
   c->so_kmax = 0;
   c->so_planes = false;
+  c->so_err = 0;
   CK(cudaStreamSynchronize(c->stream));
   RET(grow(c, c->w_nlc, sizeof(sep_nlc) * (size_t)std::max<long>(1, natom * nnlc)));
   RET(grow(c, c->w_nl, sizeof(long) * (size_t)std::max<long>(1, natom)));
@@ -680,12 +696,16 @@ int spinor_filter_device(sep_ctx* c, const double* d_start, long ns, const doubl
   const long ms2 = 2 * ms;
   // per spinor: 2 slots of (K history grids + 1 transform grid), 2 x 2 ms2
   // accumulators per point, Vso psi and the list points' contributions to it
-  const size_t per_sp = 2 * (sizeof(cx<double>) * (size_t)n * (K + 1) +
-                             sizeof(double) * 2 * (size_t)ms2 * n) +
-                        sizeof(double) * (size_t)L + vso_scratch(c);
-  const size_t have = c->w_hist.bytes + c->w_fft.bytes + c->w_acc.bytes + c->w_so.bytes +
-                      c->w_soc.bytes;
-  long long Bs = (long long)(((size_t)(0.6 * (double)free_device_bytes()) + have) / per_sp);
+  const auto fit = [&] {
+    const size_t per_sp = 2 * (sizeof(cx<double>) * (size_t)n * (K + 1) +
+                               sizeof(double) * 2 * (size_t)ms2 * n) +
+                          sizeof(double) * (size_t)L + vso_scratch(c);
+    const size_t have = c->w_hist.bytes + c->w_fft.bytes + c->w_acc.bytes + c->w_so.bytes +
+                        c->w_soc.bytes;
+    return (long long)(((size_t)(0.6 * (double)free_device_bytes()) + have) / per_sp);
+  };
+  long long Bs = fit();
+  if (Bs < 1 && release_kept_operator(c)) Bs = fit();
   if (Bs < 1) return arg_fail("spinor filter: not enough device memory for one spinor");
   Bs = std::min<long long>({Bs, (long long)ns, 32767LL});
   const long long Bc = 2 * Bs;  // complex grids (slots) per chunk

@@ -477,3 +477,47 @@ def test_one_long_list_among_many_short_ones():
         assert np.array_equal(*out) == same
         assert np.abs(out[0] - out[1]).max() <= 1e-13 * np.abs(out[0]).max()
     ctx.close()
+
+
+@pytest.mark.parametrize("call", ["filter", "hamiltonian"])
+def test_operator_gives_its_kept_memory_back(call):
+    """An operator of 8 lists of 2048 points keeps 1 GB (K, its digits, their
+    workspace).  With 200 MB of the device left, a filter whose history needs 190
+    MB of them per spinor (of which it takes 0.6) and an apply to 250 spinors (1.0
+    GB) run all the same: the operator gives that memory back and forms K on each
+    apply.  Same values as with room to spare, to the tolerance of the operator's
+    other tests."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(13)
+    dims, h = (32, 32, 40), 0.5
+    ngrid = int(np.prod(dims))
+    nlc = np.stack([_list_entries(rng, 2048, ngrid) for _ in range(8)])
+    nl = np.full(8, 2048, dtype=np.int64)
+    ns = 2 if call == "filter" else 250
+    psi = rng.normal(size=(ns, 2 * ngrid)) + 1j * rng.normal(size=(ns, 2 * ngrid))
+
+    def run(path):
+        if call == "hamiltonian":
+            return path.hamiltonian(psi)
+        return path.filter(psi, np.eye(8, 130) + 0j, np.zeros(130), 1e-4, -1.0)
+
+    out = []
+    torch.cuda.empty_cache()
+    for left in (None, 200 << 20):
+        ctx = binding.Context(dims, (h, h, h), potl=np.zeros(ngrid), precision="f64", ekinmax=20.0)
+        ctx.set_block_steps(128 if call == "filter" else 32)
+        before = torch.cuda.mem_get_info()[0]
+        path = spinor.SpinorPath(ctx, nlc, nl, sigma=h)
+        assert before - torch.cuda.mem_get_info()[0] > 800 << 20
+        hog = []
+        try:
+            while left and torch.cuda.mem_get_info()[0] > left + (64 << 20):
+                room = torch.cuda.mem_get_info()[0] - left
+                hog.append(torch.empty(min(room, 16 << 30), dtype=torch.uint8, device="cuda"))
+            out.append(run(path))
+        finally:
+            hog.clear()
+            torch.cuda.empty_cache()
+            ctx.close()
+    for s in range(ns):
+        assert np.abs(out[1][s] - out[0][s]).max() <= 1e-13 * np.abs(out[0][s]).max()
