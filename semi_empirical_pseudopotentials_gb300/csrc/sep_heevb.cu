@@ -593,6 +593,7 @@ __global__ void __launch_bounds__(32)
     }
     s2 = warp_sum(s2);
     warp_largest(big, jmax);
+    __syncwarp();  // x[jmax] was last written by another lane; shuffles order no memory
     double scl = 1.0 / sqrt(s2);
     if (x[jmax] < 0.0) scl = -scl;
     double* zj = Zm + (size_t)jj * n;
