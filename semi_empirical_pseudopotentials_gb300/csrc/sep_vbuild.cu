@@ -396,7 +396,10 @@ int sep_vbuild_backward(sep_ctx* c, long natom, const double* xyz, const int* ty
   if (e == cudaSuccess) e = cudaMemsetAsync(d_tab, 0, sizeof(double) * nb, c->stream);
   if (e == cudaSuccess && d_sc) e = cudaMemsetAsync(d_sc, 0, sizeof(double) * natom, c->stream);
   if (e == cudaSuccess) {
-    const int smem_bins = (nb * sizeof(double) <= 32 * 1024) ? (int)nb : 0;  // beside 15 KB
+    // bins in shared memory as far as a block's 48 KB go beside the 16 KB of
+    // each_pair; beyond it global atomics are the faster (2260 atoms on 128^3, whole
+    // calls: 2 x 2049 to 2 x 2304 bins 42 to 40 ms, 46 with 36 KB of shared bins)
+    const int smem_bins = (nb * sizeof(double) <= 32 * 1024) ? (int)nb : 0;
     dim3 g((unsigned)((c->nx + BX - 1) / BX), (unsigned)((c->ny + BY - 1) / BY),
            (unsigned)((c->nz + BZ - 1) / BZ));
     k_vbuild_bwd<<<g, kNT, smem_bins * sizeof(double), c->stream>>>(a, d_g, smem_bins, d_tab,
