@@ -311,13 +311,14 @@ template <int LX, int LY, int NT> __device__ __forceinline__ void row_fwd_b(C* p
   }
 }
 
-// x inverse stage A', the Newton epilogue and (FWD) x forward stage A in one
-// step: item (row, n1) holds the natural elements n1 + N1 n2 of its row, which
+// x inverse stage A', the Newton epilogue and x forward stage A in one step (the
+// last pass of a filter has no use for the latter, which it makes in shared
+// memory all the same: the step's kernel serves all modes): item (row, n1) holds the natural elements n1 + N1 n2 of its row, which
 // are also the inputs of forward item (row, x1 = n1).  psi_{j-1}, V and psi_j
 // (plane offsets off in the batch, goff in one grid) are accessed at those
 // elements: N1 adjacent threads cover N1 adjacent elements (64 bytes for N1 =
 // 8) of a row.
-template <int LX, int LY, int NT, bool FWD>
+template <int LX, int LY, int NT>
 __device__ __forceinline__ void row_inv_a_epi(C* pl, const C* tw, const PassArgs<float>& a,
                                               long long off, long long goff, float alpha,
                                               float beta) {
@@ -350,13 +351,11 @@ __device__ __forceinline__ void row_inv_a_epi(C* pl, const C* tw, const PassArgs
       pout[g0 + S::n1x * n2] = o;
       u[n2] = o;
     }
-    if constexpr (FWD) {
-      Dft<S::n2x, -1, float>::run(u);
+    Dft<S::n2x, -1, float>::run(u);
 #pragma unroll
-      for (int k2 = 1; k2 < S::n2x; ++k2) u[k2] = mul<float>(u[k2], tw[(n1 * k2) % LX]);
+    for (int k2 = 1; k2 < S::n2x; ++k2) u[k2] = mul<float>(u[k2], tw[(n1 * k2) % LX]);
 #pragma unroll
-      for (int k2 = 0; k2 < S::n2x; ++k2) p[S::n1x * k2] = u[k2];
-    }
+    for (int k2 = 0; k2 < S::n2x; ++k2) p[S::n1x * k2] = u[k2];
   }
 }
 
@@ -443,7 +442,7 @@ __global__ void __launch_bounds__(NT, MINB) xy_plane_pass(PassArgs<float> a, int
       __syncthreads();
       xy::row_inv_b<LX, LY, NT>(pl, tw);  // x inverse, epilogue and x forward stage A
       __syncthreads();
-      xy::row_inv_a_epi<LX, LY, NT, true>(pl, tw, a, off, goff, alpha, beta);
+      xy::row_inv_a_epi<LX, LY, NT>(pl, tw, a, off, goff, alpha, beta);
     }
     prefetch_data(p + gridDim.x);
     if (mode == kInvEpi) continue;
