@@ -207,3 +207,31 @@ def test_filter_into_a_buffer_at_any_double(precision, ns):
     ctx.close()
     assert np.abs(got[0]).max() > 0.0
     assert np.array_equal(got[0], got[1])
+
+
+@pytest.mark.parametrize("ms", [1, 4, 9, 20, 32])
+@pytest.mark.parametrize("nc,K", [(70, 32), (33, 8)])
+def test_accumulation_against_the_states_themselves(ms, nc, K):
+    """The complex64 accumulation against sums formed here in FP64 from the states
+    psi_j of the same recursion, which filters with unit coefficients return as
+    they are (every other product is zero): each sum of nc products, added in FP32
+    within blocks of K steps and then block by block, errs by less than (K + nc / K
+    + 2) 2^-24 of sum |a_j psi_j|.  An odd number of states, points that are no
+    whole number of 64."""
+    dims, ns = (14, 18, 20), 3
+    ctx, pot, dv, npts = _job(dims, 6, "mixed")
+    ctx.set_block_steps(K)
+    vmin, dE = float(pot.min()), 40.0
+    ar, ai, zn = sep.coefficients(np.linspace(-1.2, -0.2, ms), nc, dE, vmin,
+                                  (nc / (2.5 * dE)) ** 2)
+    start = sep.start_states(-15, ns, npts, dv)
+    psi = np.concatenate([ctx.filter(start, np.eye(nc)[j:j + 32], zn, 4.0 / dE, vmin)
+                          for j in range(0, nc, 32)], axis=1)
+    got = ctx.filter(start, ar, zn, 4.0 / dE, vmin)
+    ctx.close()
+    assert np.array_equal(psi, psi.astype(np.float32))
+    a = ar.astype(np.float32).astype(np.float64)
+    ref = np.einsum("ej,sjg->seg", a, psi)
+    size = np.einsum("ej,sjg->seg", np.abs(a), np.abs(psi))
+    assert np.abs(ref).max() > 0.0
+    assert np.all(np.abs(got - ref) <= (K + nc / K + 2) * 2.0 ** -24 * size)
