@@ -21,6 +21,7 @@
 
 #include <algorithm>
 #include <cstdio>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/sep_gb300.h"
@@ -41,9 +42,8 @@ using namespace sep;
 
 namespace {
 
-constexpr int BX = 8, BY = 8, BZ = 8;  // points per brick
-constexpr int kNT = 128;               // threads per block, four z points each
-constexpr int kPZ = 4;
+constexpr int BX = 8, BY = 8;  // points per brick in x and y; in z 2 PZ
+constexpr int kNT = 128;       // threads per block, PZ z points each
 constexpr int kListCap = 512;          // atoms kept per round
 constexpr int kTile = 64;              // atoms whose squares are in shared memory at once
 
@@ -125,20 +125,21 @@ __device__ int collect(const VArgs& a, long long a0, double bx0, double bx1, dou
   return tot;
 }
 
-// Calls body(u, d, atom, type, segment) in atom order for the four points u of
+// Calls body(u, d, atom, type, segment) in atom order for the PZ points u of
 // this thread (x, y, z0 + u of the brick) and every atom whose table reaches
 // them; d = |r_g - R_a| with the reference's roundings.  (x - X)^2, (y - Y)^2
 // and (z - Z)^2 take 24 values per atom and brick, which the block forms once,
 // so a pair costs one addition and the square root; a third of the pairs of a
 // brick lie beyond the table, which FP32 decides where all of a warp do.
-template <typename F> __device__ __forceinline__ void each_pair(const VArgs& a, F body) {
+template <int PZ, typename F> __device__ __forceinline__ void each_pair(const VArgs& a, F body) {
+  constexpr int BZ = kNT / (BX * BY) * PZ;
   __shared__ int list[kListCap];
   __shared__ double sq[kTile][BX + BY + BZ];
   __shared__ int atom_type[kTile];
   __shared__ double tab_dr[kTile];
   __shared__ float tab_inv[kTile], tab_end[kTile];
   const int tid = threadIdx.x;
-  const int x = tid % BX, y = tid / BX % BY, z0 = tid / (BX * BY) * kPZ;
+  const int x = tid % BX, y = tid / BX % BY, z0 = tid / (BX * BY) * PZ;
   const int jx0 = blockIdx.x * BX, jy0 = blockIdx.y * BY, jz0 = blockIdx.z * BZ;
   const int ex = min(jx0 + BX, a.nx) - 1, ey = min(jy0 + BY, a.ny) - 1,
             ez = min(jz0 + BZ, a.nz) - 1;
@@ -180,7 +181,7 @@ template <typename F> __device__ __forceinline__ void each_pair(const VArgs& a, 
         const long n = a.tab_n[t];
         const double xy = __dadd_rn(sq[k][x], sq[k][BX + y]);
 #pragma unroll
-        for (int u = 0; u < kPZ; ++u) {
+        for (int u = 0; u < PZ; ++u) {
           const double d2 = __dadd_rn(xy, sq[k][BX + BY + z0 + u]);
           const float q = sqrtf((float)d2) * inv;
           if (q > fn && q < 1e30f) continue;  // past n - 1 by more than the rounding
@@ -195,10 +196,11 @@ template <typename F> __device__ __forceinline__ void each_pair(const VArgs& a, 
 }
 
 // this thread's points inside the grid: offset of point u, or -1
-__device__ __forceinline__ long long point_of(const VArgs& a, int u) {
+template <int PZ> __device__ __forceinline__ long long point_of(const VArgs& a, int u) {
+  constexpr int BZ = kNT / (BX * BY) * PZ;
   const int tid = threadIdx.x;
   const int jx = blockIdx.x * BX + tid % BX, jy = blockIdx.y * BY + tid / BX % BY,
-            jz = blockIdx.z * BZ + tid / (BX * BY) * kPZ + u;
+            jz = blockIdx.z * BZ + tid / (BX * BY) * PZ + u;
   return jx < a.nx && jy < a.ny && jz < a.nz
              ? (long long)a.nx * ((long long)a.ny * jz + jy) + jx
              : -1;
@@ -208,9 +210,10 @@ __device__ __forceinline__ long long point_of(const VArgs& a, int u) {
 // operations; with the two divisions of the segment's line and of r / dr in
 // each pair, and a thread per point, about 45).  2260 atoms on 128^3, 310 M
 // pairs within the tables: 11.9 ms, 30.1 ms before.
+template <int PZ>
 __global__ void __launch_bounds__(kNT) k_vbuild(VArgs a, double* __restrict__ potl) {
-  double sum[kPZ] = {};
-  each_pair(a, [&](int u, double d, int ia, int t, long i) {
+  double sum[PZ] = {};
+  each_pair<PZ>(a, [&](int u, double d, int ia, int t, long i) {
     double2 l;
     if (a.scale) {  // filterStrainCube/interpolate.c:11-25
       const double* tr = a.tab_r + t * a.stride;
@@ -224,14 +227,15 @@ __global__ void __launch_bounds__(kNT) k_vbuild(VArgs a, double* __restrict__ po
     sum[u] = __dadd_rn(sum[u], __dadd_rn(__dmul_rn(l.x, d), l.y));
   });
 #pragma unroll
-  for (int u = 0; u < kPZ; ++u) {
-    const long long g = point_of(a, u);
+  for (int u = 0; u < PZ; ++u) {
+    const long long g = point_of<PZ>(a, u);
     if (g >= 0) potl[g] = sum[u];
   }
 }
 
 // Bound by the FP64 pipe and by the two shared-memory additions of a pair.
 // The same case: 15.7 ms, 30.3 ms before.
+template <int PZ>
 __global__ void __launch_bounds__(kNT)
 k_vbuild_bwd(VArgs a, const double* __restrict__ dpotl, int nbins_smem,
              double* __restrict__ dtab, double* __restrict__ dscale) {
@@ -239,13 +243,13 @@ k_vbuild_bwd(VArgs a, const double* __restrict__ dpotl, int nbins_smem,
   const bool use_smem = nbins_smem > 0;
   for (int i = threadIdx.x; i < nbins_smem; i += blockDim.x) hist[i] = 0.0;
   __syncthreads();
-  double gval[kPZ];
+  double gval[PZ];
 #pragma unroll
-  for (int u = 0; u < kPZ; ++u) {
-    const long long g = point_of(a, u);
+  for (int u = 0; u < PZ; ++u) {
+    const long long g = point_of<PZ>(a, u);
     gval[u] = g >= 0 ? dpotl[g] : 0.0;
   }
-  each_pair(a, [&](int u, double d, int ia, int t, long i) {
+  each_pair<PZ>(a, [&](int u, double d, int ia, int t, long i) {
     if (gval[u] == 0.0) return;
     const long long b = (long long)t * a.stride + i;
     const double2 l = a.seg[b];
@@ -267,6 +271,34 @@ k_vbuild_bwd(VArgs a, const double* __restrict__ dpotl, int nbins_smem,
   __syncthreads();
   for (int i = threadIdx.x; i < nbins_smem; i += blockDim.x)
     if (hist[i] != 0.0) atomicAdd(&dtab[i], hist[i]);
+}
+
+// Points per thread, by the 8 x 8 x 8 bricks of the grid.  Small grids have too few
+// of them to fill the chip, and a thread's four points add one after another; the
+// lists and squares of a brick cost more with smaller ones.  400 atoms, forward /
+// backward call in us with 1, 2 and 4 points (a thread per point in 8 x 8 x 4
+// bricks, squares and divisions per pair: 14^3 1237 / 1291, 32^3 1258 / 1300):
+// 14^3 386 / 622, 656 / 1013, 1165 / 1868; 36^3 (125 bricks) 810 / 1142, 1000 / 1411,
+// 1210 / 1955; 48^3 (216) 1550 / 2150, 1472 / 2005, 1855 / 2631; 96^3 (1728) 5344 /
+// 6106, 5255 / 5786, 5701 / 6159; 128^3 (4096) 7627 / 7543, 7351 / 6935, 7271 / 6984.
+int points_per_thread(const sep_ctx* c) {
+  const auto parts = [](long n) { return (n + 7) / 8; };
+  const long bricks = parts(c->nx) * parts(c->ny) * parts(c->nz);
+  return bricks < 152 ? 1 : bricks < 2048 ? 2 : 4;
+}
+
+// launches f(points per thread, grid of bricks)
+template <typename F> void with_bricks(const sep_ctx* c, F f) {
+  const auto grid = [&](int pz) {
+    const int bz = kNT / (BX * BY) * pz;
+    return dim3((unsigned)((c->nx + BX - 1) / BX), (unsigned)((c->ny + BY - 1) / BY),
+                (unsigned)((c->nz + bz - 1) / bz));
+  };
+  switch (points_per_thread(c)) {
+    case 1: f(std::integral_constant<int, 1>{}, grid(1)); break;
+    case 2: f(std::integral_constant<int, 2>{}, grid(2)); break;
+    default: f(std::integral_constant<int, 4>{}, grid(4)); break;
+  }
 }
 
 struct VHost {
@@ -355,9 +387,9 @@ int sep_vbuild(sep_ctx* c, long natom, const double* xyz, const int* types, cons
     in.release();
     return cuda_fail(e, "cudaMalloc potl", __LINE__);
   }
-  dim3 g((unsigned)((c->nx + BX - 1) / BX), (unsigned)((c->ny + BY - 1) / BY),
-         (unsigned)((c->nz + BZ - 1) / BZ));
-  k_vbuild<<<g, kNT, 0, c->stream>>>(a, d_pot);
+  with_bricks(c, [&](auto pz, dim3 g) {
+    k_vbuild<decltype(pz)::value><<<g, kNT, 0, c->stream>>>(a, d_pot);
+  });
   e = cudaGetLastError();
   if (e == cudaSuccess && potl)
     e = cudaMemcpyAsync(potl, d_pot, sizeof(double) * c->n, cudaMemcpyDeviceToHost, c->stream);
@@ -400,10 +432,10 @@ int sep_vbuild_backward(sep_ctx* c, long natom, const double* xyz, const int* ty
     // each_pair; beyond it global atomics are the faster (2260 atoms on 128^3, whole
     // calls: 2 x 2049 to 2 x 2304 bins 42 to 40 ms, 46 with 36 KB of shared bins)
     const int smem_bins = (nb * sizeof(double) <= 32 * 1024) ? (int)nb : 0;
-    dim3 g((unsigned)((c->nx + BX - 1) / BX), (unsigned)((c->ny + BY - 1) / BY),
-           (unsigned)((c->nz + BZ - 1) / BZ));
-    k_vbuild_bwd<<<g, kNT, smem_bins * sizeof(double), c->stream>>>(a, d_g, smem_bins, d_tab,
-                                                                    d_sc);
+    with_bricks(c, [&](auto pz, dim3 g) {
+      k_vbuild_bwd<decltype(pz)::value>
+          <<<g, kNT, smem_bins * sizeof(double), c->stream>>>(a, d_g, smem_bins, d_tab, d_sc);
+    });
     e = cudaGetLastError();
   }
   if (e == cudaSuccess)

@@ -370,15 +370,18 @@ def test_fp64_transforms_of_every_length(dims):
         assert np.linalg.norm(got[s] - ref.ravel()) <= 2e-14 * np.linalg.norm(ref)
 
 
-@pytest.mark.parametrize("bins", [300, 4096, 4097, 4608, 4609])
-def test_vbuild_and_its_backward_over_the_whole_grid(bins):
+@pytest.mark.parametrize("dims,bins", [((14, 18, 20), b) for b in (300, 4096, 4097, 4608, 4609)] +
+                         [((20, 36, 112), 1024), ((48, 48, 48), 4097), ((36, 128, 256), 1024),
+                          ((256, 128, 36), 4097)])
+def test_vbuild_and_its_backward_over_the_whole_grid(dims, bins):
     """V(r) bit for bit at every point, bricks beyond the first in each axis among
     them, and the backward's table gradient against extended precision, with
-    tables on both sides of the sizes whose bins fit in shared memory.  A point's
+    tables on both sides of the sizes whose bins fit in shared memory and grids
+    that take 1, 2 and 4 points per thread, cut within a brick.  A point's
     weight w = (d - r_i) / dr errs by 3 u d / dr < 2e-12 for 4609 bins, so a bin by
     that times the sum of what it collects."""
     rng = np.random.default_rng(bins)
-    dims, h, natom = (14, 18, 20), 0.7, 9
+    h, natom = 0.7, 9 if max(dims) < 100 else 3
     mins = [-0.5 * n * h for n in dims]
     ax = [np.cumsum(np.concatenate([[m], np.full(n - 1, h)])) for n, m in zip(dims, mins)]
     xyz = rng.uniform(-5, 5, (natom, 3))
