@@ -1,5 +1,5 @@
 // sep_heevb.cuh -- the lowest eigenpairs of many small Hermitian matrices
-// at once: Householder tridiagonalisation, bisection, inverse
+// at once: Householder tridiagonalisation, multisection, inverse
 // iteration and back-transformation (see sep_heevb.cu).
 #pragma once
 
