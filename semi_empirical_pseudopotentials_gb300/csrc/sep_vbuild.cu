@@ -128,7 +128,7 @@ __device__ int collect(const VArgs& a, long long a0, double bx0, double bx1, dou
 // Calls body(u, d, atom, type, segment) in atom order for the PZ points u of
 // this thread (x, y, z0 + u of the brick) and every atom whose table reaches
 // them; d = |r_g - R_a| with the reference's roundings.  (x - X)^2, (y - Y)^2
-// and (z - Z)^2 take 24 values per atom and brick, which the block forms once,
+// and (z - Z)^2 take 18 to 24 values per atom and brick, which the block forms once,
 // so a pair costs one addition and the square root; a third of the pairs of a
 // brick lie beyond the table, which FP32 decides where all of a warp do.
 template <int PZ, typename F> __device__ __forceinline__ void each_pair(const VArgs& a, F body) {
